@@ -22,10 +22,9 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-I", os.path.join(REPO, "include")]
 
 # FP32 kernels: fast single-precision math (MUFU exp/log/pow, approximate
-# division and square root, denormals flushed) and FP32 saturation terms inside
-# the FP64 canopy solve.  Their error against the float64 kernels is measured by
-# tests/test_gpu_precision.py.
-F32_FLAGS = ["-use_fast_math", "-DIBIS_FAST_SAT=1"]
+# division and square root, denormals flushed).  Their error against the float64
+# kernels is measured by tests/test_gpu_precision.py.
+F32_FLAGS = ["-use_fast_math"]
 
 # translation unit -> extra flags
 UNITS = {

@@ -4,10 +4,6 @@
 #include "ibis_column.cuh"
 #include "gauss9_gen.cuh"
 
-#ifndef IBIS_FAST_SAT
-#define IBIS_FAST_SAT 0
-#endif
-
 namespace ibis {
 
 // ---------------------------------------------------------------------------
@@ -485,8 +481,8 @@ __device__ __forceinline__ void stomata(Stom<R>& o, Col<R>& c, R tu, R tl, R t12
 }
 
 // ---------------------------------------------------------------------------
-// turvap: 9x9 implicit canopy / air / ground / snow system (canopy_exchange.py:470-811)
-// Always double.  Unknowns: tu ts tl t12 t34 q12 q34 tg ti.
+// turvap: 9x9 implicit canopy / air / ground / snow system (canopy_exchange.py:470-811),
+// the reference's operations.  Unknowns: tu ts tl t12 t34 q12 q34 tg ti.
 // ---------------------------------------------------------------------------
 
 // Inputs of turvap that do not change across the three passes (stored in R;
@@ -513,21 +509,8 @@ struct TvOut {
 struct Sat64 { double q, dq; };
 
 // Saturation humidity and its capped derivative at the blended temperature.
-// The float kernels evaluate the Lowe polynomials in R (they carry R-precision
-// inputs anyway) and widen the result; the float64 kernels stay in double.
-template <typename R>
 __device__ __forceinline__ Sat64 sat64(double t, double ps) {
     Sat64 s;
-#if IBIS_FAST_SAT
-    if constexpr (sizeof(R) == 4) {
-        const float tf = (float)t, pf = (float)ps;
-        const float e = esat(tf);
-        const float q = qsat(e, pf);
-        s.q = q;
-        s.dq = fminf(dqsat(tf, q, e), q * 0.1f);
-        return s;
-    }
-#endif
     double e = esat(t);
     s.q = qsat(e, ps);
     s.dq = fmin(dqsat(t, s.q, e), s.q * 0.1);
@@ -548,42 +531,22 @@ __device__ __forceinline__ void turvap(double (&W)[9], TvOut<R>& o, const double
     const double tg = wg * W[7] + (1.0 - wg) * old[3];
     const double ti = wi * W[8] + (1.0 - wi) * old[4];
     const double t34 = W[4], q12 = W[5], q34 = W[6];
-    const Sat64 Su = sat64<R>(tu, ps), Ss = sat64<R>(ts, ps), Sl = sat64<R>(tl, ps), Sg = sat64<R>(tg, ps),
-                Si = sat64<R>(ti, ps);
+    const Sat64 Su = sat64(tu, ps), Ss = sat64(ts, ps), Sl = sat64(tl, ps), Sg = sat64(tg, ps),
+                Si = sat64(ti, ps);
     const double qu = Su.q, dqu = Su.dq, qs = Ss.q, dqs = Ss.dq, ql = Sl.q, dql = Sl.dq;
     const double qg = Sg.q, dqg = Sg.dq, qi = Si.q, dqi = Si.dq;
 
     // soil-surface humidity factor (canopy_exchange.py:532-572)
-    double hfac;
-    if constexpr (sizeof(R) == 4) {
-        // float kernels: the matric-potential factor in float (it scales qg only)
-        const float psig = -P.grav * X.suction0 * powf(X.zwtot, -X.bex0);
-        hfac = (double)expf(psig / (P.rvap * (float)tg));
-    } else {
-        const double psig = -(double)P.grav * (double)X.suction0 * pow((double)X.zwtot, -(double)X.bex0);
-        hfac = exp(psig / ((double)P.rvap * tg));
-    }
-    const double hfac2 = dv<R>(q34, fmax(qg, eps));
-    double betaw = clip(dv<R>((double)X.zwtot - (double)X.swilt0, fmax(1.0 - (double)X.swilt0, eps)), 0.0, 1.0);
-    if (beta_power != 1.0) {
-        if constexpr (sizeof(R) == 4) betaw = (double)powf((float)betaw, (float)beta_power);   // betaw in [0, 1]
-        else betaw = pow(betaw, beta_power);
-    }
-    double qs1, dqs1;
-    if constexpr (sizeof(R) == 4) {
-        // float kernels: the canopy-air saturation terms in float, like the
-        // five surface saturation terms above (they only weight betaw)
-        const float t34f = (float)t34, e34f = esat(t34f);
-        const float qs1f = qsat(e34f, (float)ps);
-        qs1 = qs1f; dqs1 = dqsat(t34f, qs1f, e34f);
-    } else {
-        const double e34 = esat(t34);
-        qs1 = qsat(e34, ps);
-        dqs1 = dqsat(t34, qs1, e34);
-    }
-    const double xden = cp + dv<R>((double)P.zir * cube(t34), (double)T.sg);
-    const double bfac = dv<R>(hvap * dqs1, xden);
-    const double betas = dv<R>(betaw, 1.0 + bfac * (1.0 - betaw));
+    const double psig = -(double)P.grav * (double)X.suction0 * pow((double)X.zwtot, -(double)X.bex0);
+    const double hfac = exp(psig / ((double)P.rvap * tg));
+    const double hfac2 = (q34 / fmax(qg, eps));
+    double betaw = clip((((double)X.zwtot - (double)X.swilt0) / fmax(1.0 - (double)X.swilt0, eps)), 0.0, 1.0);
+    if (beta_power != 1.0) betaw = pow(betaw, beta_power);
+    const double e34 = esat(t34);
+    const double qs1 = qsat(e34, ps), dqs1 = dqsat(t34, qs1, e34);
+    const double xden = cp + (((double)P.zir * cube(t34)) / (double)T.sg);
+    const double bfac = ((hvap * dqs1) / xden);
+    const double betas = (betaw / (1.0 + bfac * (1.0 - betaw)));
     double qgfac = (betas > 0.0) ? betas * hfac + (1.0 - betas) * hfac2 : hfac2;
     const double qeps = 1.0e-10;
     if (q34 > qg + qeps) qgfac = 1.0;
@@ -597,19 +560,19 @@ __device__ __forceinline__ void turvap(double (&W)[9], TvOut<R>& o, const double
     double fr[12];
 #pragma unroll
     for (int j = 0; j < 12; ++j) fr[j] = (double)S(IBIS_STAT_FRAC, j);
-    const double suw = fmin(fwux * su, dv<R>(0.8 * (X.wliqu + X.wsnou), fmax(dt * (qu - q12), eps)));
+    const double suw = fmin(fwux * su, ((0.8 * (X.wliqu + X.wsnou)) / fmax(dt * (qu - q12), eps)));
     const double sut = fmax(0.0, (1.0 - fwux) * 0.5 * (tb * fr[0] + tb * fr[1] + tb * fr[2] + tc * fr[3]
                                                       + tb * fr[4] + tc * fr[5] + tb * fr[6] + tb * fr[7]));
     const double hvu = hvap + cvap * (ta - tmelt) - ch2o * (tu - tmelt);
     const double hsu = hsub + cvap * (ta - tmelt) - cice * (tu - tmelt);
     const double suh = suw * (X.rliqu * hvu + (1.0 - X.rliqu) * hsu) + sut * hvu;
-    const double ssw = fmin(fwsx * ss, dv<R>(0.8 * (X.wliqs + X.wsnos), fmax(dt * (qs - q12), eps)));
+    const double ssw = fmin(fwsx * ss, ((0.8 * (X.wliqs + X.wsnos)) / fmax(dt * (qs - q12), eps)));
     const double ssh = ssw * (X.rliqs * (hvap + cvap * (ta - tmelt) - ch2o * (ts - tmelt))
                               + (1.0 - X.rliqs) * (hsub + cvap * (ta - tmelt) - cice * (ts - tmelt)));
-    const double slw = fmin(fwlx * sl, dv<R>(0.8 * (X.wliql + X.wsnol), fmax(dt * (ql - q34), eps)));
+    const double slw = fmin(fwlx * sl, ((0.8 * (X.wliql + X.wsnol)) / fmax(dt * (ql - q34), eps)));
     const double tls = st.tcls, tl3 = st.tcl3, tl4 = st.tcl4;
     const double slt0 = fmax(0.0, (1.0 - fwlx) * 0.5 * (tls * fr[8] + tls * fr[9] + tl4 * fr[10] + tl3 * fr[11]));
-    const double slt = dv<R>(slt0 * (double)X.lai0, fmax((double)X.lsl0, eps));
+    const double slt = ((slt0 * (double)X.lai0) / fmax((double)X.lsl0, eps));
     const double hvl = hvap + cvap * (ta - tmelt) - ch2o * (tl - tmelt);
     const double slh = slw * (X.rliql * hvl + (1.0 - X.rliql) * (hsub + cvap * (ta - tmelt) - cice * (tl - tmelt)))
                      + slt * hvl;

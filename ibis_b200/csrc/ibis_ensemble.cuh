@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(256, 1) ensemble_kernel(const EnsArgs e, const
     const int lane = threadIdx.x & 31;
     const int nitem = (e.nwork + 31) >> 5;
     const bool kahan = (P.flags & IBIS_FLAG_KAHAN) != 0;
-    const Diag<float> D{nullptr, 0};
+    const Diag<float, false> D{nullptr, 0};
     for (;;) {
         int item = 0;
         if (lane == 0) item = atomicAdd(e.queue, 1);
@@ -262,7 +262,7 @@ __global__ void __launch_bounds__(128, 2) ensemble_hour_kernel(const EnsArgs e, 
     const Stat<float> S{e.stat + site, e.ld_site};
     const Acc<float> A{e.acc ? e.acc + r : nullptr, e.ld_run, (P.flags & IBIS_FLAG_KAHAN) != 0, hour + 1 == nstep};
     const Forc<float> F = load_forc_record(e.forc + (size_t)(first + hour) * IBIS_FORC_COUNT);
-    column_step<float, NT, SU, SL>(c, F, S, Diag<float>{nullptr, 0}, A, P, q);
+    column_step<float, NT, SU, SL>(c, F, S, Diag<float, false>{nullptr, 0}, A, P, q);
     if (e.yearly && (pos + hour + 1) % e.year_steps == 0) {
         const int y = (pos + hour + 1) / e.year_steps - 1;
         if (y < e.nyear) yearly_snapshot(e, A, r, y);

@@ -4,12 +4,6 @@
 #pragma once
 #include "ibis_column.cuh"
 
-// 1: the FP32 kernels solve soil water in float for the hour's increments
-// (soil_water_increments); 0: in double on absolute contents (soil_water).
-#ifndef IBIS_SOILW_INCREMENTS
-#define IBIS_SOILW_INCREMENTS 1
-#endif
-
 namespace ibis {
 
 // Thomas algorithm (solvers.py:17-83) on N unknowns held in registers.
@@ -109,7 +103,7 @@ __device__ __forceinline__ void readapt_layers(R (&h)[NS], R (&t)[NS], R htop, R
 }
 
 // ---------------------------------------------------------------------------
-// soilh2o (soil_physics.py:196-373), always double
+// soilh2o (soil_physics.py:196-373)
 // ---------------------------------------------------------------------------
 template <typename R>
 __device__ __forceinline__ void soil_water(double (&w)[NL], double& wpud, double (&wflo)[NL + 1],
@@ -144,14 +138,8 @@ __device__ __forceinline__ void soil_water(double (&w)[NL], double& wpud, double
         double bwn = bwn1 * wa;
         if (bwn < dmin) bwn1 = 0.0;
         bwn = fmax(bwn, dmin);
-        double dw, wam1;
-        if constexpr (sizeof(R) == 4) {
-            dw = (w[k] - w[k - 1]) * P.sw_rhm[k];
-            wam1 = pw1 * pw1;                           // wa**(m-1) = (wa**(nn-1))**2
-        } else {
-            dw = (w[k] - w[k - 1]) / P.sw_hm[k];
-            wam1 = ipow(wa, m - 1);
-        }
+        const double dw = (w[k] - w[k - 1]) / P.sw_hm[k];
+        const double wam1 = ipow(wa, m - 1);
         double ek = (-1.0 + (double)m) * a * (wam1 * wa) + ((0.0 * bwn) - (double)nn * bwn1 * wa) * dw;
         double fk = (double)(-m) * a * wam1 + (double)nn * bwn1 * dw;
         double zi = fmax(0.0, 1.0 - fmax(wisoi[k - 1], wisoi[k]));
@@ -171,36 +159,21 @@ __device__ __forceinline__ void soil_water(double (&w)[NL], double& wpud, double
 #pragma unroll
     for (int k = 0; k < NL; ++k) {
         const double h = (double)P.hsoi[k];
-        const double dt = dv<R>(dtime, fmax(pflo[k] * h, 1e-30));
+        const double dt = (dtime / fmax(pflo[k] * h, 1e-30));
         double d1, d2, d3;
         double rk = w[k] + dt * (e[k + 1] - e[k]);
-        if constexpr (sizeof(R) == 4) {
-            // the layer geometry as precomputed multipliers
-            const double rhb = P.sw_rhb[k];
-            d1 = dt * (f[k] * P.sw_c1[k] - g[k] * rhb);
-            if (k == 0) rk = rk + dt * (fwtop + fwpud) * P.rrhow64;
-            if (k < NL - 1) {
-                const double rhp = P.sw_rhp[k];
-                d2 = 1.0 + dt * (-f[k + 1] * P.sw_c3[k] + f[k] * P.sw_c5[k] + g[k + 1] * rhp + g[k] * rhb);
-                d3 = dt * (-f[k + 1] * P.sw_c6[k] - g[k + 1] * rhp);
-            } else {
-                d2 = 1.0 + dt * (-f[k + 1] + f[k] * P.sw_c5[k] + g[k] * rhb);
-                d3 = 0.0;
-            }
+        const double hm = P.sw_hb[k];
+        const int km1 = k > 0 ? k - 1 : 0;
+        d1 = dt * (f[k] * 0.5 * h / hm - g[k] / hm);
+        if (k == 0) rk = rk + dt * (fwtop + fwpud) / rhow;
+        if (k < NL - 1) {
+            const double hp = P.sw_hp[k];
+            d2 = 1.0 + dt * (-f[k + 1] * 0.5 * (double)P.hsoi[k + 1] / hp + f[k] * 0.5 * (double)P.hsoi[km1] / hm
+                             + g[k + 1] / hp + g[k] / hm);
+            d3 = dt * (-f[k + 1] * 0.5 * h / hp - g[k + 1] / hp);
         } else {
-            const double hm = P.sw_hb[k];
-            const int km1 = k > 0 ? k - 1 : 0;
-            d1 = dt * (f[k] * 0.5 * h / hm - g[k] / hm);
-            if (k == 0) rk = rk + dt * (fwtop + fwpud) / rhow;
-            if (k < NL - 1) {
-                const double hp = P.sw_hp[k];
-                d2 = 1.0 + dt * (-f[k + 1] * 0.5 * (double)P.hsoi[k + 1] / hp + f[k] * 0.5 * (double)P.hsoi[km1] / hm
-                                 + g[k + 1] / hp + g[k] / hm);
-                d3 = dt * (-f[k + 1] * 0.5 * h / hp - g[k + 1] / hp);
-            } else {
-                d2 = 1.0 + dt * (-f[k + 1] + f[k] * 0.5 * (double)P.hsoi[km1] / hm + g[k] / hm);
-                d3 = 0.0;
-            }
+            d2 = 1.0 + dt * (-f[k + 1] + f[k] * 0.5 * (double)P.hsoi[km1] / hm + g[k] / hm);
+            d3 = 0.0;
         }
         if (k == 0) d1 = 0.0;
         lo[k] = d1; di[k] = d2; up[k] = d3; r[k] = rk;
@@ -211,10 +184,10 @@ __device__ __forceinline__ void soil_water(double (&w)[NL], double& wpud, double
 #pragma unroll
     for (int k = NL - 1; k >= 0; --k) {
         double zz = rhow * poros[k] * fmax(eps, 1.0 - wisoi[k]) * (double)P.hsoi[k];
-        double wk = wn[k] + dv<R>(dtime * fsq, zz);
-        double fsn = dv<R>(fmax(wk - 1.0, 0.0) * zz, dtime);
+        double wk = wn[k] + ((dtime * fsq) / zz);
+        double fsn = ((fmax(wk - 1.0, 0.0) * zz) / dtime);
         wk = fmin(wk, 1.0);
-        wflo[k] = wflo[k + 1] + dv<R>((wk - w[k]) * zz, dtime);
+        wflo[k] = wflo[k + 1] + (((wk - w[k]) * zz) / dtime);
         wn[k] = wk;
         fsq = fsn;
     }
@@ -224,204 +197,19 @@ __device__ __forceinline__ void soil_water(double (&w)[NL], double& wpud, double
     for (int k = 0; k < NL; ++k) w[k] = wn[k];
 }
 
-// The FP32 kernels' soilh2o (soil_physics.py:196-373): the same implicit system
-// in float, solved for the hour's increments delta = w_new - w.  Its
-// right-hand side holds the flux divergence and the implicit terms applied to
-// the current profile, so float32 rounds relative to the hour's change where a
-// layer changes slowly, and relative to w where the implicit terms dominate
-// (wet, conductive layers), as the float32 state's own storage does.  The
-// saturation bound and the upward excess flux work on the increments too.
-template <typename R>
-__device__ __forceinline__ void soil_water_increments(float (&w)[NL], float& wpud, float (&wflo)[NL + 1],
-                                                      const float (&wisoi)[NL], const float (&poros)[NL],
-                                                      const float (&pflo)[NL], const Stat<R>& S, float fwtop,
-                                                      float fwpud, const DevParams<R>& P) {
-    const float dmin = 1e-9f;
-    const float dtime = P.dtime, rhow = P.rhow, eps = P.epsilon;
-    const bool consistent = (P.flags & IBIS_FLAG_H2O_CONSISTENT) != 0;
-    float e[NL + 1], f[NL + 1], g[NL + 1];
-    e[0] = f[0] = g[0] = 0.0f;
-    f[NL] = g[NL] = 0.0f;
-    float hyd_prev = S(IBIS_STAT_HYDRAUL, 0);
-    float suc_prev = S(IBIS_STAT_SUCTION, 0);
-    float bex_prev = S(IBIS_STAT_BEX, 0);
-#pragma unroll
-    for (int k = 1; k < NL; ++k) {
-        const float hyd = S(IBIS_STAT_HYDRAUL, k);
-        const float suc = S(IBIS_STAT_SUCTION, k);
-        const float bex = S(IBIS_STAT_BEX, k);
-        const float wp = P.sw32_wp[k], wm = P.sw32_wm[k];
-        const float a = wm * hyd_prev + wp * hyd;
-        const float b = wm * hyd_prev * suc_prev * bex_prev + wp * hyd * suc * bex;
-        const float zb = wm * bex_prev + wp * bex;
-        const int nb = (int)floorf(zb + 0.5f);
-        const int m = 2 * nb + 3;
-        const int nn = nb + 2;
-        const float ws = consistent ? wp * w[k - 1] + wm * w[k] : wm * w[k - 1] + wp * w[k];
-        const float wa = fminf(ws, 1.0f);
-        const float pw1 = ipow(wa, nn - 1);
-        float bwn1 = b * pw1;
-        float bwn = bwn1 * wa;
-        if (bwn < dmin) bwn1 = 0.0f;
-        bwn = fmaxf(bwn, dmin);
-        const float dw = (w[k] - w[k - 1]) * P.sw32_rhm[k];
-        const float wam1 = pw1 * pw1;                   // wa**(m-1) = (wa**(nn-1))**2
-        const float ek = (float)(m - 1) * a * (wam1 * wa) - (float)nn * bwn1 * wa * dw;
-        const float fk = (float)(-m) * a * wam1 + (float)nn * bwn1 * dw;
-        float zi = fmaxf(0.0f, 1.0f - fmaxf(wisoi[k - 1], wisoi[k]));
-        zi = zi * zi;
-        e[k] = zi * ek;
-        f[k] = zi * fk;
-        g[k] = zi * bwn;
-        hyd_prev = hyd; suc_prev = suc; bex_prev = bex;
-    }
-    {
-        const float wab = fminf(w[NL - 1], 1.0f);
-        const int mb = 2 * (int)floorf(bex_prev + 0.5f) + 3;
-        const float zi = fmaxf(0.0f, 1.0f - wisoi[NL - 1]);
-        e[NL] = (zi * zi) * (-hyd_prev * ipow(wab, mb) * P.bperm);
-    }
-    float lo[NL], di[NL], up[NL], r[NL], dl[NL];
-#pragma unroll
-    for (int k = 0; k < NL; ++k) {
-        const float dt = dtime / fmaxf(pflo[k] * P.hsoi[k], 1e-30f);
-        const float rhb = P.sw32_rhb[k];
-        float d1 = dt * (f[k] * P.sw32_c1[k] - g[k] * rhb);
-        float d2m, d3;                                  // d2m: the diagonal less its 1
-        if (k < NL - 1) {
-            const float rhp = P.sw32_rhp[k];
-            d2m = dt * (-f[k + 1] * P.sw32_c3[k] + f[k] * P.sw32_c5[k] + g[k + 1] * rhp + g[k] * rhb);
-            d3 = dt * (-f[k + 1] * P.sw32_c6[k] - g[k + 1] * rhp);
-        } else {
-            d2m = dt * (-f[k + 1] + f[k] * P.sw32_c5[k] + g[k] * rhb);
-            d3 = 0.0f;
-        }
-        float rk = dt * (e[k + 1] - e[k]) - d2m * w[k];
-        if (k == 0) {
-            d1 = 0.0f;
-            rk = rk + dt * (fwtop + fwpud) / rhow;
-        } else {
-            rk = rk - d1 * w[k - 1];
-        }
-        if (k < NL - 1) rk = rk - d3 * w[k + 1];
-        lo[k] = d1; di[k] = 1.0f + d2m; up[k] = d3; r[k] = rk;
-    }
-    thomas(lo, di, up, r, dl);
-    wflo[NL] = -rhow * e[NL];
-    float fsq = 0.0f;
-#pragma unroll
-    for (int k = NL - 1; k >= 0; --k) {
-        const float zz = rhow * poros[k] * fmaxf(eps, 1.0f - wisoi[k]) * P.hsoi[k];
-        float dwk = dl[k] + dtime * fsq / zz;           // w_new - w before the saturation bound
-        const float over = (w[k] - 1.0f) + dwk;         // w_new - 1
-        const float fsn = fmaxf(over, 0.0f) * zz / dtime;
-        if (over > 0.0f) dwk = 1.0f - w[k];
-        wflo[k] = wflo[k + 1] + dwk * zz / dtime;
-        w[k] = over > 0.0f ? 1.0f : w[k] + dwk;
-        fsq = fsn;
-    }
-    wpud = fmaxf(wpud + (fsq - fwpud) * dtime, 0.0f);
-    wflo[0] = wflo[0] + fsq - fwpud;
-}
-
 // ---------------------------------------------------------------------------
 // soilheat / soilheat_with_bedrock (soil_physics.py:385-490, bedrock.py:88-153)
 // NT = 6 (no bedrock) or 9; the first NL layers carry water.
 // ---------------------------------------------------------------------------
-// The soil heat solve of the FP32 kernels in increment form: the same system
-// for delta = T_new - t, whose right-hand side holds only small terms -- the
-// heat-capacity change times t, the transpired water's heat, the flux
-// divergence, and the conduction of the current temperature differences -- so
-// float32 rounds relative to the hour's change, not to the temperature.
-template <int NT>
-__device__ __forceinline__ void soil_heat_increments(float (&t)[NT], float (&hflo)[NL + 1], const float (&dtp)[NL],
-                                                     const float (&owsoi)[NL], const float (&wsoi)[NL],
-                                                     const float (&wisoi)[NL], const float (&poros)[NL],
-                                                     const float (&consoi)[NL], const float (&csoi)[NL],
-                                                     const float (&rhosoi)[NL], float c0pud0, float c1pud0,
-                                                     float fhtop, const float (&wflo)[NL + 1],
-                                                     const DevParams<float>& P) {
-    float h[NT], con[NT + 1], whf[NT + 1], c0[NT], c1[NT], dc[NT], ts[NT];
-#pragma unroll
-    for (int k = 0; k < NT; ++k) {
-        h[k] = k < NL ? P.hsoi[k] : P.hsoi_bed[k - NL];
-        ts[k] = k < NL ? t[k] + dtp[k] : t[k];      // the starting temperatures, for the advected heat
-    }
-    auto cons = [&](int k) -> float { return k < NL ? consoi[k] : P.consoi_bed; };
-    con[0] = 0.0f;
-    con[NT] = 0.0f;
-    whf[0] = wflo[0] * P.ch2o * ts[0];
-#pragma unroll
-    for (int k = 1; k < NT; ++k) {
-        con[k] = 1.0f / (0.5f * (h[k - 1] / fmaxf(cons(k - 1), 1e-12f) + h[k] / fmaxf(cons(k), 1e-12f)));
-        if (k < NL) whf[k] = wflo[k] * P.ch2o * ((h[k] * ts[k - 1] + h[k - 1] * ts[k]) / (h[k - 1] + h[k]));
-    }
-    const float drain = wflo[NL] * P.ch2o * ts[NL - 1];
-#pragma unroll
-    for (int k = NL; k <= NT; ++k) whf[k] = drain;
-#pragma unroll
-    for (int k = 0; k < NT; ++k) {
-        if (k < NL) {
-            const float r1 = (1.0f - poros[k]) * csoi[k] * rhosoi[k];
-            const float r2 = poros[k] * (1.0f - wisoi[k]) * P.ch2o * P.rhow;
-            const float r3 = poros[k] * wisoi[k] * P.cice * P.rhow;
-            c0[k] = (k == 0 ? c0pud0 : 0.0f) + (r1 + r2 * owsoi[k] + r3) * h[k];
-            c1[k] = (k == 0 ? c1pud0 : 0.0f) + (r1 + r2 * wsoi[k] + r3) * h[k];
-            dc[k] = (k == 0 ? c0pud0 - c1pud0 : 0.0f) + r2 * (owsoi[k] - wsoi[k]) * h[k];   // c0 - c1
-        } else {
-            c0[k] = c1[k] = P.csoi_bed * P.rhosoi_bed * h[k];
-            dc[k] = 0.0f;
-        }
-    }
-    float lo[NT], di[NT], up[NT], r[NT], dl[NT];
-#pragma unroll
-    for (int k = 0; k < NT; ++k) {
-        const float rw = P.dtime / c1[k];
-        lo[k] = -rw * con[k];
-        di[k] = 1.0f + rw * (con[k] + con[k + 1]);
-        up[k] = -rw * con[k + 1];
-        // (c0/c1) ts + rw (F - conduction of t) - t, term by term
-        float cond = con[k] * (t[k] - (k > 0 ? t[k - 1] : t[k]));
-        if (k + 1 < NT) cond = cond + con[k + 1] * (t[k] - t[k + 1]);
-        float flux = whf[k] - whf[k + 1] + (k == 0 ? fhtop : 0.0f);
-        r[k] = (dc[k] / c1[k]) * t[k] + (c0[k] / c1[k]) * (k < NL ? dtp[k] : 0.0f) + rw * (flux - cond);
-    }
-    thomas(lo, di, up, r, dl);
-    float s = fhtop;
-    hflo[0] = s;
-#pragma unroll
-    for (int k = 0; k < NT; ++k) {
-        // (c1 T_new - c0 ts) / dt with T_new = t + delta and ts = t + dtp
-        s = s - (c1[k] * dl[k] - dc[k] * t[k] - c0[k] * (k < NL ? dtp[k] : 0.0f)) / P.dtime;
-        if (k < NL) hflo[k + 1] = s;
-    }
-#pragma unroll
-    for (int k = 0; k < NT; ++k) t[k] = t[k] + dl[k];
-}
-
 // soilheat (soil_physics.py:385-490) or soilheat_with_bedrock (bedrock.py:88-153).
-// The FP64 kernels perform the reference's operations on absolute temperatures.
-// The FP32 kernels solve for the increments (soil_heat_increments above): on
-// absolute temperatures (~280 K, one ulp 3e-5 K) float32 rounds each hour by a
-// sizeable part of a deep layer's change (~1e-4 K), and the residue repeats
-// while a layer changes slowly -- over a year it cooled the deep column of every
-// cell by 0.03-0.09 K against the float64 kernels, and with it the runoff, ET
-// and CH4 sums drifted by up to 4e-4.
-//
 // The layers' starting temperatures are t[k] + dtp[k] (dtp: the heat of the
-// transpired water, loops.py:1008-1025), kept apart because in float32 an
-// hourly increment below half an ulp of the temperature would be dropped.
+// transpired water, loops.py:1008-1025).
 template <typename R, int NT>
 __device__ __forceinline__ void soil_heat(R (&t)[NT], R (&hflo)[NL + 1], const R (&dtp)[NL], const R (&owsoi)[NL],
                                           const R (&wsoi)[NL], const R (&wisoi)[NL], const R (&poros)[NL],
                                           const R (&consoi)[NL], const R (&csoi)[NL], const R (&rhosoi)[NL],
                                           R c0pud0, R c1pud0, R fhtop, const R (&wflo)[NL + 1],
                                           const DevParams<R>& P) {
-    if constexpr (sizeof(R) == 4) {
-        soil_heat_increments<NT>(t, hflo, dtp, owsoi, wsoi, wisoi, poros, consoi, csoi, rhosoi, c0pud0, c1pud0, fhtop,
-                                 wflo, P);
-        return;
-    }
     using D = double;
     D h[NT], con[NT + 1], whf[NT + 1], c0[NT], c1[NT], td[NT];
 #pragma unroll
@@ -436,9 +224,9 @@ __device__ __forceinline__ void soil_heat(R (&t)[NT], R (&hflo)[NL + 1], const R
     whf[0] = (D)wflo[0] * ch2o * td[0];
 #pragma unroll
     for (int k = 1; k < NT; ++k) {
-        con[k] = dv<R>(1.0, 0.5 * (dv<R>(h[k - 1], fmax(cons(k - 1), 1e-12)) + dv<R>(h[k], fmax(cons(k), 1e-12))));
+        con[k] = (1.0 / (0.5 * ((h[k - 1] / fmax(cons(k - 1), 1e-12)) + (h[k] / fmax(cons(k), 1e-12)))));
         if (k < NL) {
-            D tav = dv<R>(h[k] * td[k - 1] + h[k - 1] * td[k], h[k - 1] + h[k]);
+            D tav = ((h[k] * td[k - 1] + h[k - 1] * td[k]) / (h[k - 1] + h[k]));
             whf[k] = (D)wflo[k] * ch2o * tav;
         }
     }
@@ -467,19 +255,19 @@ __device__ __forceinline__ void soil_heat(R (&t)[NT], R (&hflo)[NL + 1], const R
     D lo[NT], di[NT], up[NT], r[NT], tn[NT];
 #pragma unroll
     for (int k = 0; k < NT; ++k) {
-        D rw = dv<R>(dtime, c1[k]);
+        D rw = (dtime / c1[k]);
         lo[k] = -rw * con[k];
         di[k] = 1.0 + rw * (con[k] + con[k + 1]);
         up[k] = -rw * con[k + 1];
-        r[k] = dv<R>(c0[k], c1[k]) * td[k] + rw * (whf[k] - whf[k + 1]);
-        if (k == 0) r[k] = r[k] + dv<R>(dtime, c1[k]) * (D)fhtop;
+        r[k] = (c0[k] / c1[k]) * td[k] + rw * (whf[k] - whf[k + 1]);
+        if (k == 0) r[k] = r[k] + (dtime / c1[k]) * (D)fhtop;
     }
     thomas(lo, di, up, r, tn);
     D s = (D)fhtop;
     hflo[0] = (R)s;
 #pragma unroll
     for (int k = 0; k < NT; ++k) {
-        s = s - dv<R>(c1[k] * tn[k] - c0[k] * td[k], dtime);
+        s = s - ((c1[k] * tn[k] - c0[k] * td[k]) / dtime);
         if (k < NL) hflo[k + 1] = (R)s;
     }
 #pragma unroll

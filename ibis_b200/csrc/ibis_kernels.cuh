@@ -121,54 +121,42 @@ __device__ __forceinline__ Forc<R> load_forc(const R* __restrict__ f, int ld) {
     return F;
 }
 
-// Accumulators of the fused kernel kept in shared memory for the launch: plane p
-// of thread t at sacc[p * BLOCK + t] (consecutive threads, consecutive banks)
-// for the kAccOnChip planes every day loop keeps, then their compensation
-// planes; the optional planes from kAccOnChip on stay in global memory.  Only
-// the planes the flags write move: loaded before the first hour, stored after
-// the last, so the hourly read-modify-writes stay on chip.
-__device__ __forceinline__ bool acc_plane_used(int p, unsigned flags) {
-    const int q = p < IBIS_ACC_COUNT ? p : p - IBIS_ACC_COUNT;
-    const bool last_value = q == IBIS_ACC_STRESSTU_LAST || q == IBIS_ACC_STRESSTL_LAST;    // no Kahan terms
-    if (p >= IBIS_ACC_COUNT && (!(flags & IBIS_FLAG_KAHAN) || last_value)) return false;
-    if (q == IBIS_ACC_CH4) return (flags & IBIS_FLAG_CH4) != 0;
-    if (q >= IBIS_ACC_TSOI_MEAN && q < IBIS_ACC_AFSENA) return (flags & IBIS_FLAG_SOIL_MEANS) != 0;
-    if (q >= IBIS_ACC_ET_TRANS && q <= IBIS_ACC_ET_SNOWSUB)
-        return (flags & IBIS_FLAG_ACC) && (flags & IBIS_FLAG_ETPARTS);
-    if (q == IBIS_ACC_NEE_NIGHT || q == IBIS_ACC_NEE_DAY)
-        return (flags & IBIS_FLAG_ACC) && (flags & IBIS_FLAG_NEEPARTS);
-    return (flags & IBIS_FLAG_ACC) != 0;
-}
-
-// The planes move in batches of kAccMoveBatch: all loads of a batch are issued
-// before its stores, so a thread has that many global loads in flight instead
-// of waiting out one load latency per plane at the start of every launch.
-constexpr int kAccMoveBatch = 16;
-
-template <typename R, bool TO_SMEM>
-__device__ __forceinline__ void acc_move(R* __restrict__ g, int ld, R* __restrict__ sacc, int sld, unsigned flags) {
-    constexpr int kPlanes = 2 * kAccOnChip;
-    auto global_plane = [](int p) { return p < kAccOnChip ? p : p - kAccOnChip + IBIS_ACC_COUNT; };
-#pragma unroll 1
-    for (int p0 = 0; p0 < kPlanes; p0 += kAccMoveBatch) {
-        R v[kAccMoveBatch];
-        bool use[kAccMoveBatch];
+// Accumulators of the fused kernel kept in shared memory for the launch (Acc's
+// on-chip form): the slots the flags write are loaded before the first hour and
+// stored after the last, so the hourly read-modify-writes stay on chip.  All loads
+// are issued before the stores, so a launch waits out one memory latency.
+template <bool TO_SMEM>
+__device__ __forceinline__ void acc_move(float* __restrict__ g, int ld, float2* __restrict__ chip, int sld,
+                                         unsigned flags) {
+    const bool sums = (flags & IBIS_FLAG_ACC) != 0, ch4 = (flags & IBIS_FLAG_CH4) != 0;
+    const bool kahan = (flags & IBIS_FLAG_KAHAN) != 0;
+    float v[2][2 * kAccPairs];
 #pragma unroll
-        for (int j = 0; j < kAccMoveBatch; ++j) {
-            const int p = p0 + j;
-            use[j] = p < kPlanes && acc_plane_used(global_plane(p), flags);
-            if (TO_SMEM) v[j] = use[j] ? g[(size_t)global_plane(p) * ld] : R(0.0);
-            else v[j] = use[j] ? sacc[p * sld] : R(0.0);
-        }
+    for (int c = 0; c < 2; ++c) {
 #pragma unroll
-        for (int j = 0; j < kAccMoveBatch; ++j) {
-            const int p = p0 + j;
-            if (!use[j]) continue;
-            if (TO_SMEM) sacc[p * sld] = v[j];
-            else g[(size_t)global_plane(p) * ld] = v[j];
+        for (int s = 0; s < 2 * kAccPairs; ++s) {
+            const bool use = s < kAccSlots && (acc_slot_plane(s) == IBIS_ACC_CH4 ? ch4 : sums) &&
+                             (c == 0 || kahan);
+            float* const p = g + (size_t)(acc_slot_plane(s) + c * IBIS_ACC_COUNT) * ld;
+            if constexpr (TO_SMEM) {
+                v[c][s] = use ? *p : 0.0f;
+            } else if (use) {
+                const float2 w = chip[(c * kAccPairs + s / 2) * sld];
+                *p = s & 1 ? w.y : w.x;
+            }
         }
     }
+    if constexpr (TO_SMEM) {
+#pragma unroll
+        for (int c = 0; c < 2; ++c)
+#pragma unroll
+            for (int j = 0; j < kAccPairs; ++j)
+                chip[(c * kAccPairs + j) * sld] = make_float2(v[c][2 * j], v[c][2 * j + 1]);
+    }
 }
+
+// Bytes of shared memory per thread the on-chip accumulators take
+constexpr size_t kAccChipBytes = 2 * kAccPairs * sizeof(float2);
 
 // Whether a fused configuration keeps its accumulators in shared memory: the
 // column state plus the on-chip accumulator planes of MINB resident blocks must fit
@@ -180,7 +168,7 @@ template <typename R, int BLOCK, int MINB, bool ACCSM = true>
 struct AccInSmem {
     static constexpr bool value =
         ACCSM && StateInSmem<R>::value &&
-        ((sizeof(Col<R>) + 2 * kAccOnChip * sizeof(R)) * BLOCK + 1024) * MINB <= 228 * 1024;
+        ((sizeof(Col<R>) + kAccChipBytes) * BLOCK + 1024) * MINB <= 228 * 1024;
 };
 constexpr int kAccSmemMinSteps = 4;
 
@@ -194,7 +182,8 @@ __device__ __forceinline__ auto uniform_source(const DevParams<R>& P) {
 
 // Status word written by the kernels: [0] bit 0 = a column left the step with a
 // non-finite prognostic value; [1] = smallest such cell index (INT_MAX if none).
-template <typename R, int NT, bool SU, bool SL, int BLOCK, int MINB, bool ACCSM, bool X3>
+// DG: whether the kernel can write diagnostics.
+template <typename R, int NT, bool SU, bool SL, int BLOCK, int MINB, bool ACCSM, bool X3, bool DG>
 __global__ void __launch_bounds__(BLOCK, MINB) hourly_step_kernel(R* __restrict__ prog, const R* __restrict__ stat,
                                                              const R* __restrict__ forc, R* __restrict__ diag,
                                                              R* __restrict__ acc, int ncell, int ld, int nstep,
@@ -210,22 +199,22 @@ __global__ void __launch_bounds__(BLOCK, MINB) hourly_step_kernel(R* __restrict_
     Col<R>& c = *cp;
     load_col(c, prog + i, ld);
     Stat<R> S{stat + i, ld};
-    Diag<R> D{diag ? diag + i : nullptr, ld};
+    const Diag<R, DG> D{DG && diag ? diag + i : nullptr, ld};
     constexpr bool kAccSmem = AccInSmem<R, BLOCK, MINB, ACCSM>::value;
-    // with the accumulators on chip the view always points at shared memory
-    // (acc == nullptr comes with no accumulator flags, so nothing is added)
-    R* const sacc = kAccSmem ? reinterpret_cast<R*>(smem_raw + BLOCK * sizeof(Col<R>)) + threadIdx.x : nullptr;
-    const bool kahan = (P.flags & IBIS_FLAG_KAHAN) != 0;
-    using AccT = Acc<R, kAccSmem ? BLOCK : 0>;
-    AccT A = kAccSmem ? AccT{sacc, ld, kahan, true, acc ? acc + i : nullptr} : AccT{acc ? acc + i : nullptr, ld, kahan};
-    if (kAccSmem && acc) acc_move<R, true>(acc + i, ld, sacc, BLOCK, P.flags);
+    Acc<R, kAccSmem ? BLOCK : 0> A{acc ? acc + i : nullptr, ld, (P.flags & IBIS_FLAG_KAHAN) != 0};
+    if constexpr (kAccSmem) {
+        A.chip = reinterpret_cast<float2*>(smem_raw + BLOCK * sizeof(Col<R>)) + threadIdx.x;
+        if (acc) acc_move<true>(acc + i, ld, A.chip, BLOCK, P.flags);
+    }
 #pragma unroll 1
     for (int s = 0; s < nstep; ++s) {
         Forc<R> F = load_forc(forc + (size_t)s * forc_stride + i, ld);
         A.last = (s + 1 == nstep);
         column_step<R, NT, SU, SL>(c, F, S, D, A, P, uniform_source<R, X3>(P));
     }
-    if (kAccSmem && acc) acc_move<R, false>(acc + i, ld, sacc, BLOCK, P.flags);
+    if constexpr (kAccSmem) {
+        if (acc) acc_move<false>(acc + i, ld, A.chip, BLOCK, P.flags);
+    }
     R sum = store_col(c, prog + i, ld);
     if (status && !finite(sum)) {
         atomicOr(status, 1);
@@ -325,7 +314,7 @@ __device__ __forceinline__ Forc<R> read_forc_tile(const R* t, int block) {
 template <typename R, int BLOCK, int MINB>
 struct StagedSmem {
     static constexpr size_t col = (size_t)BLOCK * sizeof(Col<R>);
-    static constexpr size_t acc = (size_t)BLOCK * 2 * kAccOnChip * sizeof(R);
+    static constexpr size_t acc = (size_t)BLOCK * kAccChipBytes;
     static constexpr size_t stage_off = (col + acc + 15) / 16 * 16;
     static constexpr size_t total = stage_off + ForcStage<R, BLOCK>::bytes;
 };
@@ -340,9 +329,8 @@ __device__ __forceinline__ void stage_give_up(volatile int* abort_word, int* sta
 
 template <typename R, int NT, bool SU, bool SL, int BLOCK, int MINB, bool X3>
 __global__ void __launch_bounds__(BLOCK, MINB) hourly_step_staged_kernel(
-    R* __restrict__ prog, const R* __restrict__ stat, const R* __restrict__ forc, R* __restrict__ diag,
-    R* __restrict__ acc, int ncell, int ld, int nstep, long long forc_stride, const DevParams<R> P,
-    int* __restrict__ status) {
+    R* __restrict__ prog, const R* __restrict__ stat, const R* __restrict__ forc, R* __restrict__ acc, int ncell,
+    int ld, int nstep, long long forc_stride, const DevParams<R> P, int* __restrict__ status) {
     static_assert(sizeof(R) == 4 && StateInSmem<R>::value, "the staged form is the FP32 shared-memory kernel");
     static_assert(AccInSmem<R, BLOCK, MINB>::value, "the staged form keeps the accumulators on chip");
     using SM = StagedSmem<R, BLOCK, MINB>;
@@ -377,12 +365,10 @@ __global__ void __launch_bounds__(BLOCK, MINB) hourly_step_staged_kernel(
     Col<R>& c = *(reinterpret_cast<Col<R>*>(smem_raw) + threadIdx.x);
     load_col(c, prog + i, ld);
     Stat<R> S{stat + i, ld};
-    Diag<R> D{diag ? diag + i : nullptr, ld};
-    R* const sacc = reinterpret_cast<R*>(smem_raw + SM::col) + threadIdx.x;
-    const bool kahan = (P.flags & IBIS_FLAG_KAHAN) != 0;
-    using AccT = Acc<R, BLOCK>;
-    AccT A{sacc, ld, kahan, true, acc ? acc + i : nullptr};
-    if (acc) acc_move<R, true>(acc + i, ld, sacc, BLOCK, P.flags);
+    const Diag<R, false> D{nullptr, ld};
+    Acc<R, BLOCK> A{acc ? acc + i : nullptr, ld, (P.flags & IBIS_FLAG_KAHAN) != 0};
+    A.chip = reinterpret_cast<float2*>(smem_raw + SM::col) + threadIdx.x;
+    if (acc) acc_move<true>(acc + i, ld, A.chip, BLOCK, P.flags);
 #pragma unroll 1
     for (int s = 0; s < nstep; ++s) {
         const unsigned parity = (unsigned)(s & 1);
@@ -400,7 +386,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) hourly_step_staged_kernel(
         A.last = (s + 1 == nstep);
         column_step<R, NT, SU, SL>(c, F, S, D, A, P, uniform_source<R, X3>(P));
     }
-    if (acc) acc_move<R, false>(acc + i, ld, sacc, BLOCK, P.flags);
+    if (acc) acc_move<false>(acc + i, ld, A.chip, BLOCK, P.flags);
     R sum = store_col(c, prog + i, ld);
     if (threadIdx.x == 0 && *abort_word) {
         // after a give-up the last copy may still be landing: let it finish
@@ -417,7 +403,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) hourly_step_staged_kernel(
 // Two-kernel form of one hour: the surface phase writes the hand-off values to
 // `mid` (kMidCount planes), the ground phase reads them.  Both phases load the
 // column from `prog` and write back what they change.
-template <typename R, bool SU, bool SL, int BLOCK, int MINB, bool X3>
+template <typename R, bool SU, bool SL, int BLOCK, int MINB, bool X3, bool DG>
 __global__ void __launch_bounds__(BLOCK, MINB) surface_kernel(R* __restrict__ prog, const R* __restrict__ stat,
                                                                     const R* __restrict__ forc, R* __restrict__ diag,
                                                                     R* __restrict__ mid, int ncell, int ld,
@@ -432,15 +418,16 @@ __global__ void __launch_bounds__(BLOCK, MINB) surface_kernel(R* __restrict__ pr
     Col<R>& c = *cp;
     load_col(c, prog + i, ld);
     Stat<R> S{stat + i, ld};
-    Diag<R> D{diag ? diag + i : nullptr, ld};
+    const Diag<R, DG> D{DG && diag ? diag + i : nullptr, ld};
     Forc<R> F = load_forc(forc + i, ld);
     Mid<R> M;
-    surface_phase<R, SU, SL>(c, F, S, D, P, uniform_source<R, X3>(P), M);
+    SoilHour G;      // formed again by the ground kernel
+    surface_phase32<SU, SL>(c, F, S, D, P, uniform_source<R, X3>(P), M, G);
     mid_store(M, mid + i, ld);
     store_col(c, prog + i, ld);
 }
 
-template <typename R, int NT, int BLOCK, int MINB, bool X3>
+template <typename R, int NT, int BLOCK, int MINB, bool X3, bool DG>
 __global__ void __launch_bounds__(BLOCK, MINB) ground_kernel(R* __restrict__ prog, const R* __restrict__ stat,
                                                                    const R* __restrict__ forc, R* __restrict__ diag,
                                                                    R* __restrict__ acc, const R* __restrict__ mid,
@@ -456,12 +443,14 @@ __global__ void __launch_bounds__(BLOCK, MINB) ground_kernel(R* __restrict__ pro
     Col<R>& c = *cp;
     load_col(c, prog + i, ld);
     Stat<R> S{stat + i, ld};
-    Diag<R> D{diag ? diag + i : nullptr, ld};
+    const Diag<R, DG> D{DG && diag ? diag + i : nullptr, ld};
     Acc<R> A{acc ? acc + i : nullptr, ld, (P.flags & IBIS_FLAG_KAHAN) != 0};
     Forc<R> F = load_forc(forc + i, ld);
     Mid<R> M;
     mid_load(M, mid + i, ld);
-    ground_phase<R, NT>(c, F, S, D, A, P, uniform_source<R, X3>(P), M);
+    SoilHour G;
+    soil_hour32(G, c, F, S, P, uniform_source<R, X3>(P));
+    ground_phase32<NT>(c, F, S, D, A, P, uniform_source<R, X3>(P), M, G);
     R sum = store_col(c, prog + i, ld);
     if (status && !finite(sum)) {
         atomicOr(status, 1);
@@ -503,22 +492,38 @@ static DevParams<R> make_dev_params(const IbisParams& h) {
         double hp = k < NL - 1 ? 0.5 * (h.hsoi[k] + h.hsoi[k + 1]) : 1.0;
         d.sw_hp[k] = hp > 1e-30 ? hp : 1e-30;
         const int km1 = k > 0 ? k - 1 : 0, kp1 = k < NL - 1 ? k + 1 : k;
-        d.sw_rhm[k] = k > 0 ? 1.0 / d.sw_hm[k] : 0.0;
-        d.sw_rhb[k] = 1.0 / d.sw_hb[k];
-        d.sw_rhp[k] = 1.0 / d.sw_hp[k];
-        d.sw_c1[k] = 0.5 * h.hsoi[k] / d.sw_hb[k];
-        d.sw_c3[k] = 0.5 * h.hsoi[kp1] / d.sw_hp[k];
-        d.sw_c5[k] = 0.5 * h.hsoi[km1] / d.sw_hb[k];
-        d.sw_c6[k] = 0.5 * h.hsoi[k] / d.sw_hp[k];
+        d.sw32_wp[k] = (float)d.sw_wp[k];
+        d.sw32_wm[k] = (float)d.sw_wm[k];
+        d.sw32_rhm[k] = k > 0 ? (float)(1.0 / d.sw_hm[k]) : 0.0f;
+        d.sw32_rhb[k] = (float)(1.0 / d.sw_hb[k]);
+        d.sw32_rhp[k] = (float)(1.0 / d.sw_hp[k]);
+        d.sw32_c1[k] = (float)(0.5 * h.hsoi[k] / d.sw_hb[k]);
+        d.sw32_c3[k] = (float)(0.5 * h.hsoi[kp1] / d.sw_hp[k]);
+        d.sw32_c5[k] = (float)(0.5 * h.hsoi[km1] / d.sw_hb[k]);
+        d.sw32_c6[k] = (float)(0.5 * h.hsoi[k] / d.sw_hp[k]);
+    }
+    const double drip[3] = {h.tdripu, h.tdrips, h.tdripl}, blow[3] = {h.tblowu, h.tblows, h.tblowl};
+    for (int k = 0; k < 3; ++k) {
+        d.rtdrip[k] = (R)(1.0 / drip[k]);
+        d.rtblow[k] = (R)(1.0 / blow[k]);
+        d.kdrip[k] = (R)(1.0 - h.dtime / drip[k]);
+        d.kblow[k] = (R)(1.0 - h.dtime / blow[k]);
+    }
+    d.rtheta3 = (R)(1.0 / h.theta3);
+    d.rbeta3 = (R)(1.0 / h.beta3);
+    d.rtheta4 = (R)(1.0 / h.theta4);
+    d.rbeta4 = (R)(1.0 / h.beta4);
+    for (int k = 1; k < NL; ++k) {
+        d.hs_below[k] = (R)(h.hsoi[k] / (h.hsoi[k - 1] + h.hsoi[k]));
+        d.hs_above[k] = (R)(h.hsoi[k - 1] / (h.hsoi[k - 1] + h.hsoi[k]));
+    }
+    const double cbed = h.consoi_bed > 1e-12 ? h.consoi_bed : 1e-12;
+    for (int k = 0; k < NB; ++k) {
+        d.bed_res[k] = (R)(0.5 * h.hsoi_bed[k] / cbed);
+        d.bed_con[k] = k + 1 < NB ? (R)(1.0 / (0.5 * (h.hsoi_bed[k] + h.hsoi_bed[k + 1]) / cbed)) : (R)0.0;
+        d.bed_rw[k] = (R)(h.dtime / (h.csoi_bed * h.rhosoi_bed * h.hsoi_bed[k]));
     }
     d.rdt64 = 1.0 / h.dtime;
-    d.rrhow64 = 1.0 / h.rhow;
-    for (int k = 0; k < NL; ++k) {
-        d.sw32_wp[k] = (float)d.sw_wp[k]; d.sw32_wm[k] = (float)d.sw_wm[k];
-        d.sw32_rhm[k] = (float)d.sw_rhm[k]; d.sw32_rhb[k] = (float)d.sw_rhb[k]; d.sw32_rhp[k] = (float)d.sw_rhp[k];
-        d.sw32_c1[k] = (float)d.sw_c1[k]; d.sw32_c3[k] = (float)d.sw_c3[k];
-        d.sw32_c5[k] = (float)d.sw_c5[k]; d.sw32_c6[k] = (float)d.sw_c6[k];
-    }
     // respiration tables formed in float32 as the reference does (loops_gswp3.py:185-190)
     const float per_s = (float)(h.ndaypy * 86400.0), mol = (float)(1000.0 / 12.0);
     for (int j = 0; j < 12; ++j) {
@@ -601,14 +606,14 @@ cudaError_t fit_smem_once(unsigned long long& done, K k, int block, size_t smem,
     return e;
 }
 
-template <typename R, int NT, bool SU, bool SL, int BLOCK, int MINB, bool ACCSM, bool X3>
+template <typename R, int NT, bool SU, bool SL, int BLOCK, int MINB, bool ACCSM, bool X3, bool DG>
 cudaError_t launch_fused(R* prog, const R* stat, const R* forc, R* diag, R* acc, int ncell, int ld, int nstep,
                          long long fstride, const DevParams<R>& P, int* status, cudaStream_t s) {
     const int grid = (ncell + BLOCK - 1) / BLOCK;
     const size_t col_smem = StateInSmem<R>::value ? BLOCK * sizeof(Col<R>) : 0;
-    const size_t acc_smem = AccInSmem<R, BLOCK, MINB, ACCSM>::value ? BLOCK * 2 * kAccOnChip * sizeof(R) : 0;
+    const size_t acc_smem = AccInSmem<R, BLOCK, MINB, ACCSM>::value ? BLOCK * kAccChipBytes : 0;
     const size_t smem = col_smem + acc_smem;
-    auto k = hourly_step_kernel<R, NT, SU, SL, BLOCK, MINB, ACCSM, X3>;
+    auto k = hourly_step_kernel<R, NT, SU, SL, BLOCK, MINB, ACCSM, X3, DG>;
     static unsigned long long fitted = 0;
     cudaError_t e = fit_smem_once(fitted, k, BLOCK, col_smem + acc_smem, col_smem + acc_smem);
     if (e != cudaSuccess) return e;
@@ -621,29 +626,29 @@ cudaError_t launch_fused(R* prog, const R* stat, const R* forc, R* diag, R* acc,
 // cells) runs the unstaged kernel of the same block size instead: the results
 // are the same, only the loads differ.
 template <typename R, int NT, bool SU, bool SL, int BLOCK, int MINB, bool X3>
-cudaError_t launch_staged(R* prog, const R* stat, const R* forc, R* diag, R* acc, int ncell, int ld, int nstep,
+cudaError_t launch_staged(R* prog, const R* stat, const R* forc, R* acc, int ncell, int ld, int nstep,
                           long long fstride, const DevParams<R>& P, int* status, cudaStream_t s) {
     if ((reinterpret_cast<uintptr_t>(forc) & 15) != 0 || (fstride & 3) != 0 || (ld & 3) != 0)
-        return launch_fused<R, NT, SU, SL, BLOCK, MINB, true, X3>(prog, stat, forc, diag, acc, ncell, ld, nstep,
-                                                                  fstride, P, status, s);
+        return launch_fused<R, NT, SU, SL, BLOCK, MINB, true, X3, false>(prog, stat, forc, nullptr, acc, ncell, ld,
+                                                                         nstep, fstride, P, status, s);
     using SM = StagedSmem<R, BLOCK, MINB>;
     const int grid = (ncell + BLOCK - 1) / BLOCK;
     auto k = hourly_step_staged_kernel<R, NT, SU, SL, BLOCK, MINB, X3>;
     static unsigned long long fitted = 0;
     cudaError_t e = fit_smem_once(fitted, k, BLOCK, SM::total, SM::total);
     if (e != cudaSuccess) return e;
-    k<<<grid, BLOCK, SM::total, s>>>(prog, stat, forc, diag, acc, ncell, ld, nstep, fstride, P, status);
+    k<<<grid, BLOCK, SM::total, s>>>(prog, stat, forc, acc, ncell, ld, nstep, fstride, P, status);
     return cudaGetLastError();
 }
 
-template <typename R, int NT, bool SU, bool SL, int B1, int M1, int B2, int M2, bool X3>
+template <typename R, int NT, bool SU, bool SL, int B1, int M1, int B2, int M2, bool X3, bool DG>
 cudaError_t launch_split(R* prog, const R* stat, const R* forc, R* diag, R* acc, R* mid, int ncell, int ld,
                          int nstep, long long fstride, const DevParams<R>& P, int* status, cudaStream_t s) {
     const int g1 = (ncell + B1 - 1) / B1, g2 = (ncell + B2 - 1) / B2;
     const size_t sm1 = StateInSmem<R>::value ? B1 * sizeof(Col<R>) : 0;
     const size_t sm2 = StateInSmem<R>::value ? B2 * sizeof(Col<R>) : 0;
-    auto k1 = surface_kernel<R, SU, SL, B1, M1, X3>;
-    auto k2 = ground_kernel<R, NT, B2, M2, X3>;
+    auto k1 = surface_kernel<R, SU, SL, B1, M1, X3, DG>;
+    auto k2 = ground_kernel<R, NT, B2, M2, X3, DG>;
     static unsigned long long fitted1 = 0, fitted2 = 0;
     cudaError_t e = fit_smem_once(fitted1, k1, B1, sm1, sm1);
     if (e == cudaSuccess) e = fit_smem_once(fitted2, k2, B2, sm2, sm2);
@@ -656,26 +661,40 @@ cudaError_t launch_split(R* prog, const R* stat, const R* forc, R* diag, R* acc,
     return cudaGetLastError();
 }
 
+// Launches that write diagnostics run the default configuration of their form
+// (dispatch_config), the only ones compiled with the diagnostics writer; the
+// float64 kernels always carry it.
 template <typename R, int NT, bool SU, bool SL, int CFG, bool X3 = false>
 cudaError_t run_config(R* prog, const R* stat, const R* forc, R* diag, R* acc, R* mid, int ncell, int ld, int nstep,
                        long long fs, const DevParams<R>& P, int* status, cudaStream_t s) {
     constexpr LaunchConfig C = kConfigs[CFG];
-    if constexpr (C.form == 0) {
+    if constexpr (sizeof(R) == 8) {
+        return launch_fused<R, NT, SU, SL, C.block, C.minb, false, X3, true>(prog, stat, forc, diag, acc, ncell, ld,
+                                                                             nstep, fs, P, status, s);
+    } else if constexpr (C.form == 0) {
+#define IBIS_FUSED(ACCSM, DG)                                                                                       \
+    launch_fused<R, NT, SU, SL, C.block, C.minb, ACCSM, X3, DG>(prog, stat, forc, diag, acc, ncell, ld, nstep, fs, P, \
+                                                                status, s)
         // the default fused configuration (the plain entry points' and the
         // per-hour callers') also has a global-accumulator twin for short launches
-        if constexpr (CFG == kDefaultFused && AccInSmem<R, C.block, C.minb>::value) {
-            if (nstep < kAccSmemMinSteps)
-                return launch_fused<R, NT, SU, SL, C.block, C.minb, false, X3>(prog, stat, forc, diag, acc, ncell,
-                                                                               ld, nstep, fs, P, status, s);
+        if constexpr (CFG == kDefaultFused) {
+            if (diag) return nstep < kAccSmemMinSteps ? IBIS_FUSED(false, true) : IBIS_FUSED(true, true);
+            if (nstep < kAccSmemMinSteps) return IBIS_FUSED(false, false);
         }
-        return launch_fused<R, NT, SU, SL, C.block, C.minb, true, X3>(prog, stat, forc, diag, acc, ncell, ld, nstep,
-                                                                      fs, P, status, s);
+        return IBIS_FUSED(true, false);
+#undef IBIS_FUSED
     } else if constexpr (C.form == 2) {
-        return launch_staged<R, NT, SU, SL, C.block, C.minb, X3>(prog, stat, forc, diag, acc, ncell, ld, nstep, fs, P,
-                                                                 status, s);
+        return launch_staged<R, NT, SU, SL, C.block, C.minb, X3>(prog, stat, forc, acc, ncell, ld, nstep, fs, P, status,
+                                                                 s);
     } else {
-        return launch_split<R, NT, SU, SL, C.block, C.minb, C.block2, C.minb2, X3>(prog, stat, forc, diag, acc, mid,
-                                                                                  ncell, ld, nstep, fs, P, status, s);
+#define IBIS_SPLIT(DG)                                                                                              \
+    launch_split<R, NT, SU, SL, C.block, C.minb, C.block2, C.minb2, X3, DG>(prog, stat, forc, diag, acc, mid, ncell, ld, \
+                                                                            nstep, fs, P, status, s)
+        if constexpr (CFG == kDefaultSplit) {
+            if (diag) return IBIS_SPLIT(true);
+        }
+        return IBIS_SPLIT(false);
+#undef IBIS_SPLIT
     }
 }
 
@@ -708,6 +727,10 @@ cudaError_t dispatch_config(int cfg, R* prog, const R* stat, const R* forc, R* d
         // the float64 kernels always carry the IBIS 3.0 extensions: with their
         // switches off they perform the F77 step's operations
         return run_config<R, NT, SU, SL, kDefaultFused, true>(IBIS_ARGS);
+    } else if (diag) {
+        // only the default configurations are compiled with the diagnostics writer
+        if (kConfigs[cfg].form != 1) return run_config<R, NT, SU, SL, kDefaultFused, X3>(IBIS_ARGS);
+        return run_config<R, NT, SU, SL, kDefaultSplit, X3>(IBIS_ARGS);
     } else if constexpr (X3) {
         if (cfg == kLongFused && SU == SL) return run_config<R, NT, SU, SL, kLongFused, true>(IBIS_ARGS);
         if (kConfigs[cfg].form != 1) return run_config<R, NT, SU, SL, kDefaultFused, true>(IBIS_ARGS);

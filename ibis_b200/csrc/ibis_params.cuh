@@ -22,20 +22,16 @@ struct DevParams {
     R znorm;           // 1 - exp(stressfac) (stomata.py:545)
     R rdt;             // 1 / dtime
     R zir;             // 4 * 0.95 * stef (loops.py:170; canopy_exchange.py:566)
-    // soil-water solve geometry, always double (soil_physics.py:238-330)
+    // soil-water solve geometry in double (soil_physics.py:238-330)
     double sw_hm[6];   // interface k (1..5): 0.5 * (h[k-1] + h[k])
     double sw_wp[6];   // 0.5 * h[k] / sw_hm[k]
     double sw_wm[6];   // 1 - sw_wp[k]
     double sw_hb[6];   // row k: max(0.5 h[0] | 0.5 h[k-1] + 0.5 h[k], 1e-30)
     double sw_hp[6];   // row k < 5: max(0.5 * (h[k] + h[k+1]), 1e-30)
-    // the same geometry as multipliers, so the solve divides only by values
-    // that change per cell: 1/sw_hm, 1/sw_hb, 1/sw_hp, 0.5 h[k]/sw_hb,
-    // 0.5 h[k+1]/sw_hp, 0.5 h[k-1]/sw_hb, 0.5 h[k]/sw_hp
-    double sw_rhm[6], sw_rhb[6], sw_rhp[6], sw_c1[6], sw_c3[6], sw_c5[6], sw_c6[6];
     double rdt64;      // 1 / dtime in double
-    double rrhow64;    // 1 / rhow in double
-    // float copies of sw_wp, sw_wm and the multipliers, for the FP32 kernels'
-    // increment-form soil-water solve
+    // the same geometry in float as multipliers, for the FP32 kernels' increment-form
+    // solve: sw_wp, sw_wm, 1/sw_hm, 1/sw_hb, 1/sw_hp, 0.5 h[k]/sw_hb, 0.5 h[k+1]/sw_hp,
+    // 0.5 h[k-1]/sw_hb, 0.5 h[k]/sw_hp
     float sw32_wp[6], sw32_wm[6], sw32_rhm[6], sw32_rhb[6], sw32_rhp[6], sw32_c1[6], sw32_c3[6], sw32_c5[6],
         sw32_c6[6];
     R rwood_s[12], rroot_s[12], keep[12];  // float32-formed respiration rates (loops_gswp3.py:185-190)
@@ -51,6 +47,14 @@ struct DevParams {
     // index of the launch's first column in the caller's numbering: a launch
     // over a group of columns (ibis_step_host_f32) reports status[1] in it
     int cell0;
+    // reciprocals and geometry the FP32 step multiplies by (formed in double on the host)
+    R rtdrip[3], rtblow[3];  // 1 / drip and blow-off times of the upper leaves, upper stems, lower canopy
+    R kdrip[3], kblow[3];    // 1 - dtime / time
+    R rtheta3, rbeta3, rtheta4, rbeta4;
+    R hs_below[6], hs_above[6];   // interface k (1..5): h[k] and h[k-1] over h[k-1] + h[k]
+    R bed_res[3];            // bedrock layer: half its thermal resistance
+    R bed_con[3];            // conductance to the layer below
+    R bed_rw[3];             // dtime over the heat capacity
     // per-band thickness weights of the wetland water-table average and their
     // sums (IBIS_FLAG_CH4_BANDS: from ch4b_z_wt_ref as ch4_wtop from z_wt_ref)
     R ch4b_wtop[3][6];

@@ -1,102 +1,11 @@
 // The hourly step of one column: timestep_body followed by the day-loop
-// accumulators (reference loops.py:234-1284, loops_gswp3.py:161-318).
+// accumulators (reference loops.py:234-1284, loops_gswp3.py:161-318).  The phases
+// here are the float64 kernels'; the FP32 kernels' are in ibis_f32.cuh.
 #pragma once
-#include "ibis_canopy.cuh"
-#include "ibis_ground.cuh"
+#include "ibis_f32.cuh"
+#include "ibis_phase.cuh"
 
 namespace ibis {
-
-// Planes below kAccOnChip are the accumulators every day loop keeps; the
-// planes from kAccOnChip on (the optional ET and NEE components) are summed
-// only under their own flags.  A kernel that holds the accumulators on chip
-// holds the first kind and leaves the second in the global buffer.
-constexpr int kAccOnChip = IBIS_ACC_ET_TRANS;
-static_assert(IBIS_ACC_NEE_DAY + 1 == IBIS_ACC_COUNT && IBIS_ACC_STRESSTL_LAST < kAccOnChip,
-              "the optional accumulator planes close the accumulator block");
-
-// Accumulator view of one cell: value planes then compensation planes.  In
-// the global form (SLD = 0) ``base`` addresses every plane with leading
-// dimension ``ld`` and the compensation term of plane p is plane
-// p + IBIS_ACC_COUNT.  In the on-chip form (SLD = the block size) ``base``
-// holds planes [0, kAccOnChip) with stride SLD and their compensation terms at
-// p + kAccOnChip; the optional planes stay in the global buffer ``far``
-// (leading dimension ``ld``).
-template <typename R, int SLD = 0>
-struct Acc {
-    R* __restrict__ base;  // nullptr: no accumulators
-    int ld;
-    bool kahan;
-    bool last = true;      // the launch's last hour for this cell: keep the end-of-hour values
-    R* __restrict__ far = nullptr;
-    __device__ __forceinline__ R& at(int plane) const {
-        if constexpr (SLD > 0) {
-            if (plane >= kAccOnChip) return far[(size_t)plane * ld];
-            return base[plane * SLD];
-        } else {
-            return base[(size_t)plane * ld];
-        }
-    }
-    __device__ __forceinline__ R& comp(int plane) const {
-        if constexpr (SLD > 0) {
-            if (plane >= kAccOnChip) return far[(size_t)(plane + IBIS_ACC_COUNT) * ld];
-            return base[(plane + kAccOnChip) * SLD];
-        } else {
-            return base[(size_t)(plane + IBIS_ACC_COUNT) * ld];
-        }
-    }
-    __device__ __forceinline__ void add(int plane, R x) const {
-        R& v = at(plane);
-        if (kahan) {
-            R& cmp = comp(plane);
-            R s = v, cc = cmp;
-            R y = x - cc;
-            R t = s + y;
-            cmp = (t - s) - y;
-            v = t;
-        } else {
-            v = v + x;
-        }
-    }
-    __device__ __forceinline__ R get(int plane) const { return at(plane); }
-};
-
-// Values the surface phase (steps 1-9 of timestep_body) hands to the ground
-// phase (steps 10-12 and the accumulators).  In the fused kernel they stay in
-// registers; the two-kernel form passes them through a scratch buffer of
-// IBIS_MID_COUNT planes.
-template <typename R>
-struct Mid {
-    R heatg, heati, fvapg, fvapi, fvaput, fvaplt, ginvap, gsuvap, gtrans;
-    R raing, traing, snowg, tsnowg, rainl, trainl, snowl, tsnowl;
-    R an_u[2], ag_u[2], an_l[3], ag_l[3];
-    R fsena;
-};
-constexpr int kMidCount = 28;
-
-template <typename R>
-__device__ __forceinline__ void mid_store(const Mid<R>& m, R* __restrict__ p, int ld) {
-    const R v[kMidCount] = {m.heatg, m.heati, m.fvapg, m.fvapi, m.fvaput, m.fvaplt, m.ginvap, m.gsuvap, m.gtrans,
-                            m.raing, m.traing, m.snowg, m.tsnowg, m.rainl, m.trainl, m.snowl, m.tsnowl,
-                            m.an_u[0], m.an_u[1], m.ag_u[0], m.ag_u[1], m.an_l[0], m.an_l[1], m.an_l[2],
-                            m.ag_l[0], m.ag_l[1], m.ag_l[2], m.fsena};
-#pragma unroll
-    for (int q = 0; q < kMidCount; ++q) p[(size_t)q * ld] = v[q];
-}
-
-template <typename R>
-__device__ __forceinline__ void mid_load(Mid<R>& m, const R* __restrict__ p, int ld) {
-    R v[kMidCount];
-#pragma unroll
-    for (int q = 0; q < kMidCount; ++q) v[q] = p[(size_t)q * ld];
-    m.heatg = v[0]; m.heati = v[1]; m.fvapg = v[2]; m.fvapi = v[3]; m.fvaput = v[4]; m.fvaplt = v[5];
-    m.ginvap = v[6]; m.gsuvap = v[7]; m.gtrans = v[8];
-    m.raing = v[9]; m.traing = v[10]; m.snowg = v[11]; m.tsnowg = v[12];
-    m.rainl = v[13]; m.trainl = v[14]; m.snowl = v[15]; m.tsnowl = v[16];
-    m.an_u[0] = v[17]; m.an_u[1] = v[18]; m.ag_u[0] = v[19]; m.ag_u[1] = v[20];
-    m.an_l[0] = v[21]; m.an_l[1] = v[22]; m.an_l[2] = v[23];
-    m.ag_l[0] = v[24]; m.ag_l[1] = v[25]; m.ag_l[2] = v[26];
-    m.fsena = v[27];
-}
 
 // setsoi (soil_physics.py:37-140): conductivity of layer k; with X3 and
 // IBIS_FLAG_FORGANIC the dry conductivity of organic solids blended in
@@ -117,48 +26,6 @@ __device__ __forceinline__ R layer_conductivity(const Col<R>& c, const Stat<R>& 
         }
     }
     return dry * pw(R(56.0), pliq) * pw(R(224.0), pice);
-}
-
-// setsoi (soil_physics.py:37-140): evaporation source fractions and latent heats
-template <typename R>
-__device__ __forceinline__ void evap_sources(const Col<R>& c, const Forc<R>& F, const DevParams<R>& P, R& q1, R& q2,
-                                             R& q3, R& q4, R& hvasug, R& hvasui) {
-    const R eps = P.epsilon;
-    {
-        R pud = c.wpud + c.wipud;
-        R zwpud = clip(P.zwpmax * pud / mx(P.wpudmax, eps), R(0.0), P.zwpmax);
-        R w0 = c.wsoi[0], i0 = c.wisoi[0];
-        R zwsoi = (R(1.0) - i0) * w0 + i0;
-        bool soilw = zwsoi >= eps, haspud = zwpud >= eps;
-        R r1 = R(1.0) / mx(zwsoi, eps);
-        R r2 = R(1.0) / mx(pud, eps);
-        q1 = soilw ? (haspud ? (R(1.0) - zwpud) * (R(1.0) - i0) * w0 * r1 : (R(1.0) - i0) * w0 * r1) : R(0.0);
-        q2 = soilw ? (haspud ? (R(1.0) - zwpud) * i0 * r1 : i0 * r1) : R(0.0);
-        bool warm = c.tsoi[0] >= P.tmelt - R(1.0e-9);
-        q3 = haspud ? zwpud * c.wpud * r2 : (soilw ? R(0.0) : (warm ? R(1.0) : R(0.0)));
-        q4 = haspud ? zwpud * c.wipud * r2 : (soilw ? R(0.0) : (warm ? R(0.0) : R(1.0)));
-        R zvap = P.hvap + P.cvap * (F.ta - P.tmelt) - P.ch2o * (c.tsoi[0] - P.tmelt);
-        R zsub = P.hsub + P.cvap * (F.ta - P.tmelt) - P.cice * (c.tsoi[0] - P.tmelt);
-        hvasug = (q1 + q3) * zvap + (q2 + q4) * zsub;
-        hvasui = P.hsub + P.cvap * (F.ta - P.tmelt) - P.cice * (c.tsno[0] - P.tmelt);
-    }
-}
-
-// capacity_shares (stomata.py:566-577) of one big leaf: the capacity-weighted
-// leaf area (floored at 1e-12), the leaf area, and whether the capacity shares apply
-template <typename R, int N, typename Q>
-__device__ __forceinline__ void capacity_group(const int (&idx)[N], const Stat<R>& S, const Q& q, R& twm, R& tf,
-                                               bool& on) {
-    R tw = R(0.0);
-    tf = R(0.0);
-#pragma unroll
-    for (int i = 0; i < N; ++i) {
-        const R f = S(IBIS_STAT_FRAC, idx[i]);
-        tw = tw + f * q.vmax(idx[i]);
-        tf = tf + f;
-    }
-    on = tw > R(1.0e-12);
-    twm = mx(tw, R(1.0e-12));
 }
 
 // drystress (stomata.py:515-562)
@@ -183,8 +50,8 @@ __device__ __forceinline__ void soil_stress(const Col<R>& c, const Stat<R>& S, c
 // three canopy passes (turcof + stomata + turvap), evaporation of intercepted
 // water, the bare-story reset and the surface fluxes (loops.py:318-674).
 // Leaves tu/ts/tl/tg unclamped in `c` (the ground phase clamps them).
-template <typename R, bool SUN_U, bool SUN_L, typename Q>
-__device__ __forceinline__ void surface_phase(Col<R>& c, const Forc<R>& F, const Stat<R>& S, const Diag<R>& D,
+template <typename R, bool SUN_U, bool SUN_L, typename Q, typename DD>
+__device__ __forceinline__ void surface_phase(Col<R>& c, const Forc<R>& F, const Stat<R>& S, const DD& D,
                                               const DevParams<R>& P, const Q& q, Mid<R>& M) {
     const R eps = P.epsilon;
     const R fi = c.fi;
@@ -330,42 +197,17 @@ __device__ __forceinline__ void surface_phase(Col<R>& c, const Forc<R>& F, const
     c.wliqu = wliqu; c.wliqs = wliqs; c.wliql = wliql;
     c.wsnou = wsnou; c.wsnos = wsnos; c.wsnol = wsnol;
 
-    // ---- diagnostics of the surface phase (loops.py:1158-1241)
-    if (D.base) {
-#pragma unroll
-        for (int j = 0; j < 2; ++j) { D.put(IBIS_DIAG_AN_UPPER, j, st.an_u[j]); D.put(IBIS_DIAG_AG_UPPER, j, st.ag_u[j]); }
-#pragma unroll
-        for (int j = 0; j < 3; ++j) { D.put(IBIS_DIAG_AN_LOWER, j, st.an_l[j]); D.put(IBIS_DIAG_AG_LOWER, j, st.ag_l[j]); }
-        D.put(IBIS_DIAG_FWETU, fwetu); D.put(IBIS_DIAG_FWETS, fwets); D.put(IBIS_DIAG_FWETL, fwetl);
-        D.put(IBIS_DIAG_RLIQU, rliqu); D.put(IBIS_DIAG_RLIQS, rliqs); D.put(IBIS_DIAG_RLIQL, rliql);
-        D.put(IBIS_DIAG_SOLU, Rd.solu); D.put(IBIS_DIAG_SOLS, Rd.sols); D.put(IBIS_DIAG_SOLL, Rd.soll);
-        D.put(IBIS_DIAG_SOLG, Rd.solg); D.put(IBIS_DIAG_SOLI, Rd.soli);
-        D.put(IBIS_DIAG_FIRU, Rd.firu); D.put(IBIS_DIAG_FIRS, Rd.firs); D.put(IBIS_DIAG_FIRL, Rd.firl);
-        D.put(IBIS_DIAG_FIRG, (R)tv.firg); D.put(IBIS_DIAG_FIRI, (R)tv.firi); D.put(IBIS_DIAG_FIRB, (R)tv.firb);
-#pragma unroll
-        for (int b = 0; b < 2; ++b) { D.put(IBIS_DIAG_ASURD, b, Rd.asurd[b]); D.put(IBIS_DIAG_ASURI, b, Rd.asuri[b]); }
-        D.put(IBIS_DIAG_TOPPARU, Rd.topparu); D.put(IBIS_DIAG_TOPPARL, Rd.topparl);
-#pragma unroll
-        for (int j = 0; j < 4; ++j) { D.put(IBIS_DIAG_SCALCOEFU, j, Rd.scu[j]); D.put(IBIS_DIAG_SCALCOEFL, j, Rd.scl[j]); }
-        D.put(IBIS_DIAG_FSENU, (R)tv.fsenu); D.put(IBIS_DIAG_FSENS, (R)tv.fsens); D.put(IBIS_DIAG_FSENL, (R)tv.fsenl);
-        D.put(IBIS_DIAG_FSENG, (R)tv.fseng); D.put(IBIS_DIAG_FSENI, (R)tv.fseni);
-        D.put(IBIS_DIAG_FVAPG, M.fvapg); D.put(IBIS_DIAG_FVAPI, M.fvapi);
-        D.put(IBIS_DIAG_RAING, C.raing); D.put(IBIS_DIAG_SNOWG, C.snowg); D.put(IBIS_DIAG_RHOA, A.rhoa);
-        D.put(IBIS_DIAG_HVASUG, hvasug); D.put(IBIS_DIAG_HVASUI, hvasui);
-        D.put(IBIS_DIAG_QGLIF, 0, q1); D.put(IBIS_DIAG_QGLIF, 1, q2); D.put(IBIS_DIAG_QGLIF, 2, q3); D.put(IBIS_DIAG_QGLIF, 3, q4);
-        D.put(IBIS_DIAG_HEATI, M.heati);
-        D.put(IBIS_DIAG_GINVAP, M.ginvap); D.put(IBIS_DIAG_GSUVAP, M.gsuvap); D.put(IBIS_DIAG_GTRANS, M.gtrans);
-        D.put(IBIS_DIAG_RAINL, C.rainl); D.put(IBIS_DIAG_SNOWL, C.snowl);
-        D.put(IBIS_DIAG_TRAINL, C.trainl); D.put(IBIS_DIAG_TSNOWL, C.tsnowl);
-        D.put(IBIS_DIAG_FSENA, M.fsena);
-    }
+    if (D.on())
+        surface_diagnostics(D, st, fwetu, fwets, fwetl, rliqu, rliqs, rliql, Rd, (R)tv.firg, (R)tv.firi, (R)tv.firb,
+                            (R)tv.fsenu, (R)tv.fsens, (R)tv.fsenl, (R)tv.fseng, (R)tv.fseni, M, A.rhoa, hvasug, hvasui,
+                            q1, q2, q3, q4);
 }
 
 // Steps 10-12 of timestep_body -- snow, soil water and heat (+ bedrock),
 // freeze/thaw, the surface-temperature bound -- then the fire counters and the
 // day-loop accumulators (loops.py:676-1275; loops_gswp3.py:161-318).
-template <typename R, int NT, typename Q, int SLD>
-__device__ __forceinline__ void ground_phase(Col<R>& c, const Forc<R>& F, const Stat<R>& S, const Diag<R>& D,
+template <typename R, int NT, typename Q, typename DD, int SLD>
+__device__ __forceinline__ void ground_phase(Col<R>& c, const Forc<R>& F, const Stat<R>& S, const DD& D,
                                              const Acc<R, SLD>& Ac, const DevParams<R>& P, const Q& q, const Mid<R>& M) {
     const R eps = P.epsilon, dt = P.dtime;
     const R fi = c.fi;
@@ -539,26 +381,10 @@ __device__ __forceinline__ void ground_phase(Col<R>& c, const Forc<R>& F, const 
     }
     const R fhtop_soil = heatg_avg + raing_avg * P.ch2o * (traing_avg - tpt[0])
                        - grunof * P.ch2o * mx(P.tmelt - tpt[0], R(0.0));
-    // soil water (soil_physics.py:196-373): increment form in the FP32 kernels,
-    // double in the FP64 kernels
-    R wnew[NL], wflo[NL + 1], wpud_h;
-    if constexpr (sizeof(R) == 4 && IBIS_SOILW_INCREMENTS) {
+    R wnew[NL], wflo[NL + 1], wpud_h = wpw;
 #pragma unroll
-        for (int k = 0; k < NL; ++k) wnew[k] = wsw[k];
-        wpud_h = wpw;
-        soil_water_increments(wnew, wpud_h, wflo, wisw, poros, pflo, S, fwtop, fwpud, P);
-    } else {
-        double w64[NL], i64[NL], p64[NL], pf64[NL], wf64[NL + 1];
-#pragma unroll
-        for (int k = 0; k < NL; ++k) { w64[k] = wsw[k]; i64[k] = wisw[k]; p64[k] = poros[k]; pf64[k] = pflo[k]; }
-        double wp64 = wpw;
-        soil_water(w64, wp64, wf64, i64, p64, pf64, S, (double)fwtop, (double)fwpud, P);
-#pragma unroll
-        for (int k = 0; k < NL; ++k) wnew[k] = (R)w64[k];
-#pragma unroll
-        for (int k = 0; k <= NL; ++k) wflo[k] = (R)wf64[k];
-        wpud_h = (R)wp64;
-    }
+    for (int k = 0; k < NL; ++k) wnew[k] = wsw[k];
+    soil_water(wnew, wpud_h, wflo, wisw, poros, pflo, S, fwtop, fwpud, P);
     const R c1pud0 = P.ch2o * wpud_h + P.cice * wiw;
     R hflo[NL + 1];
     // the solve starts from tsoi + dtp, the increment kept apart (soil_heat)
@@ -592,25 +418,9 @@ __device__ __forceinline__ void ground_phase(Col<R>& c, const Forc<R>& F, const 
     c.tg = clip(c.tg, lo_, hi_);
     fire_counters(c, S(IBIS_STAT_SWILT, 0), F, P);
 
-    // ---- diagnostics of the ground phase (loops.py:1158-1241)
-    if (D.base) {
-#pragma unroll
-        for (int k = 0; k < NL; ++k) {
-            D.put(IBIS_DIAG_CONSOI, k, consoi[k]);
-            D.put(IBIS_DIAG_STRESSU, k, stressu[k]);
-            D.put(IBIS_DIAG_STRESSL, k, stressl[k]);
-            D.put(IBIS_DIAG_POROSFLO, k, pflo_ft[k]);
-        }
-#pragma unroll
-        for (int k = 0; k <= NL; ++k) D.put(IBIS_DIAG_HFLO, k, hflo[k]);
-        D.put(IBIS_DIAG_HEATG, heatg_avg);
-        D.put(IBIS_DIAG_STRESSTU, stresstu); D.put(IBIS_DIAG_STRESSTL, stresstl);
-        D.put(IBIS_DIAG_GTRANSU, gtransu); D.put(IBIS_DIAG_GTRANSL, gtransl); D.put(IBIS_DIAG_GRUNOF, grunof);
-        D.put(IBIS_DIAG_GDRAIN, wflo[NL]); D.put(IBIS_DIAG_GADJUST, gadj); D.put(IBIS_DIAG_WTOT, R(0.0));
-        D.put(IBIS_DIAG_RAING_AVG, raing_avg); D.put(IBIS_DIAG_TRAING_AVG, traing_avg);
-        D.put(IBIS_DIAG_FHTOP_SOIL, fhtop_soil);
-        D.put(IBIS_DIAG_SFLO_BOT, sflo_bot); D.put(IBIS_DIAG_FHTOP_SNOW, fhtop_snow);
-    }
+    if (D.on())
+        ground_diagnostics(D, consoi, stressu, stressl, pflo_ft, hflo, heatg_avg, stresstu, stresstl, gtransu, gtransl,
+                           grunof, wflo[NL], gadj, raing_avg, traing_avg, fhtop_soil, sflo_bot, fhtop_snow);
 
     // ---- accumulators of the day loop (loops_gswp3.py:161-318)
     if (Ac.base) {
@@ -731,12 +541,18 @@ __device__ __forceinline__ void ground_phase(Col<R>& c, const Forc<R>& F, const 
 }
 
 // One full hourly step of a column in one kernel.
-template <typename R, int NT, bool SUN_U, bool SUN_L, typename Q, int SLD>
-__device__ __forceinline__ void column_step(Col<R>& c, const Forc<R>& F, const Stat<R>& S, const Diag<R>& D,
+template <typename R, int NT, bool SUN_U, bool SUN_L, typename Q, typename DD, int SLD>
+__device__ __forceinline__ void column_step(Col<R>& c, const Forc<R>& F, const Stat<R>& S, const DD& D,
                                             const Acc<R, SLD>& Ac, const DevParams<R>& P, const Q& q) {
     Mid<R> M;
-    surface_phase<R, SUN_U, SUN_L>(c, F, S, D, P, q, M);
-    ground_phase<R, NT>(c, F, S, D, Ac, P, q, M);
+    if constexpr (sizeof(R) == 4) {
+        SoilHour G;
+        surface_phase32<SUN_U, SUN_L>(c, F, S, D, P, q, M, G);
+        ground_phase32<NT>(c, F, S, D, Ac, P, q, M, G);
+    } else {
+        surface_phase<R, SUN_U, SUN_L>(c, F, S, D, P, q, M);
+        ground_phase<R, NT>(c, F, S, D, Ac, P, q, M);
+    }
 }
 
 }  // namespace ibis
