@@ -19,7 +19,9 @@ from . import synth
 from .params import StepParams, FLAG_DIAG, FLAG_ACC, FLAG_CH4, FLAG_SOIL_MEANS
 
 INT_MAX = 2 ** 31 - 1
-AUTO_FUSED = 6          # fused, block 224, accumulators on chip
+# the fused configurations ibis_step_f32 chooses from (auto_config, csrc/ibis_kernels.cuh)
+AUTO_SMALL = 4          # single-warp blocks: batches of up to a warp per SM
+AUTO_FUSED = 6          # one block of 224 per SM, accumulators on chip
 AUTO_MIN_HOURS = 4      # shorter launches keep the accumulators in global memory (configuration 0)
 _ACC_FLAGS = FLAG_ACC | FLAG_CH4 | FLAG_SOIL_MEANS
 
@@ -62,10 +64,8 @@ class Columns:
         """``fused`` (one kernel per launch), ``split`` (surface + ground kernels per hour),
         or an integer launch configuration (see ``lib.configs()``).
 
-        ``fused`` picks the configuration per call in FP32: block 224 with the
-        accumulators on chip (configuration 6, the fastest at 95,333 cells)
-        for launches of ``AUTO_MIN_HOURS`` hours or more, the default
-        configuration 0 (global accumulators) for shorter ones; ``tune.tune``
+        ``fused`` leaves the configuration to the library in FP32, by the batch's
+        size and the hours of the call (:meth:`launch_config`); ``tune.tune``
         times every configuration on the caller's own batch instead."""
         if mode is None:
             mode = "fused"
@@ -156,10 +156,17 @@ class Columns:
 
     # -------------------------------------------------------------- compute
     def launch_config(self, nstep: int) -> int:
-        """The launch configuration a call of ``nstep`` hours uses."""
+        """The launch configuration a call of ``nstep`` hours uses: the columns' own, or
+        the library's choice for the batch (``auto_config``, csrc/ibis_kernels.cuh)."""
         if self.config is not None:
             return self.config
-        return AUTO_FUSED if nstep >= AUTO_MIN_HOURS else 0
+        sms = torch.cuda.get_device_properties(self.device).multi_processor_count
+        if self.ncell <= 32 * sms:
+            return AUTO_SMALL
+        if nstep < AUTO_MIN_HOURS or self.ncell <= 128 * sms:
+            return 0
+        waves = lambda threads: -(-self.ncell // (threads * sms))
+        return AUTO_FUSED if waves(224) <= waves(256) else 0
 
     def run(self, forc: torch.Tensor, params: StepParams, nstep: int | None = None, stream=None):
         """Advance the columns ``nstep`` hours with forcing ``forc`` (asynchronous)."""
@@ -183,10 +190,10 @@ class Columns:
         p.flags = flags
         if stream is None:
             stream = torch.cuda.current_stream(self.device)
-        if self.dtype == torch.float32:
+        if self.config is not None and self.dtype == torch.float32:
             rc = self._cfg_fn(_ptr(self.prog), _ptr(self.stat), _ptr(forc), _ptr(self.diag), _ptr(self.acc),
                               _ptr(self.scratch), self.ncell, self.ld, nstep, ctypes.byref(p), _ptr(self.status),
-                              ctypes.c_void_p(stream.cuda_stream), self.launch_config(nstep))
+                              ctypes.c_void_p(stream.cuda_stream), self.config)
         else:
             rc = self._fn(_ptr(self.prog), _ptr(self.stat), _ptr(forc), _ptr(self.diag), _ptr(self.acc), self.ncell,
                           self.ld, nstep, ctypes.byref(p), _ptr(self.status), ctypes.c_void_p(stream.cuda_stream))
@@ -220,9 +227,7 @@ class Columns:
         nstep = host_forc.shape[0]
         if getattr(self, "_host_forc", None) is None or self._host_forc.shape[0] < nstep:
             self._host_forc = torch.empty((nstep, L.N_FORC, self.ld), dtype=self.dtype, device=self.device)
-        cfg = self.launch_config(nstep)
-        if _lib.configs()[cfg]["form"] != "fused":
-            cfg = -1                       # a two-kernel configuration needs scratch: the library's own choice
+        cfg = -1 if self.config is None or self.mode != "fused" else self.config    # -1: the library's own choice
         flags = params.flags & ~FLAG_DIAG if self.diag is None else params.flags | FLAG_DIAG
         if self.acc is None:
             flags &= ~_ACC_FLAGS
@@ -267,9 +272,7 @@ class Columns:
             self._host_daily = torch.empty((nday, L.N_DAILY, self.ld), dtype=torch.float32, device=self.device)
         if getattr(self, "_host_forc", None) is None or self._host_forc.shape[0] < nday * nh:
             self._host_forc = torch.empty((nday * nh, L.N_FORC, self.ld), dtype=self.dtype, device=self.device)
-        cfg = self.launch_config(nday * nh)
-        if _lib.configs()[cfg]["form"] != "fused":
-            cfg = -1
+        cfg = -1 if self.config is None or self.mode != "fused" else self.config
         flags = params.flags & ~FLAG_DIAG if self.diag is None else params.flags | FLAG_DIAG
         if self.acc is None:
             flags &= ~_ACC_FLAGS

@@ -44,6 +44,11 @@ struct Stat {
     int ld;
     __device__ __forceinline__ R operator()(int plane) const { return __ldg(base + (size_t)plane * ld); }
     __device__ __forceinline__ R operator()(int plane, int k) const { return __ldg(base + (size_t)(plane + k) * ld); }
+    // Called once an hour: the compiler must take the view for a new one.  Otherwise it
+    // hoists the loads of a hundred planes and their addresses out of the hour loop,
+    // where no register holds them: they were most of the kernel's local frame (1,056
+    // of 488 bytes more in FP32), read back every hour past an L1 they did not fit.
+    __device__ __forceinline__ void renew() { asm volatile("" : "+l"(base), "+r"(ld)); }
 };
 
 // Optional writer of one cell's diagnostic planes.  ON = false compiles it out, and

@@ -172,6 +172,15 @@ __device__ __forceinline__ void flag_nonfinite(const EnsArgs& e, float sum, int 
 template <bool X3>
 using RunSource = std::conditional_t<X3, RunQ3<float>, RunQ<float>>;
 
+// The thread's record of the hour (HourScratch): after the block's column states and
+// run parameters (71 and 33 words a thread, so it starts on a 64-bit word)
+template <bool SUN, bool X3>
+__device__ __forceinline__ HourScratch<SUN, X3>& ens_hour(unsigned char* smem) {
+    static_assert((sizeof(Col<float>) + sizeof(RunQ<float>)) % 8 == 0, "64-bit words");
+    return reinterpret_cast<HourScratch<SUN, X3>*>(
+        smem + blockDim.x * (sizeof(Col<float>) + sizeof(RunQ<float>)))[threadIdx.x];
+}
+
 template <int NT, bool SU, bool SL, bool DAILY, bool X3>
 __global__ void __launch_bounds__(256, 1) ensemble_kernel(const EnsArgs e, const DevParams<float> P) {
     extern __shared__ unsigned char smem_raw[];
@@ -179,9 +188,11 @@ __global__ void __launch_bounds__(256, 1) ensemble_kernel(const EnsArgs e, const
     RunSource<X3>& q =
         reinterpret_cast<RunSource<X3>*>(smem_raw + blockDim.x * sizeof(Col<float>))[threadIdx.x];
     DayCache* const dc =
-        DAILY ? reinterpret_cast<DayCache*>(smem_raw + blockDim.x * (sizeof(Col<float>) + sizeof(RunQ<float>))) +
+        DAILY ? reinterpret_cast<DayCache*>(smem_raw + blockDim.x * (sizeof(Col<float>) + sizeof(RunQ<float>) +
+                                                                     sizeof(HourScratch<SU || SL, X3>))) +
                     threadIdx.x
               : nullptr;
+    auto& hour = ens_hour<SU || SL, X3>(smem_raw);
     const int lane = threadIdx.x & 31;
     const int nitem = (e.nwork + 31) >> 5;
     const bool kahan = (P.flags & IBIS_FLAG_KAHAN) != 0;
@@ -207,7 +218,7 @@ __global__ void __launch_bounds__(256, 1) ensemble_kernel(const EnsArgs e, const
             }
             load_col(c, e.prog + r, e.ld_run);
             load_run_params(q, e.run_params + r, e.ld_run, P);
-            const Stat<float> S{e.stat + site, e.ld_site};
+            Stat<float> S{e.stat + site, e.ld_site};
             Acc<float> A{e.acc ? e.acc + r : nullptr, e.ld_run, kahan};
             // steps of this call until the run's next year end, and that year's index
             int next_year = e.year_steps - pos % e.year_steps;
@@ -224,7 +235,8 @@ __global__ void __launch_bounds__(256, 1) ensemble_kernel(const EnsArgs e, const
                     F = load_forc_record(f + (size_t)s * IBIS_FORC_COUNT);
                 }
                 A.last = (s + 1 == nstep);
-                column_step<float, NT, SU, SL>(c, F, S, D, A, P, q);
+                S.renew();
+                column_step<float, NT, SU, SL>(c, hour, F, S, D, A, P, q);
                 if (s + 1 == next_year) {
                     if (e.yearly && year < e.nyear) yearly_snapshot(e, A, r, year);
                     ++year;
@@ -262,7 +274,7 @@ __global__ void __launch_bounds__(128, 2) ensemble_hour_kernel(const EnsArgs e, 
     const Stat<float> S{e.stat + site, e.ld_site};
     const Acc<float> A{e.acc ? e.acc + r : nullptr, e.ld_run, (P.flags & IBIS_FLAG_KAHAN) != 0, hour + 1 == nstep};
     const Forc<float> F = load_forc_record(e.forc + (size_t)(first + hour) * IBIS_FORC_COUNT);
-    column_step<float, NT, SU, SL>(c, F, S, Diag<float, false>{nullptr, 0}, A, P, q);
+    column_step<float, NT, SU, SL>(c, ens_hour<SU || SL, X3>(smem_raw), F, S, Diag<float, false>{nullptr, 0}, A, P, q);
     if (e.yearly && (pos + hour + 1) % e.year_steps == 0) {
         const int y = (pos + hour + 1) / e.year_steps - 1;
         if (y < e.nyear) yearly_snapshot(e, A, r, y);
@@ -274,15 +286,36 @@ static __global__ void advance_hour(int* hour0, int n) { *hour0 += n; }
 
 constexpr int kEnsHourBlock = 128;
 
-inline size_t ens_smem(int block, bool daily = false) {
-    return (size_t)block * (sizeof(Col<float>) + sizeof(RunQ<float>) + (daily ? sizeof(DayCache) : 0));
+template <bool SUN, bool X3>
+size_t ens_smem(int block, bool daily = false) {
+    return (size_t)block * (sizeof(Col<float>) + sizeof(RunQ<float>) + sizeof(HourScratch<SUN, X3>) +
+                            (daily ? sizeof(DayCache) : 0));
+}
+
+// The largest block (whole warps, at most `block`) whose shared memory an SM holds:
+// 256 threads except with the sunlit/shaded canopies, the IBIS 3.0 switches and daily
+// weather together.
+template <bool SUN, bool X3>
+int ens_block(int block, bool daily) {
+    while (block > 32 && ens_smem<SUN, X3>(block, daily) > 227 * 1024) block -= 32;
+    return block;
+}
+
+// The kernel's shared-memory attributes for a launch of `block` threads.  The bytes
+// allowed are always the largest block's, so launches of different blocks from several
+// threads cannot take each other's away.
+template <int NT, bool SU, bool SL, bool DAILY, bool X3>
+cudaError_t ens_fit(int block) {
+    return fit_smem(ensemble_kernel<NT, SU, SL, DAILY, X3>, block, ens_smem<SU || SL, X3>(block, DAILY),
+                    ens_smem<SU || SL, X3>(ens_block<SU || SL, X3>(256, DAILY), DAILY));
 }
 
 template <int NT, bool SU, bool SL, bool DAILY = false, bool X3 = false>
 cudaError_t launch_ensemble(const EnsArgs& e, const DevParams<float>& P, int block, int grid, cudaStream_t s) {
+    block = ens_block<SU || SL, X3>(block, DAILY);
     auto k = ensemble_kernel<NT, SU, SL, DAILY, X3>;
-    const size_t smem = ens_smem(block, DAILY);
-    cudaError_t err = fit_smem(k, block, smem, ens_smem(256, DAILY));
+    const size_t smem = ens_smem<SU || SL, X3>(block, DAILY);
+    cudaError_t err = ens_fit<NT, SU, SL, DAILY, X3>(block);
     if (err != cudaSuccess) return err;
     k<<<grid, block, smem, s>>>(e, P);
     return cudaGetLastError();
@@ -292,7 +325,7 @@ template <int NT, bool SU, bool SL, bool X3 = false>
 cudaError_t launch_ensemble_hours(const EnsArgs& e, const DevParams<float>& P, int* hour0, int nhour,
                                   cudaStream_t s) {
     auto k = ensemble_hour_kernel<NT, SU, SL, X3>;
-    const size_t smem = ens_smem(kEnsHourBlock);
+    const size_t smem = ens_smem<SU || SL, X3>(kEnsHourBlock);
     static unsigned long long fitted = 0;
     cudaError_t err = fit_smem_once(fitted, k, kEnsHourBlock, smem, smem);
     if (err != cudaSuccess) return err;
@@ -306,9 +339,11 @@ cudaError_t launch_ensemble_hours(const EnsArgs& e, const DevParams<float>& P, i
 template <int NT, bool SU, bool SL, bool DAILY = false, bool X3 = false>
 int ensemble_occupancy(int block) {
     int n = 0;
+    block = ens_block<SU || SL, X3>(block, DAILY);
     auto k = ensemble_kernel<NT, SU, SL, DAILY, X3>;
-    if (fit_smem(k, block, ens_smem(block, DAILY), ens_smem(256, DAILY)) != cudaSuccess) return 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, block, ens_smem(block, DAILY)) != cudaSuccess) return 0;
+    const size_t smem = ens_smem<SU || SL, X3>(block, DAILY);
+    if (ens_fit<NT, SU, SL, DAILY, X3>(block) != cudaSuccess) return 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, block, smem) != cudaSuccess) return 0;
     return n;
 }
 

@@ -332,28 +332,32 @@ __device__ __forceinline__ void cascade32(Casc<float>& o, const Col32& c, const 
 //   a/E + b E = 2k x,  bd (a/E - b E) = 2 tau / D.
 // The lower story's profile depends on nothing a pass changes, so all of it is formed
 // here; of the upper story's, x changes with the stability of the layer below.
-struct Aero32 {
-    float rhoa, cp;
+struct alignas(8) Aero32 {
     F2 gdz;          // 2 g dz of the two layers the stability corrections act on
     F2 alt;          // log heights of their tops (lower layer: alog2, upper: aloga)
-    F2 alb;          // of their bottoms, before the first pass
-    F2 u0;           // wind below each layer's top: u2 (changes with the passes), ua
-    float alogl;     // alogl after the first pass
-    float alog1, ht; // ta tfac (1 + 0.622 qa)
-    float xu0, sh, ch, sh2, ch2, rbdu;   // upper profile: x sm, sinh and cosh of h and h/2, 1/bd
     F2 c3;           // lower profile: (u3, u34)**2 over taul
     float c4;        // u4**2 over taul
-    float kca, kbi, kci, kdi, kei, kfi, ksu, kss, ksl;
+    float kca, kb, kd, ke;            // conductance factors: to the air, upper, between the stories, lower
+    float rhoa, ua, ht;               // ht: ta tfac (1 + 0.622 qa)
+    float alogl, alog1;               // alogl after the first pass
+    float xu0, rbdu, sh, ch, sh2, ch2;   // upper profile: x sm, 1/bd, sinh and cosh of h and h/2
 };
 
-__device__ __forceinline__ void aero_geometry32(Aero32& A, const Forc32& F, const Stat32& S, float fi,
+// What a pass of turcof carries to the next
+struct Turc {
+    F2 sm, sh;        // stability corrections of the lower and upper layer
+    F2 alb;           // log heights of the bottoms: alogl, alogu
+    float u2;
+};
+
+__device__ __forceinline__ void aero_geometry32(Aero32& A, Turc& tc, float& cp, const Forc32& F, const Stat32& S, float fi,
                                                 const Par32& P) {
     const F2 ztop = stat2(S, IBIS_STAT_ZTOP, 0), zbot = stat2(S, IBIS_STAT_ZBOT, 0);
     const float fu = S(IBIS_STAT_FU), fl = S(IBIS_STAT_FL), z0soi = S(IBIS_STAT_Z0SOI);
     const float pa = F.ps * 0.999f;
     const float rhoa = pa / (P.rair * F.ta * (1.0f + float((double)P.rvap / (double)P.rair - 1.0) * F.qa));
     A.rhoa = rhoa;
-    A.cp = P.cair * (1.0f + float((double)P.cvap / (double)P.cair - 1.0) * F.qa);
+    cp = P.cair * (1.0f + float((double)P.cvap / (double)P.cair - 1.0) * F.qa);
     const float za = mx((F.ps - pa) / (rhoa * P.grav), ztop.hi() + 1.0f);
     const F2 leaf = (stat2(S, IBIS_STAT_LAI, 0) + stat2(S, IBIS_STAT_SAI, 0)) * 2.0f * F2(fl * (1.0f - fi), fu);
     const F2 x = mn2(leaf * F2(1.0f / P.alaiml, 1.0f / P.alaimu), 3.0f);
@@ -378,9 +382,11 @@ __device__ __forceinline__ void aero_geometry32(Aero32& A, const Forc32& F, cons
     const float alog3 = l32.lo(), alog2 = l32.hi(), alog1 = l1a.lo(), aloga = l1a.hi();
     A.alog1 = alog1;
     A.alt = F2(alog2, aloga);
-    A.alb = lg2(mx2(dz * 0.1f, 0.01f));
+    tc.alb = lg2(mx2(dz * 0.1f, 0.01f));
+    tc.sm = tc.sh = F2(1.0f);
     A.gdz = mx2(F2(z2 - z3, za - z1), 0.0f) * (2.0f * P.grav);
-    A.u0 = F2(F.ua * ex(-0.5f * h.hi()), F.ua);
+    tc.u2 = F.ua * ex(-0.5f * h.hi());
+    A.ua = F.ua;
     A.ht = F.ta * P.tfac * (1.0f + 0.622f * F.qa);
     // sinh and cosh of h/2 from expm1, of h by doubling (no cancellation)
     const F2 e = F2(em1(0.5f * h.lo()), em1(0.5f * h.hi()));
@@ -392,38 +398,29 @@ __device__ __forceinline__ void aero_geometry32(Aero32& A, const Forc32& F, cons
     float v = (alog4 - alogav) * rvk;
     const float bdl = bd.lo(), rbdl = 1.0f / bdl, xl = (v * v) * bdl;
     const float nl = xl * ch.lo() + sh.lo(), dl = xl * sh.lo() + ch.lo(), rdl = 1.0f / dl;
-    A.alogl = alog3 - P.vonk * sq(nl * rdl * rbdl);
+    const float alogl = alog3 - P.vonk * sq(nl * rdl * rbdl);
+    A.alogl = alogl;
     const float kl = 0.5f * rdl * rbdl;
     A.c3 = F2(nl, xl * ch2.lo() + sh2.lo()) * (2.0f * kl);
     A.c4 = 2.0f * kl * xl;
-    v = (alog2 - A.alogl) * rvk;
+    v = (alog2 - alogl) * rvk;
     A.xu0 = (v * v) * bd.hi();
     A.sh = sh.hi(); A.ch = ch.hi(); A.sh2 = sh2.hi(); A.ch2 = ch2.hi();
     A.rbdu = 1.0f / bd.hi();
     const float rr = 1.0f / rhoa;
     A.kca = F.ua * P.vonk2 * rhoa / (aloga - alog1);
     // the layers' mid heights are halfway: z1 - z12 = z12 - z2 = (z1 - z2) / 2
-    A.kbi = A.kci = rdveg.hi() * (z1 - z2) * rr;
-    A.kei = A.kfi = rdveg.lo() * (z3 - z4) * rr;
-    A.kdi = (alog2 - A.alogl) * (alog2 - alog3) * rr / P.vonk2;
-    A.ksu = rhoa * P.cleaf * sq(1.0f / P.dleaf[1]);
-    A.kss = rhoa * P.cstem * sq(1.0f / P.dstem[1]);
-    A.ksl = rhoa * P.cgrass * sq(1.0f / P.dleaf[0]);
+    A.kb = rdveg.hi() * (z1 - z2) * rr;
+    A.ke = rdveg.lo() * (z3 - z4) * rr;
+    A.kd = (alog2 - alogl) * (alog2 - alog3) * rr / P.vonk2;
 }
-
-// What a pass of turcof carries to the next
-struct Turc {
-    F2 sm, sh;        // stability corrections of the lower and upper layer
-    F2 alb;           // alogl, alogu
-    float u2;
-};
 
 // fstrat (canopy_exchange.py:287-326) of both layers and turcof (:333-426)
 __device__ __forceinline__ void transfer32(Trans<float>& T, Turc& c, const Aero32& A, float t12, float t34, float q12,
                                            float q34, bool first, const Par32& P) {
     const float h12 = t12 * (1.0f + 0.622f * q12), h34 = t34 * (1.0f + 0.622f * q34);
     const F2 zht(h12, A.ht), zhb(h34, h12);
-    const F2 u(c.u2, A.u0.hi());
+    const F2 u(c.u2, A.ua);
     const F2 rich = clip2(A.gdz * (zht - zhb) * rcp2((zht + zhb) * (u * u)), -2.0f, 1.0f);
     // unstable (rich <= 0): 1 - 10 rich/E, 1 - 15 rich/E with E = 1 + 75 (vonk/xm)^2 e^(xm/2) sqrt(-rich);
     // stable: 1/(1 + 10 rich/r), 1/(1 + 15 rich r) with r = sqrt(1 + 5 rich)
@@ -442,7 +439,7 @@ __device__ __forceinline__ void transfer32(Trans<float>& T, Turc& c, const Aero3
     const float nu = xu * A.ch + A.sh, rd = 1.0f / (xu * A.sh + A.ch);
     const float alogu = A.alog1 - P.vonk * sq(nu * rd * A.rbdu);
     const float aloga = A.alt.hi();
-    const float v = A.u0.hi() * P.vonk / (aloga - alogu);
+    const float v = A.ua * P.vonk / (aloga - alogu);
     const float taul = (v * v) * c.sm.hi() * rd;                 // tauu / D
     const float ku = taul * A.rbdu;
     const F2 u1 = mx2(sq2(mx2(F2(nu, xu * A.ch2 + A.sh2) * ku, 0.0f)), 0.01f);
@@ -451,15 +448,15 @@ __device__ __forceinline__ void transfer32(Trans<float>& T, Turc& c, const Aero3
     const float u12 = u1.hi(), nu2 = ue.lo(), u34 = u3.hi(), u4 = ue.hi();
     const float ca = mn(P.cdmax * A.rhoa, A.kca * c.sh.hi() / (aloga - alogu));
     const float ub = u1.lo() + u12;
-    T.cu = ca * ub / (ub + A.kbi * ca);
-    T.cl = 1.0f / (A.kci / (u12 + nu2) + A.kdi / (nu2 * c.sh.lo()) + A.kei / (u3.lo() + u34));
-    const float q1 = sq(u12);
-    T.su = A.ksu * q1;
-    T.ss = A.kss * q1;
-    T.sl = A.ksl * sq(u34);
+    T.cu = ca * ub / (ub + A.kb * ca);
+    T.cl = 1.0f / (A.kb / (u12 + nu2) + A.kd / (nu2 * c.sh.lo()) + A.ke / (u3.lo() + u34));
+    const float q1 = A.rhoa * sq(u12);
+    T.su = q1 * P.ksu;
+    T.ss = q1 * P.kss;
+    T.sl = A.rhoa * sq(u34) * P.ksl;
     const F2 s0 = A.rhoa * (F2(0.004f, 0.003f) + F2(0.012f, 0.010f) * u4);
     const float uf = u34 + u4;
-    const F2 sg = s0 * uf * rcp2(uf + A.kfi * s0);
+    const F2 sg = s0 * uf * rcp2(uf + A.ke * s0);
     T.sg = sg.lo();
     T.si = sg.hi();
     c.u2 = nu2;
@@ -544,27 +541,29 @@ __device__ __forceinline__ F2 leaf_conductance2(const F2& anc, const Story& t, c
     return gsc * t.s * rcp2(gsc + t.s * float(1.0 / 0.029));      // 1 / (1/s + (1/0.029)/g)
 }
 
+// The light and capacity of a story's sunlit and shaded leaves (sunshade_canopy), per
+// leaf area: (sunlit, shaded) pairs
+struct Sun4 { F2 p, v; };
+
 // Two C3 leaves of a story: rates, Ball-Berry, scaled rates and conductance.
-// vn, cm: nominal vmax and slope; jf/jon, cap, fcap: the IBIS 3.0 factors.
+// vn, cm: nominal vmax and slope; jf, cap, fcap: the IBIS 3.0 factors.
 template <bool SUN, bool X3>
 __device__ __forceinline__ F2 c3_pair(F2& cs, F2& gs, F2& ci_, F2& ag_o, F2& an_o, const Story& t, float gst,
                                       float kco, float vm3, const F2& vn, const F2& cm, const F2& gamma, const F2& b0,
-                                      const F2& gmin, const SunShade<float>& ss, float rlai, const F2& jf, bool jon,
-                                      bool cap, float fcap, const Par32& P) {
+                                      const F2& gmin, const Sun4& ss, const F2& jf, bool cap, float fcap,
+                                      const Par32& P) {
     const F2 ci = clip2(ci_, t.gmn, P.cimax);
     const F2 vmax = vn * (vm3 * t.stress);
     const F2 rd = gamma * vn * vm3;
     const F2 X = (ci - gst) * rcp2(ci + 2.0f * gst) * (4.59e-06f * P.alpha3);
     const F2 Y = vmax * ((ci - gst) * rcp2(ci + kco)), Z = vmax * float(1.0 / 2.2);
     F2 Xf = X;
-    if constexpr (X3) {
-        if (jon) Xf = X * jf;
-    }
+    if constexpr (X3) Xf = X * jf;
     F2 ag, an;
     if constexpr (SUN) {
-        const F2 a = c3_gross(Xf * ss.psun, Y * ss.vsun, Z * ss.vsun, P) + c3_gross(Xf * ss.psha, Y * ss.vsha, Z * ss.vsha, P);
-        ag = a * rlai;
-        an = (a - rd * (ss.vsun + ss.vsha)) * rlai;
+        ag = c3_gross(Xf * ss.p.lo(), Y * ss.v.lo(), Z * ss.v.lo(), P) +
+             c3_gross(Xf * ss.p.hi(), Y * ss.v.hi(), Z * ss.v.hi(), P);
+        an = ag - rd * ss.v.sum();
     } else {
         ag = c3_gross(Xf * t.par, Y, Z, P);
         an = ag - rd;
@@ -585,65 +584,108 @@ __device__ __forceinline__ F2 c3_pair(F2& cs, F2& gs, F2& ci_, F2& ag_o, F2& an_
     return leaf_conductance2(an, t, cm, b0, gmin, P);
 }
 
-// canopy_scaling (stomata.py:442-512) of both stories; advances the carried means
-__device__ __forceinline__ F2 light_scaling2(const F2& toppar, const F2& k, const F2& h, const F2 (&sc)[4],
-                                             const F2& lai, const F2& sai, Col32& c, bool leaf_only, const Par32& P) {
-    const F2 ext = clip2((k * sc[0] + h * (sc[1] - sc[2])) * rcp2(mx2(sc[3], P.epsilon)), 0.1f, 10.0f);
+// canopy_scaling (stomata.py:442-512) of both stories.  Nothing it reads changes
+// between the hour's passes except its own carried means, and those only by day, when
+// it does not read them: so it is formed once, and the means advanced once per pass.
+__device__ __forceinline__ F2 light_scaling2(const Rad<float>& Rd, const F2& lai, const F2& sai, Col32& c,
+                                             bool leaf_only, const Par32& P) {
+    const F2 toppar(Rd.topparu, Rd.topparl), k(Rd.termu6, Rd.terml6), h(Rd.termu7, Rd.terml7);
+    const F2 sc0(Rd.scu[0], Rd.scl[0]), sc12(Rd.scu[1] - Rd.scu[2], Rd.scl[1] - Rd.scl[2]), sc3(Rd.scu[3], Rd.scl[3]);
+    const F2 ext = clip2((k * sc0 + h * sc12) * rcp2(mx2(sc3, P.epsilon)), 0.1f, 10.0f);
     const F2 pxai = ext * (lai + sai), plai = ext * lai;
     const F2 sday = (1.0f - ex2(pxai * -1.0f)) * rcp2(mx2(leaf_only ? pxai : plai, P.epsilon));
-    const F2 as(c.a10su, c.a10sl), ad(c.a10du, c.a10dl);
+    F2 as(c.a10su, c.a10sl), ad(c.a10du, c.a10dl);
     const F2 snight = as * rcp2(mx2(ad, P.epsilon));
     const float z = P.zweight;
-    const F2 tz = toppar * (1.0f - z);
-    const F2 asn = as * z + sday * tz, adn = ad * z + tz;
+    const F2 tz = toppar * (1.0f - z), ts = sday * tz;
+#pragma unroll
+    for (int it = 0; it < 3; ++it) {
+        as = as * z + ts;
+        ad = ad * z + tz;
+    }
     const bool hu = plai.lo() > 0.0f, hl = plai.hi() > 0.0f, du = toppar.lo() > 10.0f, dl = toppar.hi() > 10.0f;
-    if (hu && du) { c.a10su = asn.lo(); c.a10du = adn.lo(); }
-    if (hl && dl) { c.a10sl = asn.hi(); c.a10dl = adn.hi(); }
+    if (hu && du) { c.a10su = as.lo(); c.a10du = ad.lo(); }
+    if (hl && dl) { c.a10sl = as.hi(); c.a10dl = ad.hi(); }
     return sel2(hu, hl, sel2(du, dl, sday, snight), F2(0.0f));
 }
 
+// ===========================================================================
+// What the three canopy passes share, kept in shared memory for the hour
+//
+// The passes read some eighty values that none of them changes.  In registers they
+// cannot stay (the double canopy solve needs the file), and spilled they miss: eight
+// warps' local frames are three times what L1 has left, and two of three local loads
+// went to L2, the largest stall of the kernel.  Here they are read in 64-bit words at
+// shared-memory latency.  A record is an odd number of 64-bit words, so a warp's
+// loads of one word touch every bank once per half-warp.
+// ===========================================================================
+
+template <bool SUN, bool X3>
+struct HourExtra {};
+template <>
+struct alignas(8) HourExtra<true, false> { Sun4 su, sl; };
+// with the IBIS 3.0 switches also the big leaves' nominal vmax, slopes and light
+// factors (C4 grass last) and the capacity integrals (upper, lower)
+template <>
+struct alignas(8) HourExtra<false, true> { F2 vnl, cmu, cml, jfu, jfl, cap; float vn4, cm4, jf4, unused; };
+template <>
+struct alignas(8) HourExtra<true, true> { Sun4 su, sl; F2 vnl, cmu, cml, jfu, jfl, cap; float vn4, cm4, jf4, unused; };
+
+// Pairs: (upper leaves, upper stems) `_us`, (lower canopy, ground) `_lg`, (ground, snow) `_gi`
+struct alignas(8) TvHour {
+    F2 x_us, ch_us, ch_lg, wl_us, ws_us, wl_lg, ws_lg, rl_us, fw_us, frad_us, pf_us;
+    F2 hv_gi, sol_gi, fir_gi, zir_gi, co_gi;
+    F2 stress, toppar, scale;       // (upper, lower)
+    F2 vnu;                         // nominal vmax of the upper big leaves
+    float xl, rliql, fwetl, fradl, pfluxl, psig, cp, firb, ta, qa, ps, fi;
+    double betaw;                   // soil-surface wetness factor
+    double fb, fc, fs, rlai;        // leaf-area shares of the big leaves; lai0 / (lai0 + sai0)
+};
+
+template <bool SUN, bool X3>
+struct alignas(8) HourWords : HourExtra<SUN, X3> {
+    Aero32 A;
+    TvHour X;
+};
+
+template <bool EVEN>
+struct WordPad {};
+template <>
+struct WordPad<true> { unsigned long long pad; };
+template <bool SUN, bool X3>
+struct HourScratch : HourWords<SUN, X3>, WordPad<(sizeof(HourWords<SUN, X3>) / 8) % 2 == 0> {};
+
 // One pass of stomata over the five big leaves (see the template in ibis_canopy.cuh)
-template <bool SUN_U, bool SUN_L, typename Q>
-__device__ __forceinline__ void stomata32(Stom<float>& o, Col32& c, float tu, float tl, const F2& tair, const F2& qair,
-                                          const F2& qs_air, float su, float sl, const Rad<float>& Rd, float fwetu,
-                                          float fwetl, const Stat32& S, float stresstu, float stresstl, const Par32& P,
+template <bool SUN_U, bool SUN_L, typename Y, typename Q>
+__device__ __forceinline__ void stomata32(Stom<float>& o, Col32& c, float tu, float tl, const F2& qair,
+                                          const F2& qs_air, float su, float sl, const Y& y, const Par32& P,
                                           const Q& q) {
     constexpr bool X3 = Q::x3;
-    const F2 lai(S(IBIS_STAT_LAI, 1), S(IBIS_STAT_LAI, 0)), sai(S(IBIS_STAT_SAI, 1), S(IBIS_STAT_SAI, 0));
-    const bool leaf_only = X3 && (P.flags & IBIS_FLAG_LEAF_ONLY) != 0;
+    const TvHour& X = y.X;
     const Kin2 K = kinetics2(F2(tu, tl), P);
     const F2 rh = mx2(qair * rcp2(mx2(qs_air, P.epsilon)), 0.30f);
     const F2 rgb = rcp2(clip2(F2(su, sl) * 25.5f, 0.1f, 10.0f));
-    const F2 sc[4] = {F2(Rd.scu[0], Rd.scl[0]), F2(Rd.scu[1], Rd.scl[1]), F2(Rd.scu[2], Rd.scl[2]),
-                      F2(Rd.scu[3], Rd.scl[3])};
-    // the light scaling reads and advances only its own carried means
-    const F2 scale = light_scaling2(F2(Rd.topparu, Rd.topparl), F2(Rd.termu6, Rd.terml6), F2(Rd.termu7, Rd.terml7), sc,
-                                    lai, sai, c, leaf_only, P);
-    SunShade<float> ss{};
-    float rlai = 0.0f;
+    const F2 stress = X.stress, toppar = X.toppar, scale = X.scale;
+    const bool cap = X3 && (P.flags & IBIS_FLAG_CAP_SCALE_L) != 0 && !SUN_L;
     // ---------------- upper canopy: broadleaf and conifer
     {
-        float vn[2], jf[2] = {1.0f, 1.0f}, cm[2];
-        bool jon = false;
+        const Story t{1.05f * K.gst.lo(), rgb.lo(), rh.lo(), stress.lo(), scale.lo(), su, toppar.lo(), X.fw_us.lo()};
+        F2 cs(c.cs_u[0], c.cs_u[1]), gs(c.gs_u[0], c.gs_u[1]), ci(c.ci_u[0], c.ci_u[1]), ag, an, cm, jf(1.0f);
+        Sun4 ss{};
+        float fcap = 0.0f;
+        bool capu = false;
         if constexpr (X3) {
-            big_leaves<float, false>(vn, jf, cm, jon, S, P, q);
+            cm = y.cmu;
+            jf = y.jfu;
+            fcap = y.cap.lo();
+            capu = !SUN_U && (P.flags & IBIS_FLAG_CAP_SCALE_U) != 0;
         } else {
-            vn[0] = S(IBIS_STAT_EXIST, 0) > 0.5f ? q.vmax(0) : (S(IBIS_STAT_EXIST, 2) > 0.5f ? q.vmax(2) : q.vmax(4));
-            vn[1] = S(IBIS_STAT_EXIST, 3) > 0.5f ? q.vmax(3) : q.vmax(5);
-            cm[0] = q.coefm(0);
-            cm[1] = q.coefm(1);
+            cm = F2(q.coefm(0), q.coefm(1));
         }
-        const bool cap = X3 && !SUN_U && (P.flags & IBIS_FLAG_CAP_SCALE_U) != 0;
-        const float fcap = cap ? capacity_integral(lai.lo(), P.cap_kn) : 0.0f;
-        if constexpr (SUN_U) {
-            ss = sunshade(Rd.scu, Rd.dbeamu, Rd.termu6, Rd.termu7, lai.lo(), sai.lo(), P);
-            rlai = lai.lo() > 0.0f ? 1.0f / mx(lai.lo(), 1.0e-6f) : 0.0f;
-        }
-        const Story t{1.05f * K.gst.lo(), rgb.lo(), rh.lo(), stresstu, scale.lo(), su, Rd.topparu, fwetu};
-        F2 cs(c.cs_u[0], c.cs_u[1]), gs(c.gs_u[0], c.gs_u[1]), ci(c.ci_u[0], c.ci_u[1]), ag, an;
-        const F2 tc = c3_pair<SUN_U, X3>(cs, gs, ci, ag, an, t, K.gst.lo(), K.kco.lo(), K.vm3.lo(), F2(vn[0], vn[1]),
-                                         F2(cm[0], cm[1]), F2(P.gamma[0], P.gamma[1]), F2(P.coefb[0], P.coefb[1]),
-                                         F2(P.gsmin[0], P.gsmin[1]), ss, rlai, F2(jf[0], jf[1]), jon, cap, fcap, P);
+        if constexpr (SUN_U) ss = y.su;
+        const F2 tc = c3_pair<SUN_U, X3>(cs, gs, ci, ag, an, t, K.gst.lo(), K.kco.lo(), K.vm3.lo(), X.vnu, cm,
+                                         F2(P.gamma[0], P.gamma[1]), F2(P.coefb[0], P.coefb[1]),
+                                         F2(P.gsmin[0], P.gsmin[1]), ss, jf, capu, fcap, P);
         c.cs_u[0] = cs.lo(); c.cs_u[1] = cs.hi(); c.gs_u[0] = gs.lo(); c.gs_u[1] = gs.hi();
         c.ci_u[0] = ci.lo(); c.ci_u[1] = ci.hi();
         o.ag_u[0] = ag.lo(); o.ag_u[1] = ag.hi(); o.an_u[0] = an.lo(); o.an_u[1] = an.hi();
@@ -652,25 +694,22 @@ __device__ __forceinline__ void stomata32(Stom<float>& o, Col32& c, float tu, fl
     }
     // ---------------- lower canopy: shrub (group 2) and C3 grass (group 4), then C4 grass (group 3)
     {
-        float vn[3], jf[3] = {1.0f, 1.0f, 1.0f}, cm[3];
-        bool jon = false;
+        const Story t{1.05f * K.gst.hi(), rgb.hi(), rh.hi(), stress.hi(), scale.hi(), sl, toppar.hi(), X.fwetl};
+        F2 cs(c.cs_l[0], c.cs_l[1]), gs(c.gs_l[0], c.gs_l[1]), ci(c.ci_l[0], c.ci_l[1]), ag, an, vn, cm, jf(1.0f);
+        float vn4, cm4, jf4 = 1.0f, fcap = 0.0f;
+        Sun4 ss{};
         if constexpr (X3) {
-            big_leaves<float, true>(vn, jf, cm, jon, S, P, q);
+            vn = y.vnl; cm = y.cml; jf = y.jfl;
+            vn4 = y.vn4; cm4 = y.cm4; jf4 = y.jf4;
+            fcap = y.cap.hi();
         } else {
-            vn[0] = q.vmax(8); vn[1] = q.vmax(11); vn[2] = q.vmax(10);
-            cm[0] = q.coefm(2); cm[1] = q.coefm(4); cm[2] = q.coefm(3);
+            vn = F2(q.vmax(8), q.vmax(11)); cm = F2(q.coefm(2), q.coefm(4));
+            vn4 = q.vmax(10); cm4 = q.coefm(3);
         }
-        const bool cap = X3 && !SUN_L && (P.flags & IBIS_FLAG_CAP_SCALE_L) != 0;
-        const float fcap = cap ? capacity_integral(lai.hi(), P.cap_kn) : 0.0f;
-        if constexpr (SUN_L) {
-            ss = sunshade(Rd.scl, Rd.dbeaml, Rd.terml6, Rd.terml7, lai.hi(), sai.hi(), P);
-            rlai = lai.hi() > 0.0f ? 1.0f / mx(lai.hi(), 1.0e-6f) : 0.0f;
-        }
-        const Story t{1.05f * K.gst.hi(), rgb.hi(), rh.hi(), stresstl, scale.hi(), sl, Rd.topparl, fwetl};
-        F2 cs(c.cs_l[0], c.cs_l[1]), gs(c.gs_l[0], c.gs_l[1]), ci(c.ci_l[0], c.ci_l[1]), ag, an;
-        const F2 tc = c3_pair<SUN_L, X3>(cs, gs, ci, ag, an, t, K.gst.hi(), K.kco.hi(), K.vm3.hi(), F2(vn[0], vn[1]),
-                                         F2(cm[0], cm[1]), F2(P.gamma[2], P.gamma[4]), F2(P.coefb[2], P.coefb[4]),
-                                         F2(P.gsmin[2], P.gsmin[4]), ss, rlai, F2(jf[0], jf[1]), jon, cap, fcap, P);
+        if constexpr (SUN_L) ss = y.sl;
+        const F2 tc = c3_pair<SUN_L, X3>(cs, gs, ci, ag, an, t, K.gst.hi(), K.kco.hi(), K.vm3.hi(), vn, cm,
+                                         F2(P.gamma[2], P.gamma[4]), F2(P.coefb[2], P.coefb[4]),
+                                         F2(P.gsmin[2], P.gsmin[4]), ss, jf, cap, fcap, P);
         c.cs_l[0] = cs.lo(); c.cs_l[1] = cs.hi(); c.gs_l[0] = gs.lo(); c.gs_l[1] = gs.hi();
         c.ci_l[0] = ci.lo(); c.ci_l[1] = ci.hi();
         o.ag_l[0] = ag.lo(); o.ag_l[1] = ag.hi(); o.an_l[0] = an.lo(); o.an_l[1] = an.hi();
@@ -678,28 +717,25 @@ __device__ __forceinline__ void stomata32(Stom<float>& o, Col32& c, float tu, fl
         o.tcl3 = tc.hi();
         // C4 grass
         const float c4 = clip(c.ci_l[2], 0.0f, P.cimax);
-        const float vmax = vn[2] * K.vm4 * stresstl, rd = P.gamma[3] * vn[2] * K.vm4;
-        float xe = 4.59e-06f * P.alpha4;
-        if (X3 && jon) xe = xe * jf[2];
-        const float ji = 18.0e3f * vmax * c4;
+        const float vmax = vn4 * K.vm4 * t.stress, rd = P.gamma[3] * vn4 * K.vm4;
+        const float xe = 4.59e-06f * P.alpha4 * jf4, ji = 18.0e3f * vmax * c4;
         float ag4, an4;
         if constexpr (SUN_L) {
-            const float a = c4_gross(xe * ss.psun, vmax * ss.vsun, ji * ss.vsun, P) +
-                            c4_gross(xe * ss.psha, vmax * ss.vsha, ji * ss.vsha, P);
-            ag4 = a * rlai;
-            an4 = (a - rd * (ss.vsun + ss.vsha)) * rlai;
+            ag4 = c4_gross(xe * ss.p.lo(), vmax * ss.v.lo(), ji * ss.v.lo(), P) +
+                  c4_gross(xe * ss.p.hi(), vmax * ss.v.hi(), ji * ss.v.hi(), P);
+            an4 = ag4 - rd * ss.v.sum();
         } else {
             ag4 = c4_gross(xe * t.par, vmax, ji, P);
             an4 = ag4 - rd;
         }
-        const float b0s = P.coefb[3] * stresstl, gm = mx(P.gsmin[3], b0s), mr = cm[2] * t.rh;
+        const float b0s = P.coefb[3] * t.stress, gm = mx(P.gsmin[3], b0s), mr = cm4 * t.rh;
         const float csn = mx(1.0e-8f, 0.5f * (c.cs_l[2] + P.co2conc - an4 * t.rgb));
         const float gsn = mx(0.5f * (c.gs_l[2] + mr * an4 / csn + b0s), gm);
         c.ci_l[2] = clip(0.5f * (c4 + csn - 1.6f * an4 / gsn), 0.0f, P.cimax);
         c.cs_l[2] = csn;
         c.gs_l[2] = gsn;
         if constexpr (!SUN_L) {
-            if (X3 && cap) {
+            if (cap) {
                 ag4 = c4_gross(xe * (t.par * t.scale), vmax * fcap, ji * fcap, P);
                 an4 = ag4 - rd * fcap;
             } else {
@@ -709,9 +745,9 @@ __device__ __forceinline__ void stomata32(Stom<float>& o, Col32& c, float tu, fl
         }
         const float csc = mx(1.0e-8f, P.co2conc - an4 * t.rgb);
         const float gsc = mx(gm, mr * an4 / csc + b0s);
-        o.tcl4 = gsc * sl / (gsc + sl * float(1.0 / 0.029));
-        o.ag_l[2] = ag4 * (1.0f - fwetl);
-        o.an_l[2] = an4 * (1.0f - fwetl);
+        o.tcl4 = gsc * t.s / (gsc + t.s * float(1.0 / 0.029));
+        o.ag_l[2] = ag4 * (1.0f - t.fw);
+        o.an_l[2] = an4 * (1.0f - t.fw);
     }
 }
 
@@ -719,18 +755,6 @@ __device__ __forceinline__ void stomata32(Stom<float>& o, Col32& c, float tu, fl
 // turvap: the 9x9 implicit canopy / air / ground / snow system
 // (canopy_exchange.py:470-811), in double
 // ===========================================================================
-
-// What the three passes share, besides the interception and radiation results
-struct TvHour {
-    float xu, xs, xl, fi, chux, chsx, chlx, cog, coi, zirg, ziri;
-    float wu, ws, wl;               // the water (liquid and snow) on each surface
-    float rliqu, rliqs, rliql, fwetu, fwets, fwetl;
-    float hvasug, hvasui, tsoi0, tsno0, psig;
-    float fradu, frads, fradl, pfluxu, pfluxs, pfluxl;
-    float solg, soli, firg, firi;
-    double betaw;                   // soil-surface wetness factor
-    double fb, fc, fs, rlai;        // leaf-area shares of the big leaves; lai0 / (lai0 + sai0)
-};
 
 struct TvResult {
     float fsena, fsenu, fsens, fsenl, fseng, fseni;
@@ -743,12 +767,10 @@ struct TvResult {
 // Eliminating them leaves the 4x4 system of the two air layers' temperature and
 // humidity, solved by 2x2 blocks (the layers couple through -cl I).  The full
 // elimination it replaces filled 45 entries and divided by nine pivots.
-template <typename Q>
 __device__ __forceinline__ void turvap32(double (&W)[9], TvResult& o, const Col32& c, const Trans<float>& T,
-                                         float cpf, const F2& wus, const F2& wlg, float wif, const TvHour& X,
-                                         const Stom<float>& st, const Forc32& F, const Rad<float>& Rd,
-                                         const Stat32& S, float e34, float q34s, bool last, const Par32& P,
-                                         const Q& q) {
+                                         const F2& wus, const F2& wlg, float wif, const TvHour& X,
+                                         const Stom<float>& st, const Stat32& S, float e34, float q34s, bool last,
+                                         const Par32& P) {
     const double eps = (double)P.epsilon, dt = (double)P.dtime;
     const double wu = wus.lo(), ws = wus.hi(), wl = wlg.lo(), wg = wlg.hi(), wi = wif;
     // the temperatures at the hour's start (the column's are not advanced until the passes end)
@@ -760,7 +782,7 @@ __device__ __forceinline__ void turvap32(double (&W)[9], TvResult& o, const Col3
     // saturation humidities and their capped derivatives in float, two at a time
     double qu, qs, ql, qg, qi, dqu, dqs, dql, dqg, dqi, dqs1;
     {
-        const float ps = F.ps;
+        const float ps = X.ps;
         const F2 ta((float)tu, (float)ts), tb((float)tl, (float)tg), tc((float)ti, (float)t34);
         const F2 ea = esat2(ta), eb = esat2(tb);
         const F2 ec(esat(tc.lo()), e34);
@@ -772,7 +794,7 @@ __device__ __forceinline__ void turvap32(double (&W)[9], TvResult& o, const Col3
         dqu = da.lo(); dqs = da.hi(); dql = db.lo(); dqg = db.hi(); dqi = mn(dc.lo(), qc.lo() * 0.1f);
         dqs1 = dc.hi();
     }
-    const double su = T.su, ss = T.ss, sl = T.sl, sg = T.sg, si = T.si, cu = T.cu, cl = T.cl, cp = cpf;
+    const double su = T.su, ss = T.ss, sl = T.sl, sg = T.sg, si = T.si, cu = T.cu, cl = T.cl, cp = X.cp;
     const double qeps = 1.0e-10, hvap = (double)P.hvap, tmelt = (double)P.tmelt;
     // soil-surface humidity factor (canopy_exchange.py:532-572)
     const double hfac = (double)ex(X.psig / (P.rvap * (float)tg));
@@ -782,22 +804,23 @@ __device__ __forceinline__ void turvap32(double (&W)[9], TvResult& o, const Col3
     double qgfac = betas > 0.0 ? fma(betas, hfac - hfac2, hfac2) : hfac2;
     if (q34 > qg + qeps) qgfac = 1.0;
     // vapour conductances (canopy_exchange.py:587-618)
-    const double fwux = (q12 > qu + qeps) ? 1.0 : X.fwetu;
-    const double fwsx = (q12 > qs + qeps) ? 1.0 : X.fwets;
+    const F2 wet_us = X.wl_us + X.ws_us;
+    const double fwux = (q12 > qu + qeps) ? 1.0 : X.fw_us.lo();
+    const double fwsx = (q12 > qs + qeps) ? 1.0 : X.fw_us.hi();
     const double fwlx = (q34 > ql + qeps) ? 1.0 : X.fwetl;
-    const double suw = fmin(fwux * su, 0.8 * X.wu * rcp_nr(fmax(dt * (qu - q12), eps)));
-    const double ssw = fmin(fwsx * ss, 0.8 * X.ws * rcp_nr(fmax(dt * (qs - q12), eps)));
-    const double slw = fmin(fwlx * sl, 0.8 * X.wl * rcp_nr(fmax(dt * (ql - q34), eps)));
+    const double suw = fmin(fwux * su, 0.8 * wet_us.lo() * rcp_nr(fmax(dt * (qu - q12), eps)));
+    const double ssw = fmin(fwsx * ss, 0.8 * wet_us.hi() * rcp_nr(fmax(dt * (qs - q12), eps)));
+    const double slw = fmin(fwlx * sl, 0.8 * (X.wl_lg.lo() + X.ws_lg.lo()) * rcp_nr(fmax(dt * (ql - q34), eps)));
     const double sut = fmax(0.0, (0.5 - 0.5 * fwux) * (st.tcub * X.fb + st.tcuc * X.fc));
     const double slt0 = fmax(0.0, (0.5 - 0.5 * fwlx) * (st.tcls * X.fs + (double)st.tcl4 * S(IBIS_STAT_FRAC, 10) +
                                                        (double)st.tcl3 * S(IBIS_STAT_FRAC, 11)));
     const double slt = slt0 * X.rlai;
-    const double cvt = (double)P.cvap * ((double)F.ta - tmelt);
+    const double cvt = (double)P.cvap * ((double)X.ta - tmelt);
     const double hv0 = fma((double)P.ch2o, tmelt, hvap + cvt), hs0 = fma((double)P.cice, tmelt, (double)P.hsub + cvt);
     const double hvu = fma(-(double)P.ch2o, tu, hv0), hvl = fma(-(double)P.ch2o, tl, hv0), hvs = fma(-(double)P.ch2o, ts, hv0);
     const double hsu = fma(-(double)P.cice, tu, hs0), hsl = fma(-(double)P.cice, tl, hs0), hss = fma(-(double)P.cice, ts, hs0);
-    const double suh = fma(suw, fma((double)X.rliqu, hvu - hsu, hsu), sut * hvu);
-    const double ssh = ssw * fma((double)X.rliqs, hvs - hss, hss);
+    const double suh = fma(suw, fma((double)X.rl_us.lo(), hvu - hsu, hsu), sut * hvu);
+    const double ssh = ssw * fma((double)X.rl_us.hi(), hvs - hss, hss);
     const double slh = fma(slw, fma((double)X.rliql, hvl - hsl, hsl), slt * hvl);
 
     // the five local rows: x = b + r T + s Q (canopy_exchange.py:620-682)
@@ -811,38 +834,38 @@ __device__ __forceinline__ void turvap32(double (&W)[9], TvResult& o, const Col3
         r = r2 * inv;
         a = sh * inv;
     };
-    leaf(old[0], X.chux, wu, su, suh, qu, dqu, tu, (double)X.fradu - X.pfluxu, bu, ru, au);
-    leaf(old[1], X.chsx, ws, ss, ssh, qs, dqs, ts, (double)X.frads - X.pfluxs, bs, rs, as);
-    leaf(old[2], X.chlx, wl, sl, slh, ql, dql, tl, (double)X.fradl - X.pfluxl, bl, rl, al);
-    const bool bare = (X.xu + X.xs + X.xl) < P.epsilon;
+    leaf(old[0], X.ch_us.lo(), wu, su, suh, qu, dqu, tu, (double)X.frad_us.lo() - X.pf_us.lo(), bu, ru, au);
+    leaf(old[1], X.ch_us.hi(), ws, ss, ssh, qs, dqs, ts, (double)X.frad_us.hi() - X.pf_us.hi(), bs, rs, as);
+    leaf(old[2], X.ch_lg.lo(), wl, sl, slh, ql, dql, tl, (double)X.fradl - X.pfluxl, bl, rl, al);
+    const bool bare = (X.x_us.lo() + X.x_us.hi() + X.xl) < P.epsilon;
     {
-        const double r1 = sg * cp, r2 = sg * X.hvasug, g = r2 * qgfac;
-        const double inv = rcp_nr(r1 + fma(g, dqg, (double)X.cog) + X.zirg);
-        double b = fma((double)X.zirg, old[3], fma((double)X.cog, (double)X.tsoi0, (double)Rd.solg + (double)Rd.firg)) -
+        const double r1 = sg * cp, r2 = sg * X.hv_gi.lo(), g = r2 * qgfac;
+        const double inv = rcp_nr(r1 + fma(g, dqg, (double)X.co_gi.lo()) + X.zir_gi.lo());
+        double b = fma((double)X.zir_gi.lo(), old[3], fma((double)X.co_gi.lo(), (double)c.tsoi[0], (double)X.sol_gi.lo() + (double)X.fir_gi.lo())) -
                    g * fma(-dqg, tg, qg);
         // a bare cell's canopy heat goes to the ground (canopy_exchange.py:684-732)
         if (bare)
-            b = b + (((double)X.fradu - X.pfluxu) * X.xu + ((double)X.frads - X.pfluxs) * X.xs +
+            b = b + (((double)X.frad_us.lo() - X.pf_us.lo()) * X.x_us.lo() + ((double)X.frad_us.hi() - X.pf_us.hi()) * X.x_us.hi() +
                      ((double)X.fradl - X.pfluxl) * X.xl);
         bg = b * inv; rg = r1 * inv; ag = r2 * inv;
     }
     {
-        const double r1 = si * cp, r2 = si * X.hvasui;
-        const double inv = rcp_nr(r1 + fma(r2, dqi, (double)X.coi) + X.ziri);
-        bi = (fma((double)X.ziri, old[4], fma((double)X.coi, (double)X.tsno0, (double)Rd.soli + (double)Rd.firi)) -
+        const double r1 = si * cp, r2 = si * X.hv_gi.hi();
+        const double inv = rcp_nr(r1 + fma(r2, dqi, (double)X.co_gi.hi()) + X.zir_gi.hi());
+        bi = (fma((double)X.zir_gi.hi(), old[4], fma((double)X.co_gi.hi(), (double)c.tsno[0], (double)X.sol_gi.hi() + (double)X.fir_gi.hi())) -
               r2 * fma(-dqi, ti, qi)) * inv;
         ri = r1 * inv; ai = r2 * inv;
     }
     // the 4x4 system of (t12, q12 | t34, q34)
-    const double ta64 = F.ta, tap = ta64 * (double)P.tfac, qa64 = F.qa;
+    const double tap = (double)X.ta * (double)P.tfac, qa64 = X.qa;
     double n12, nq12, n34, nq34;
     {
         const double cc = cu + cl;
-        double kt = X.xu * su, kq = X.xu * (suw + sut);
+        double kt = X.x_us.lo() * su, kq = X.x_us.lo() * (suw + sut);
         double mt = wu * kt, mq = wu * kq * dqu;
         double u11 = cc + kt - mt * ru, u12 = -mt * au, f1 = fma(cu, tap, fma(kt - mt, tu, mt * bu));
         double u21 = -mq * ru, u22 = cc + kq - mq * au, f2 = fma(cu, qa64, fma(kq, qu, mq * (bu - tu)));
-        kt = X.xs * ss; kq = X.xs * ssw;
+        kt = X.x_us.hi() * ss; kq = X.x_us.hi() * ssw;
         mt = ws * kt; mq = ws * kq * dqs;
         u11 += kt - mt * rs; u12 -= mt * as; f1 += fma(kt - mt, ts, mt * bs);
         u21 -= mq * rs; u22 += kq - mq * as; f2 += fma(kq, qs, mq * (bs - ts));
@@ -892,13 +915,13 @@ __device__ __forceinline__ void turvap32(double (&W)[9], TvResult& o, const Col3
         const double fvaplw = slw * el, fvaplt = fmax(0.0, slt0 * el);
         const double fvapg = sg * (qgfac * fma(wg * dqg, ng - tg, qg) - nq34);
         const double fvapi = si * (fma(wi * dqi, ni - ti, qi) - nq34);
-        const double dg = wg * X.zirg * (ng - old[3]), di = wi * X.ziri * (ni - old[4]);
-        o.firg = (float)(Rd.firg - dg);
-        o.firi = (float)(Rd.firi - di);
-        o.firb = (float)(Rd.firb + gi * dg + fi * di);
+        const double dg = wg * X.zir_gi.lo() * (ng - old[3]), di = wi * X.zir_gi.hi() * (ni - old[4]);
+        o.firg = (float)(X.fir_gi.lo() - dg);
+        o.firi = (float)(X.fir_gi.hi() - di);
+        o.firb = (float)(X.firb + gi * dg + fi * di);
         o.fvapuw = (float)fvapuw; o.fvaput = (float)fvaput; o.fvaps = (float)fvaps;
         o.fvaplw = (float)fvaplw; o.fvaplt = (float)fvaplt; o.fvapg = (float)fvapg; o.fvapi = (float)fvapi;
-        o.ginvap = (float)(fvapuw * X.xu + fvaps * X.xs + fvaplw * X.xl);
+        o.ginvap = (float)(fvapuw * X.x_us.lo() + fvaps * X.x_us.hi() + fvaplw * X.xl);
         o.gsuvap = (float)(fvapg * gi + fvapi * fi);
         o.gtrans = (float)(fvaput * 2.0 * S(IBIS_STAT_LAI, 1) * S(IBIS_STAT_FU) +
                            fvaplt * 2.0 * S(IBIS_STAT_LAI, 0) * S(IBIS_STAT_FL) * gi);
@@ -946,76 +969,112 @@ __device__ __forceinline__ void soil_stress32(SoilHour& G, const Col32& c, const
     G.stresstu = tot.hi();
 }
 
-// Steps 1-9 of timestep_body (see surface_phase, ibis_step.cuh)
-template <bool SUN_U, bool SUN_L, typename Q, typename D32>
-__device__ __forceinline__ void surface_phase32(Col32& c, const Forc32& F, const Stat32& S, const D32& D,
+// Steps 1-9 of timestep_body (see surface_phase, ibis_step.cuh); y: the hour's record
+// in shared memory
+template <bool SUN_U, bool SUN_L, typename Y, typename Q, typename D32>
+__device__ __forceinline__ void surface_phase32(Col32& c, Y& y, const Forc32& F, const Stat32& S, const D32& D,
                                                 const Par32& P, const Q& q, Mid<float>& M, SoilHour& G) {
     const float eps = P.epsilon;
     const float fi = c.fi;
-    const float lai0 = S(IBIS_STAT_LAI, 0), lai1 = S(IBIS_STAT_LAI, 1);
-    const float sai0 = S(IBIS_STAT_SAI, 0), sai1 = S(IBIS_STAT_SAI, 1);
-    const float fu = S(IBIS_STAT_FU), fl = S(IBIS_STAT_FL);
-    float hvasug, hvasui;
-    evap_sources(c, F, P, G.q1, G.q2, G.q3, G.q4, hvasug, hvasui);
-    G.consoi0 = conductivity32<Q::x3>(S, P, 0, S(IBIS_STAT_POROS, 0), c.wsoi[0], c.wisoi[0]);
-
-    // ---- 2-3. wet fractions and radiation (loops.py:331-354)
-    Rad<float> Rd;
-    {
-        float fwu, fws, fwl, rlu, rls, rll;
-        wet_fraction(c.tu, c.wliqu, c.wsnou, q.wliqumax(), P.wsnoumax, q.fmax(), P, fwu, rlu);
-        wet_fraction(c.ts, c.wliqs, c.wsnos, q.wliqsmax(), P.wsnosmax, q.fmax(), P, fws, rls);
-        wet_fraction(c.tl, c.wliql, c.wsnol, q.wliqlmax(), P.wsnolmax, q.fmax(), P, fwl, rll);
-        radiation(Rd, c, F, S, fwu, fws, fwl, rlu, rls, rll, P);
-    }
-
-    // ---- 4-5. precipitation cascade and wet fractions after it (loops.py:359-389)
+    TvHour& X = y.X;
     Casc<float> C;
-    cascade32(C, c, F, S, P, q);
-    TvHour X;
-    wet_fraction(c.tu, C.wliqu, C.wsnou, q.wliqumax(), P.wsnoumax, q.fmax(), P, X.fwetu, X.rliqu);
-    wet_fraction(c.ts, C.wliqs, C.wsnos, q.wliqsmax(), P.wsnosmax, q.fmax(), P, X.fwets, X.rliqs);
-    wet_fraction(c.tl, C.wliql, C.wsnol, q.wliqlmax(), P.wsnolmax, q.fmax(), P, X.fwetl, X.rliql);
-
-    // ---- 6. canopy exchange (loops.py:396-611)
-    Aero32 A;
-    aero_geometry32(A, F, S, fi, P);
-    soil_stress32(G, c, S, P, q);
-    float chgx, wlgx, wigx;
+    Turc tc;
     {
-        const float csoi0 = S(IBIS_STAT_CSOI, 0) > 0.0f ? S(IBIS_STAT_CSOI, 0) : P.csoi_mineral_val;
-        const float rhosoi0 = S(IBIS_STAT_RHOSOI, 0) > 0.0f ? S(IBIS_STAT_RHOSOI, 0) : P.rhosoi_val;
-        X.xu = 2.0f * lai1 * fu;
-        X.xs = 2.0f * sai1 * fu;
+        const float lai0 = S(IBIS_STAT_LAI, 0), lai1 = S(IBIS_STAT_LAI, 1);
+        const float sai0 = S(IBIS_STAT_SAI, 0), sai1 = S(IBIS_STAT_SAI, 1);
+        const float fu = S(IBIS_STAT_FU), fl = S(IBIS_STAT_FL);
+        float hvasug, hvasui;
+        evap_sources(c, F, P, G.q1, G.q2, G.q3, G.q4, hvasug, hvasui);
+        G.consoi0 = conductivity32<Q::x3>(S, P, 0, S(IBIS_STAT_POROS, 0), c.wsoi[0], c.wisoi[0]);
+        X.hv_gi = F2(hvasug, hvasui);
+
+        // ---- 2-3. wet fractions and radiation (loops.py:331-354)
+        Rad<float> Rd;
+        {
+            float fwu, fws, fwl, rlu, rls, rll;
+            wet_fraction(c.tu, c.wliqu, c.wsnou, q.wliqumax(), P.wsnoumax, q.fmax(), P, fwu, rlu);
+            wet_fraction(c.ts, c.wliqs, c.wsnos, q.wliqsmax(), P.wsnosmax, q.fmax(), P, fws, rls);
+            wet_fraction(c.tl, c.wliql, c.wsnol, q.wliqlmax(), P.wsnolmax, q.fmax(), P, fwl, rll);
+            radiation(Rd, c, F, S, fwu, fws, fwl, rlu, rls, rll, P);
+        }
+        X.sol_gi = F2(Rd.solg, Rd.soli);
+        X.fir_gi = F2(Rd.firg, Rd.firi);
+        X.firb = Rd.firb;
+        X.frad_us = F2(lai1 > eps ? (Rd.solu + Rd.firu) / (2.0f * lai1) : 0.0f,
+                       sai1 > eps ? (Rd.sols + Rd.firs) / (2.0f * sai1) : 0.0f);
+        X.fradl = (lai0 + sai0) > eps ? (Rd.soll + Rd.firl) / (2.0f * (lai0 + sai0)) : 0.0f;
+        X.toppar = F2(Rd.topparu, Rd.topparl);
+        X.scale = light_scaling2(Rd, F2(lai1, lai0), F2(sai1, sai0), c,
+                                 Q::x3 && (P.flags & IBIS_FLAG_LEAF_ONLY) != 0, P);
+        if constexpr (SUN_U) {
+            const SunShade<float> ss = sunshade(Rd.scu, Rd.dbeamu, Rd.termu6, Rd.termu7, lai1, sai1, P);
+            const float r = lai1 > 0.0f ? 1.0f / mx(lai1, 1.0e-6f) : 0.0f;    // rates per leaf area
+            y.su = Sun4{F2(ss.psun, ss.psha) * r, F2(ss.vsun, ss.vsha) * r};
+        }
+        if constexpr (SUN_L) {
+            const SunShade<float> ss = sunshade(Rd.scl, Rd.dbeaml, Rd.terml6, Rd.terml7, lai0, sai0, P);
+            const float r = lai0 > 0.0f ? 1.0f / mx(lai0, 1.0e-6f) : 0.0f;
+            y.sl = Sun4{F2(ss.psun, ss.psha) * r, F2(ss.vsun, ss.vsha) * r};
+        }
+        // the big leaves' nominal capacities (stomata.py:592-660)
+        if constexpr (Q::x3) {
+            float vu[2], ju[2], mu[2], vl[3], jl[3], ml[3];
+            bool jon = false;
+            big_leaves<float, false>(vu, ju, mu, jon, S, P, q);
+            big_leaves<float, true>(vl, jl, ml, jon, S, P, q);
+            X.vnu = F2(vu[0], vu[1]); y.cmu = F2(mu[0], mu[1]); y.jfu = F2(ju[0], ju[1]);
+            y.vnl = F2(vl[0], vl[1]); y.cml = F2(ml[0], ml[1]); y.jfl = F2(jl[0], jl[1]);
+            y.vn4 = vl[2]; y.cm4 = ml[2]; y.jf4 = jl[2];
+            y.cap = F2(capacity_integral(lai1, P.cap_kn), capacity_integral(lai0, P.cap_kn));
+        } else {
+            X.vnu = F2(S(IBIS_STAT_EXIST, 0) > 0.5f ? q.vmax(0) : (S(IBIS_STAT_EXIST, 2) > 0.5f ? q.vmax(2) : q.vmax(4)),
+                       S(IBIS_STAT_EXIST, 3) > 0.5f ? q.vmax(3) : q.vmax(5));
+        }
+        if (D.on()) radiation_diagnostics(D, Rd);
+
+        // ---- 4-5. precipitation cascade and wet fractions after it (loops.py:359-389)
+        cascade32(C, c, F, S, P, q);
+        float fwu, fws, rlu, rls;
+        wet_fraction(c.tu, C.wliqu, C.wsnou, q.wliqumax(), P.wsnoumax, q.fmax(), P, fwu, rlu);
+        wet_fraction(c.ts, C.wliqs, C.wsnos, q.wliqsmax(), P.wsnosmax, q.fmax(), P, fws, rls);
+        wet_fraction(c.tl, C.wliql, C.wsnol, q.wliqlmax(), P.wsnolmax, q.fmax(), P, X.fwetl, X.rliql);
+        X.fw_us = F2(fwu, fws);
+        X.rl_us = F2(rlu, rls);
+        X.pf_us = F2(C.pfluxu, C.pfluxs);
+        X.pfluxl = C.pfluxl;
+
+        // ---- 6. canopy exchange (loops.py:396-611)
+        float cp;
+        aero_geometry32(y.A, tc, cp, F, S, fi, P);
+        soil_stress32(G, c, S, P, q);
+        X.stress = F2(G.stresstu, G.stresstl);
+        const float cs = S(IBIS_STAT_CSOI, 0), rs = S(IBIS_STAT_RHOSOI, 0);
+        const float csoi0 = cs > 0.0f ? cs : P.csoi_mineral_val, rhosoi0 = rs > 0.0f ? rs : P.rhosoi_val;
+        X.cp = cp;
+        X.ta = F.ta; X.qa = F.qa; X.ps = F.ps; X.fi = fi;
+        X.x_us = F2(lai1, sai1) * (2.0f * fu);
         X.xl = 2.0f * (lai0 + sai0) * fl * (1.0f - fi);
-        X.fi = fi;
-        X.cog = G.consoi0 / mx(0.5f * P.hsoi[0], eps);
-        X.coi = P.consno / mx(0.5f * mx(c.hsno[0], P.hsnotop), eps);
-        X.zirg = P.zir * cube(c.tg);
-        X.ziri = P.zir * cube(c.ti);
+        X.co_gi = F2(G.consoi0 / mx(0.5f * P.hsoi[0], eps), P.consno / mx(0.5f * mx(c.hsno[0], P.hsnotop), eps));
+        const F2 tgi(c.tg, c.ti);
+        X.zir_gi = tgi * (tgi * tgi) * P.zir;
         const float p0 = S(IBIS_STAT_POROS, 0), w0 = c.wsoi[0], i0 = c.wisoi[0];
         const float rwp = p0 * P.rhow, liq = rwp * (1.0f - i0) * w0, ice = rwp * i0;
-        chgx = P.ch2o * c.wpud + P.cice * c.wipud +
-               ((1.0f - p0) * csoi0 * rhosoi0 + liq * P.ch2o + ice * P.cice) * P.hsoi[0];
-        wlgx = c.wpud + liq * P.hsoi[0];
-        wigx = c.wipud + ice * P.hsoi[0];
-        X.wu = C.wliqu + C.wsnou; X.ws = C.wliqs + C.wsnos; X.wl = C.wliql + C.wsnol;
-        X.chux = P.chu + P.ch2o * C.wliqu + P.cice * C.wsnou;
-        X.chsx = P.chs + P.ch2o * C.wliqs + P.cice * C.wsnos;
-        X.chlx = P.chl + P.ch2o * C.wliql + P.cice * C.wsnol;
-        X.hvasug = hvasug; X.hvasui = hvasui;
-        X.tsoi0 = c.tsoi[0]; X.tsno0 = c.tsno[0];
+        const float chg = P.ch2o * c.wpud + P.cice * c.wipud +
+                          ((1.0f - p0) * csoi0 * rhosoi0 + liq * P.ch2o + ice * P.cice) * P.hsoi[0];
+        X.wl_us = F2(C.wliqu, C.wliqs);
+        X.ws_us = F2(C.wsnou, C.wsnos);
+        X.wl_lg = F2(C.wliql, c.wpud + liq * P.hsoi[0]);
+        X.ws_lg = F2(C.wsnol, c.wipud + ice * P.hsoi[0]);
+        X.ch_us = F2(P.chu, P.chs) + X.wl_us * P.ch2o + X.ws_us * P.cice;
+        X.ch_lg = F2(P.chl + P.ch2o * C.wliql + P.cice * C.wsnol, chg);
         const float zwp = clip(0.5f * (c.wpud + c.wipud) / mx(P.wpudmax, eps), 0.0f, 0.5f);
         const float zws = (1.0f - i0) * w0 + i0;
         const float zwtot = zwp + (1.0f - zwp) * zws;
         X.psig = -P.grav * S(IBIS_STAT_SUCTION, 0) * pw(zwtot, -S(IBIS_STAT_BEX, 0));
         const double sw0 = S(IBIS_STAT_SWILT, 0);
-        X.betaw = clip(((double)zwtot - sw0) * rcp_nr(fmax(1.0 - sw0, (double)eps)), 0.0, 1.0);
-        if (q.beta_power() != 1.0f) X.betaw = (double)pw((float)X.betaw, q.beta_power());
-        X.fradu = lai1 > eps ? (Rd.solu + Rd.firu) / (2.0f * lai1) : 0.0f;
-        X.frads = sai1 > eps ? (Rd.sols + Rd.firs) / (2.0f * sai1) : 0.0f;
-        X.fradl = (lai0 + sai0) > eps ? (Rd.soll + Rd.firl) / (2.0f * (lai0 + sai0)) : 0.0f;
-        X.pfluxu = C.pfluxu; X.pfluxs = C.pfluxs; X.pfluxl = C.pfluxl;
+        double betaw = clip(((double)zwtot - sw0) * rcp_nr(fmax(1.0 - sw0, (double)eps)), 0.0, 1.0);
+        if (q.beta_power() != 1.0f) betaw = (double)pw((float)betaw, q.beta_power());
+        X.betaw = betaw;
         auto fr = [&](int j) { return (double)S(IBIS_STAT_FRAC, j); };
         X.fb = fr(0) + fr(1) + fr(2) + fr(4) + fr(6) + fr(7);
         X.fc = fr(3) + fr(5);
@@ -1024,54 +1083,56 @@ __device__ __forceinline__ void surface_phase32(Col32& c, const Forc32& F, const
     }
     double Wv[9] = {(double)c.tu, (double)c.ts, (double)c.tl, (double)c.t12, (double)c.t34,
                     (double)c.q12, (double)c.q34, (double)c.tg, (double)c.ti};
-    Turc tc;
-    tc.u2 = A.u0.lo();
-    tc.alb = A.alb;
-    tc.sm = tc.sh = F2(1.0f);
     F2 wus(1.0f), wlg(1.0f);      // implicit weights of the canopy's and of the lower canopy's and ground's temperatures
     float wi = 1.0f;
     Stom<float> st;
     TvResult tv;
 #pragma unroll 1
     for (int it = 0; it < 3; ++it) {
+        asm volatile("" ::: "memory");     // read the hour's record again in each pass instead of keeping it in registers
         const bool first = (it == 0);
         const float tu = (float)Wv[0], ts = (float)Wv[1], tl = (float)Wv[2];
         const F2 tair((float)Wv[3], (float)Wv[4]), qair((float)Wv[5], (float)Wv[6]);
         Trans<float> T;
-        transfer32(T, tc, A, tair.lo(), tair.hi(), qair.lo(), qair.hi(), first, P);
-        const F2 eair = esat2(tair), qsair = qsat2(eair, F.ps);
-        stomata32<SUN_U, SUN_L>(st, c, tu, tl, tair, qair, qsair, T.su, T.sl, Rd, X.fwetu, X.fwetl, S, G.stresstu,
-                                G.stresstl, P, q);
+        transfer32(T, tc, y.A, tair.lo(), tair.hi(), qair.lo(), qair.hi(), first, P);
+        const F2 eair = esat2(tair), qsair = qsat2(eair, X.ps);
+        stomata32<SUN_U, SUN_L>(st, c, tu, tl, qair, qsair, T.su, T.sl, y, P, q);
         if (!first) {
             const float tg = (float)Wv[7], ti = (float)Wv[8];
-            wus = weight_veg2(F2(tu, ts), F2(X.chux, X.chsx), F2(C.wliqu, C.wliqs), F2(C.wsnou, C.wsnos), wus, P);
-            wlg = weight_veg2(F2(tl, tg), F2(X.chlx, chgx), F2(C.wliql, wlgx), F2(C.wsnol, wigx), wlg, P);
+            wus = weight_veg2(F2(tu, ts), X.ch_us, X.wl_us, X.ws_us, wus, P);
+            wlg = weight_veg2(F2(tl, tg), X.ch_lg, X.wl_lg, X.ws_lg, wlg, P);
             wi = weight_snow(ti, c.ti, wi, false, P);
         }
-        turvap32(Wv, tv, c, T, A.cp, wus, wlg, wi, X, st, F, Rd, S, eair.hi(), qsair.hi(), it == 2, P, q);
+        turvap32(Wv, tv, c, T, wus, wlg, wi, X, st, S, eair.hi(), qsair.hi(), it == 2, P);
     }
     const float ti_new = mn((float)Wv[8], P.tmelt);
     const float tg_w = (float)Wv[7];
 
     // ---- 7-8. evaporation of intercepted water, bare-story reset (loops.py:616-640)
     float tu = (float)Wv[0], ts = (float)Wv[1], tl = (float)Wv[2];
-    float wliqu = C.wliqu, wliqs = C.wliqs, wliql = C.wliql, wsnou = C.wsnou, wsnos = C.wsnos, wsnol = C.wsnol;
-    evap_intercepted(tu, wliqu, wsnou, X.rliqu, tv.fvapuw, P.chu, P);
-    evap_intercepted(ts, wliqs, wsnos, X.rliqs, tv.fvaps, P.chs, P);
+    float wliqu = X.wl_us.lo(), wliqs = X.wl_us.hi(), wliql = X.wl_lg.lo();
+    float wsnou = X.ws_us.lo(), wsnos = X.ws_us.hi(), wsnol = X.ws_lg.lo();
+    evap_intercepted(tu, wliqu, wsnou, X.rl_us.lo(), tv.fvapuw, P.chu, P);
+    evap_intercepted(ts, wliqs, wsnos, X.rl_us.hi(), tv.fvaps, P.chs, P);
     evap_intercepted(tl, wliql, wsnol, X.rliql, tv.fvaplw, P.chl, P);
     {
         const float tav = (1.0f - fi) * tg_w + fi * ti_new;
-        if (lai1 == 0.0f || fu == 0.0f) { tu = tav; wliqu = 0.0f; wsnou = 0.0f; }
-        if (sai1 == 0.0f || fu == 0.0f) { ts = tav; wliqs = 0.0f; wsnos = 0.0f; }
-        if (2.0f * (lai0 + sai0) == 0.0f || fl * (1.0f - fi) == 0.0f) { tl = tav; wliql = 0.0f; wsnol = 0.0f; }
+        const F2 x_us = X.x_us;
+        if (x_us.lo() == 0.0f) { tu = tav; wliqu = 0.0f; wsnou = 0.0f; }
+        if (x_us.hi() == 0.0f) { ts = tav; wliqs = 0.0f; wsnos = 0.0f; }
+        if (2.0f * (S(IBIS_STAT_LAI, 0) + S(IBIS_STAT_SAI, 0)) == 0.0f || S(IBIS_STAT_FL) * (1.0f - fi) == 0.0f) {
+            tl = tav;
+            wliql = 0.0f;
+            wsnol = 0.0f;
+        }
     }
 
     // ---- 9. surface fluxes into soil and snow (loops.py:665-674)
     const float fm = P.flux_max;
     M.fvapg = tv.fvapg;
     M.fvapi = tv.fvapi;
-    M.heatg = Rd.solg + clip(tv.firg, -fm, fm) - clip(tv.fseng, -fm, fm) - hvasug * M.fvapg;
-    M.heati = Rd.soli + clip(tv.firi, -fm, fm) - clip(tv.fseni, -fm, fm) - hvasui * M.fvapi;
+    M.heatg = X.sol_gi.lo() + clip(tv.firg, -fm, fm) - clip(tv.fseng, -fm, fm) - X.hv_gi.lo() * M.fvapg;
+    M.heati = X.sol_gi.hi() + clip(tv.firi, -fm, fm) - clip(tv.fseni, -fm, fm) - X.hv_gi.hi() * M.fvapi;
     M.fvaput = tv.fvaput;
     M.fvaplt = tv.fvaplt;
     M.ginvap = tv.ginvap;
@@ -1093,9 +1154,9 @@ __device__ __forceinline__ void surface_phase32(Col32& c, const Forc32& F, const
 
     // ---- diagnostics of the surface phase (loops.py:1158-1241)
     if (D.on()) {
-        surface_diagnostics(D, st, X.fwetu, X.fwets, X.fwetl, X.rliqu, X.rliqs, X.rliql, Rd, tv.firg, tv.firi, tv.firb,
-                            tv.fsenu, tv.fsens, tv.fsenl, tv.fseng, tv.fseni, M, A.rhoa, hvasug, hvasui, G.q1, G.q2,
-                            G.q3, G.q4);
+        surface_diagnostics(D, st, X.fw_us.lo(), X.fw_us.hi(), X.fwetl, X.rl_us.lo(), X.rl_us.hi(), X.rliql, tv.firg,
+                            tv.firi, tv.firb, tv.fsenu, tv.fsens, tv.fsenl, tv.fseng, tv.fseni, M, y.A.rhoa,
+                            X.hv_gi.lo(), X.hv_gi.hi(), G.q1, G.q2, G.q3, G.q4);
     }
 }
 

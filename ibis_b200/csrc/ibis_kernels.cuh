@@ -26,11 +26,12 @@ struct LaunchConfig {
 };
 constexpr LaunchConfig kConfigs[] = {
     {0, 128, 2, 0, 0}, {0, 64, 4, 0, 0},  {0, 96, 2, 0, 0},    {0, 128, 3, 0, 0},
-    {0, 160, 1, 0, 0}, {0, 192, 1, 0, 0}, {0, 224, 1, 0, 0},   {0, 256, 1, 0, 0},
+    {0, 32, 8, 0, 0},  {0, 192, 1, 0, 0}, {0, 224, 1, 0, 0},   {0, 256, 1, 0, 0},
     {1, 128, 2, 128, 3}, {1, 256, 1, 256, 2}, {1, 128, 3, 128, 4}, {2, 224, 1, 0, 0}};
 constexpr int kNumConfigs = sizeof(kConfigs) / sizeof(kConfigs[0]);
 constexpr int kDefaultFused = 0;
-constexpr int kLongFused = 6;      // ibis_step_f32's choice for launches of kAccSmemMinSteps hours or more
+constexpr int kLongFused = 6;
+constexpr int kSmallFused = 4;
 constexpr int kDefaultSplit = 8;
 
 // FP32 kernels keep each column's prognostic state in shared memory (array of
@@ -164,11 +165,26 @@ constexpr size_t kAccChipBytes = 2 * kAccPairs * sizeof(float2);
 // kAccSmemMinSteps hours keep them in global memory instead (ACCSM = false):
 // the on-chip copy only pays back over several hours, and the larger
 // shared-memory carveout leaves less L1 for the register spills.
-template <typename R, int BLOCK, int MINB, bool ACCSM = true>
+template <typename R, int BLOCK, int MINB, bool ACCSM = true, size_t HOUR = sizeof(HourScratch<false, false>)>
 struct AccInSmem {
     static constexpr bool value =
         ACCSM && StateInSmem<R>::value &&
-        ((sizeof(Col<R>) + kAccChipBytes) * BLOCK + 1024) * MINB <= 228 * 1024;
+        ((sizeof(Col<R>) + kAccChipBytes + HOUR) * BLOCK + 1024) * MINB <= 228 * 1024;
+};
+
+// A block's shared memory in the FP32 kernels: the columns' state, the on-chip
+// accumulators (with ACC), the records of the hour (HourScratch).
+template <typename R, bool SUN, bool X3, int BLOCK, bool ACC>
+struct BlockSmem {
+    using Hour = HourScratch<SUN, X3>;
+    static constexpr bool on = StateInSmem<R>::value;
+    static constexpr size_t acc_off = (size_t)BLOCK * sizeof(Col<R>);
+    static constexpr size_t hour_off = acc_off + (ACC ? (size_t)BLOCK * kAccChipBytes : 0);
+    static constexpr size_t total = on ? hour_off + (size_t)BLOCK * sizeof(Hour) : 0;
+    static_assert(acc_off % 8 == 0 && hour_off % 8 == 0, "64-bit words");
+    static __device__ __forceinline__ Hour& hour(unsigned char* smem) {
+        return reinterpret_cast<Hour*>(smem + hour_off)[threadIdx.x];
+    }
 };
 constexpr int kAccSmemMinSteps = 4;
 
@@ -180,6 +196,19 @@ __device__ __forceinline__ auto uniform_source(const DevParams<R>& P) {
     else return UniformQ<R>{P};
 }
 
+// The block's `n` threads (whole warps) start an hour together.  A warp that follows
+// another closely finds its instructions in the SM's instruction cache; warps spread
+// over the body each stream it from the next level (six hours of 33,152 columns: 0.146
+// ms together, 0.157 without in blocks of 64).  Once an hour is enough: a warp that
+// falls behind fetches faster than the one it follows.
+template <bool ON>
+__device__ __forceinline__ void align_warps(unsigned n) {
+    if constexpr (ON) {
+        __syncwarp();
+        asm volatile("barrier.sync 0, %0;" ::"r"(n) : "memory");
+    }
+}
+
 // Status word written by the kernels: [0] bit 0 = a column left the step with a
 // non-finite prognostic value; [1] = smallest such cell index (INT_MAX if none).
 // DG: whether the kernel can write diagnostics.
@@ -189,8 +218,14 @@ __global__ void __launch_bounds__(BLOCK, MINB) hourly_step_kernel(R* __restrict_
                                                              R* __restrict__ acc, int ncell, int ld, int nstep,
                                                              long long forc_stride, const DevParams<R> P,
                                                              int* __restrict__ status) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= ncell) return;
+    // A lane past the batch's end repeats the last cell, writing nothing, so that every
+    // warp is whole at the hours' barriers; warps past it take no part in them.
+    const int i0 = blockIdx.x * BLOCK;
+    const int nlive = ncell - i0 < BLOCK ? ncell - i0 : BLOCK;
+    const unsigned nbar = (unsigned)(nlive + 31) & ~31u;
+    if (threadIdx.x >= nbar) return;
+    const bool live = (int)threadIdx.x < nlive;
+    const int i = live ? i0 + (int)threadIdx.x : ncell - 1;
     extern __shared__ unsigned char smem_raw[];
     Col<R> creg;
     Col<R>* cp;
@@ -199,19 +234,24 @@ __global__ void __launch_bounds__(BLOCK, MINB) hourly_step_kernel(R* __restrict_
     Col<R>& c = *cp;
     load_col(c, prog + i, ld);
     Stat<R> S{stat + i, ld};
-    const Diag<R, DG> D{DG && diag ? diag + i : nullptr, ld};
-    constexpr bool kAccSmem = AccInSmem<R, BLOCK, MINB, ACCSM>::value;
+    const Diag<R, DG> D{DG && diag && live ? diag + i : nullptr, ld};
+    constexpr bool kAccSmem = AccInSmem<R, BLOCK, MINB, ACCSM, sizeof(HourScratch<SU || SL, X3>)>::value;
+    using SM = BlockSmem<R, SU || SL, X3, BLOCK, kAccSmem>;
     Acc<R, kAccSmem ? BLOCK : 0> A{acc ? acc + i : nullptr, ld, (P.flags & IBIS_FLAG_KAHAN) != 0};
+    A.live = live;
     if constexpr (kAccSmem) {
-        A.chip = reinterpret_cast<float2*>(smem_raw + BLOCK * sizeof(Col<R>)) + threadIdx.x;
+        A.chip = reinterpret_cast<float2*>(smem_raw + SM::acc_off) + threadIdx.x;
         if (acc) acc_move<true>(acc + i, ld, A.chip, BLOCK, P.flags);
     }
 #pragma unroll 1
     for (int s = 0; s < nstep; ++s) {
+        align_warps<StateInSmem<R>::value && (BLOCK > 32)>(nbar);
         Forc<R> F = load_forc(forc + (size_t)s * forc_stride + i, ld);
         A.last = (s + 1 == nstep);
-        column_step<R, NT, SU, SL>(c, F, S, D, A, P, uniform_source<R, X3>(P));
+        S.renew();
+        column_step<R, NT, SU, SL>(c, SM::hour(smem_raw), F, S, D, A, P, uniform_source<R, X3>(P));
     }
+    if (!live) return;
     if constexpr (kAccSmem) {
         if (acc) acc_move<false>(acc + i, ld, A.chip, BLOCK, P.flags);
     }
@@ -309,13 +349,12 @@ __device__ __forceinline__ Forc<R> read_forc_tile(const R* t, int block) {
     return F;
 }
 
-// The staged kernel's shared memory: column state, the on-chip accumulators,
-// then the forcing tile and its barriers (16-byte aligned).
-template <typename R, int BLOCK, int MINB>
+// The staged kernel's shared memory: the fused kernel's, then the forcing tile and
+// its barriers (16-byte aligned).
+template <typename R, bool SUN, bool X3, int BLOCK, int MINB>
 struct StagedSmem {
-    static constexpr size_t col = (size_t)BLOCK * sizeof(Col<R>);
-    static constexpr size_t acc = (size_t)BLOCK * kAccChipBytes;
-    static constexpr size_t stage_off = (col + acc + 15) / 16 * 16;
+    using Block = BlockSmem<R, SUN, X3, BLOCK, true>;
+    static constexpr size_t stage_off = (Block::total + 15) / 16 * 16;
     static constexpr size_t total = stage_off + ForcStage<R, BLOCK>::bytes;
 };
 
@@ -332,8 +371,9 @@ __global__ void __launch_bounds__(BLOCK, MINB) hourly_step_staged_kernel(
     R* __restrict__ prog, const R* __restrict__ stat, const R* __restrict__ forc, R* __restrict__ acc, int ncell,
     int ld, int nstep, long long forc_stride, const DevParams<R> P, int* __restrict__ status) {
     static_assert(sizeof(R) == 4 && StateInSmem<R>::value, "the staged form is the FP32 shared-memory kernel");
-    static_assert(AccInSmem<R, BLOCK, MINB>::value, "the staged form keeps the accumulators on chip");
-    using SM = StagedSmem<R, BLOCK, MINB>;
+    static_assert(AccInSmem<R, BLOCK, MINB, true, sizeof(HourScratch<SU || SL, X3>)>::value,
+                  "the staged form keeps the accumulators on chip");
+    using SM = StagedSmem<R, SU || SL, X3, BLOCK, MINB>;
     static_assert((SM::total + 1024) * MINB <= 228 * 1024, "staged shared memory exceeds the SM");
     extern __shared__ __align__(16) unsigned char smem_raw[];
     // fixed offsets from the shared-memory base, so none of them holds a register across the hour
@@ -367,7 +407,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) hourly_step_staged_kernel(
     Stat<R> S{stat + i, ld};
     const Diag<R, false> D{nullptr, ld};
     Acc<R, BLOCK> A{acc ? acc + i : nullptr, ld, (P.flags & IBIS_FLAG_KAHAN) != 0};
-    A.chip = reinterpret_cast<float2*>(smem_raw + SM::col) + threadIdx.x;
+    A.chip = reinterpret_cast<float2*>(smem_raw + SM::Block::acc_off) + threadIdx.x;
     if (acc) acc_move<true>(acc + i, ld, A.chip, BLOCK, P.flags);
 #pragma unroll 1
     for (int s = 0; s < nstep; ++s) {
@@ -384,7 +424,8 @@ __global__ void __launch_bounds__(BLOCK, MINB) hourly_step_staged_kernel(
             }
         }
         A.last = (s + 1 == nstep);
-        column_step<R, NT, SU, SL>(c, F, S, D, A, P, uniform_source<R, X3>(P));
+        S.renew();
+        column_step<R, NT, SU, SL>(c, SM::Block::hour(smem_raw), F, S, D, A, P, uniform_source<R, X3>(P));
     }
     if (acc) acc_move<false>(acc + i, ld, A.chip, BLOCK, P.flags);
     R sum = store_col(c, prog + i, ld);
@@ -422,7 +463,8 @@ __global__ void __launch_bounds__(BLOCK, MINB) surface_kernel(R* __restrict__ pr
     Forc<R> F = load_forc(forc + i, ld);
     Mid<R> M;
     SoilHour G;      // formed again by the ground kernel
-    surface_phase32<SU, SL>(c, F, S, D, P, uniform_source<R, X3>(P), M, G);
+    surface_phase32<SU, SL>(c, BlockSmem<R, SU || SL, X3, BLOCK, false>::hour(smem_raw), F, S, D, P,
+                            uniform_source<R, X3>(P), M, G);
     mid_store(M, mid + i, ld);
     store_col(c, prog + i, ld);
 }
@@ -513,6 +555,9 @@ static DevParams<R> make_dev_params(const IbisParams& h) {
     d.rbeta3 = (R)(1.0 / h.beta3);
     d.rtheta4 = (R)(1.0 / h.theta4);
     d.rbeta4 = (R)(1.0 / h.beta4);
+    d.ksu = (R)(h.cleaf * sqrt(1.0 / h.dleaf[1]));
+    d.kss = (R)(h.cstem * sqrt(1.0 / h.dstem[1]));
+    d.ksl = (R)(h.cgrass * sqrt(1.0 / h.dleaf[0]));
     for (int k = 1; k < NL; ++k) {
         d.hs_below[k] = (R)(h.hsoi[k] / (h.hsoi[k - 1] + h.hsoi[k]));
         d.hs_above[k] = (R)(h.hsoi[k - 1] / (h.hsoi[k - 1] + h.hsoi[k]));
@@ -610,12 +655,12 @@ template <typename R, int NT, bool SU, bool SL, int BLOCK, int MINB, bool ACCSM,
 cudaError_t launch_fused(R* prog, const R* stat, const R* forc, R* diag, R* acc, int ncell, int ld, int nstep,
                          long long fstride, const DevParams<R>& P, int* status, cudaStream_t s) {
     const int grid = (ncell + BLOCK - 1) / BLOCK;
-    const size_t col_smem = StateInSmem<R>::value ? BLOCK * sizeof(Col<R>) : 0;
-    const size_t acc_smem = AccInSmem<R, BLOCK, MINB, ACCSM>::value ? BLOCK * kAccChipBytes : 0;
-    const size_t smem = col_smem + acc_smem;
+    constexpr size_t smem =
+        BlockSmem<R, SU || SL, X3, BLOCK,
+                  AccInSmem<R, BLOCK, MINB, ACCSM, sizeof(HourScratch<SU || SL, X3>)>::value>::total;
     auto k = hourly_step_kernel<R, NT, SU, SL, BLOCK, MINB, ACCSM, X3, DG>;
     static unsigned long long fitted = 0;
-    cudaError_t e = fit_smem_once(fitted, k, BLOCK, col_smem + acc_smem, col_smem + acc_smem);
+    cudaError_t e = fit_smem_once(fitted, k, BLOCK, smem, smem);
     if (e != cudaSuccess) return e;
     k<<<grid, BLOCK, smem, s>>>(prog, stat, forc, diag, acc, ncell, ld, nstep, fstride, P, status);
     return cudaGetLastError();
@@ -631,7 +676,7 @@ cudaError_t launch_staged(R* prog, const R* stat, const R* forc, R* acc, int nce
     if ((reinterpret_cast<uintptr_t>(forc) & 15) != 0 || (fstride & 3) != 0 || (ld & 3) != 0)
         return launch_fused<R, NT, SU, SL, BLOCK, MINB, true, X3, false>(prog, stat, forc, nullptr, acc, ncell, ld,
                                                                          nstep, fstride, P, status, s);
-    using SM = StagedSmem<R, BLOCK, MINB>;
+    using SM = StagedSmem<R, SU || SL, X3, BLOCK, MINB>;
     const int grid = (ncell + BLOCK - 1) / BLOCK;
     auto k = hourly_step_staged_kernel<R, NT, SU, SL, BLOCK, MINB, X3>;
     static unsigned long long fitted = 0;
@@ -645,7 +690,7 @@ template <typename R, int NT, bool SU, bool SL, int B1, int M1, int B2, int M2, 
 cudaError_t launch_split(R* prog, const R* stat, const R* forc, R* diag, R* acc, R* mid, int ncell, int ld,
                          int nstep, long long fstride, const DevParams<R>& P, int* status, cudaStream_t s) {
     const int g1 = (ncell + B1 - 1) / B1, g2 = (ncell + B2 - 1) / B2;
-    const size_t sm1 = StateInSmem<R>::value ? B1 * sizeof(Col<R>) : 0;
+    constexpr size_t sm1 = BlockSmem<R, SU || SL, X3, B1, false>::total;
     const size_t sm2 = StateInSmem<R>::value ? B2 * sizeof(Col<R>) : 0;
     auto k1 = surface_kernel<R, SU, SL, B1, M1, X3, DG>;
     auto k2 = ground_kernel<R, NT, B2, M2, X3, DG>;
@@ -661,15 +706,16 @@ cudaError_t launch_split(R* prog, const R* stat, const R* forc, R* diag, R* acc,
     return cudaGetLastError();
 }
 
-// Launches that write diagnostics run the default configuration of their form
-// (dispatch_config), the only ones compiled with the diagnostics writer; the
-// float64 kernels always carry it.
+// Launches that write diagnostics run the default configuration of their form, or
+// the small-batch one (dispatch_config): the only ones compiled with the diagnostics
+// writer; the float64 kernels always carry it.
 template <typename R, int NT, bool SU, bool SL, int CFG, bool X3 = false>
 cudaError_t run_config(R* prog, const R* stat, const R* forc, R* diag, R* acc, R* mid, int ncell, int ld, int nstep,
                        long long fs, const DevParams<R>& P, int* status, cudaStream_t s) {
     constexpr LaunchConfig C = kConfigs[CFG];
     if constexpr (sizeof(R) == 8) {
-        return launch_fused<R, NT, SU, SL, C.block, C.minb, false, X3, true>(prog, stat, forc, diag, acc, ncell, ld,
+        // single-warp blocks: as many warps fit an SM, and a small batch spreads over more SMs
+        return launch_fused<R, NT, SU, SL, 32, 8, false, X3, true>(prog, stat, forc, diag, acc, ncell, ld,
                                                                              nstep, fs, P, status, s);
     } else if constexpr (C.form == 0) {
 #define IBIS_FUSED(ACCSM, DG)                                                                                       \
@@ -680,6 +726,8 @@ cudaError_t run_config(R* prog, const R* stat, const R* forc, R* diag, R* acc, R
         if constexpr (CFG == kDefaultFused) {
             if (diag) return nstep < kAccSmemMinSteps ? IBIS_FUSED(false, true) : IBIS_FUSED(true, true);
             if (nstep < kAccSmemMinSteps) return IBIS_FUSED(false, false);
+        } else if constexpr (CFG == kSmallFused) {
+            if (diag) return IBIS_FUSED(true, true);
         }
         return IBIS_FUSED(true, false);
 #undef IBIS_FUSED
@@ -703,21 +751,38 @@ cudaError_t run_config(R* prog, const R* stat, const R* forc, R* diag, R* acc, R
 
 // Every (variant, configuration) pair the FP32 library instantiates: the F77
 // canopy (no sunlit/shaded split) in every configuration, the sunlit/shaded
-// variants in the two default ones.  X(NT, SU, SL, CFG).
+// variants in the default ones and the small-batch one.  X(NT, SU, SL, CFG).
 #define IBIS_F77_CONFIGS(X, NT)                                                                                \
     X(NT, false, false, 0) X(NT, false, false, 1) X(NT, false, false, 2) X(NT, false, false, 3)                \
     X(NT, false, false, 4) X(NT, false, false, 5) X(NT, false, false, 6) X(NT, false, false, 7)                \
     X(NT, false, false, 8) X(NT, false, false, 9) X(NT, false, false, 10) X(NT, false, false, 11)
 #define IBIS_SUN_CONFIGS(X, NT)                                                                                \
     X(NT, true, false, 0) X(NT, false, true, 0) X(NT, true, true, 0)                                           \
+    X(NT, true, false, 4) X(NT, false, true, 4) X(NT, true, true, 4)                                           \
     X(NT, true, false, 8) X(NT, false, true, 8) X(NT, true, true, 8)
-// The IBIS 3.0 kernels (X3): every canopy variant in the two default
-// configurations, and the long fused configuration for both canopies F77 or
-// both sunlit/shaded.  X(NT, SU, SL, CFG).
+// The IBIS 3.0 kernels (X3): every canopy variant in the same three, and the long
+// fused configuration for both canopies F77 or both sunlit/shaded.  X(NT, SU, SL, CFG).
 #define IBIS_X3_CONFIGS(X, NT)                                                                                 \
-    X(NT, false, false, 0) X(NT, false, false, 6) X(NT, false, false, 8)                                       \
-    X(NT, true, true, 0) X(NT, true, true, 6) X(NT, true, true, 8)                                             \
-    X(NT, true, false, 0) X(NT, true, false, 8) X(NT, false, true, 0) X(NT, false, true, 8)
+    X(NT, false, false, 0) X(NT, false, false, 4) X(NT, false, false, 6) X(NT, false, false, 8)                \
+    X(NT, true, true, 0) X(NT, true, true, 4) X(NT, true, true, 6) X(NT, true, true, 8)                        \
+    X(NT, true, false, 0) X(NT, true, false, 4) X(NT, true, false, 8)                                          \
+    X(NT, false, true, 0) X(NT, false, true, 4) X(NT, false, true, 8)
+
+// The fused configuration of a launch that leaves it to the library, by how its
+// columns fill the chip (`sms` SMs).  Six hours on 148 SMs, milliseconds in blocks of
+// 32 / 2 x 128 / 224: 356 columns for a day 0.41 / 0.43 / 0.49; 12,007 0.125 / 0.122 /
+// 0.136; 33,152 0.169 / 0.146 / 0.144; 95,333 0.452 / 0.434 / 0.424.
+//   * up to a warp per SM: single-warp blocks, so every warp has an SM's caches to itself;
+//   * up to four: blocks of 128, one on each SM before any gets a second;
+//   * otherwise 2 x 128 or 1 x 224 threads per SM, whichever runs the batch in less: a
+//     wave of either takes the same within 2 %, so the number of waves decides.
+//     Launches too short to keep the accumulators on chip have the 128 form.
+inline int auto_config(int ncell, int nstep, int sms) {
+    if (ncell <= 32 * sms) return kSmallFused;
+    if (nstep < kAccSmemMinSteps || ncell <= 128 * sms) return kDefaultFused;
+    const int w8 = (ncell - 1) / (256 * sms), w7 = (ncell - 1) / (224 * sms);
+    return w7 <= w8 ? kLongFused : kDefaultFused;
+}
 
 template <typename R, int NT, bool SU, bool SL, bool X3>
 cudaError_t dispatch_config(int cfg, R* prog, const R* stat, const R* forc, R* diag, R* acc, R* mid, int ncell,
@@ -728,14 +793,16 @@ cudaError_t dispatch_config(int cfg, R* prog, const R* stat, const R* forc, R* d
         // switches off they perform the F77 step's operations
         return run_config<R, NT, SU, SL, kDefaultFused, true>(IBIS_ARGS);
     } else if (diag) {
-        // only the default configurations are compiled with the diagnostics writer
+        if (cfg == kSmallFused) return run_config<R, NT, SU, SL, kSmallFused, X3>(IBIS_ARGS);
         if (kConfigs[cfg].form != 1) return run_config<R, NT, SU, SL, kDefaultFused, X3>(IBIS_ARGS);
         return run_config<R, NT, SU, SL, kDefaultSplit, X3>(IBIS_ARGS);
     } else if constexpr (X3) {
+        if (cfg == kSmallFused) return run_config<R, NT, SU, SL, kSmallFused, true>(IBIS_ARGS);
         if (cfg == kLongFused && SU == SL) return run_config<R, NT, SU, SL, kLongFused, true>(IBIS_ARGS);
         if (kConfigs[cfg].form != 1) return run_config<R, NT, SU, SL, kDefaultFused, true>(IBIS_ARGS);
         return run_config<R, NT, SU, SL, kDefaultSplit, true>(IBIS_ARGS);
     } else if constexpr (SU || SL) {
+        if (cfg == kSmallFused) return run_config<R, NT, SU, SL, kSmallFused>(IBIS_ARGS);
         if (kConfigs[cfg].form != 1) return run_config<R, NT, SU, SL, kDefaultFused>(IBIS_ARGS);
         return run_config<R, NT, SU, SL, kDefaultSplit>(IBIS_ARGS);
     } else {

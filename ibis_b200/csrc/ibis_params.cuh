@@ -51,6 +51,7 @@ struct DevParams {
     R rtdrip[3], rtblow[3];  // 1 / drip and blow-off times of the upper leaves, upper stems, lower canopy
     R kdrip[3], kblow[3];    // 1 - dtime / time
     R rtheta3, rbeta3, rtheta4, rbeta4;
+    R ksu, kss, ksl;         // boundary-layer conductances of leaves, stems and lower canopy over rhoa sqrt(u)
     R hs_below[6], hs_above[6];   // interface k (1..5): h[k] and h[k-1] over h[k-1] + h[k]
     R bed_res[3];            // bedrock layer: half its thermal resistance
     R bed_con[3];            // conductance to the layer below

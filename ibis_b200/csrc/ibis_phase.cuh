@@ -184,10 +184,23 @@ __device__ __forceinline__ void capacity_group(const int (&idx)[N], const Stat<R
     twm = mx(tw, R(1.0e-12));
 }
 
+// ---- diagnostics of the radiation (loops.py:1158-1241)
+template <typename R, typename DD>
+__device__ __forceinline__ void radiation_diagnostics(const DD& D, const Rad<R>& Rd) {
+            D.put(IBIS_DIAG_SOLU, Rd.solu); D.put(IBIS_DIAG_SOLS, Rd.sols); D.put(IBIS_DIAG_SOLL, Rd.soll);
+            D.put(IBIS_DIAG_SOLG, Rd.solg); D.put(IBIS_DIAG_SOLI, Rd.soli);
+            D.put(IBIS_DIAG_FIRU, Rd.firu); D.put(IBIS_DIAG_FIRS, Rd.firs); D.put(IBIS_DIAG_FIRL, Rd.firl);
+    #pragma unroll
+            for (int b = 0; b < 2; ++b) { D.put(IBIS_DIAG_ASURD, b, Rd.asurd[b]); D.put(IBIS_DIAG_ASURI, b, Rd.asuri[b]); }
+            D.put(IBIS_DIAG_TOPPARU, Rd.topparu); D.put(IBIS_DIAG_TOPPARL, Rd.topparl);
+    #pragma unroll
+            for (int j = 0; j < 4; ++j) { D.put(IBIS_DIAG_SCALCOEFU, j, Rd.scu[j]); D.put(IBIS_DIAG_SCALCOEFL, j, Rd.scl[j]); }
+}
+
 // ---- diagnostics of the surface phase (loops.py:1158-1241)
 template <typename R, typename DD>
 __device__ __forceinline__ void surface_diagnostics(const DD& D, const Stom<R>& st, R fwetu, R fwets, R fwetl, R rliqu,
-                                                    R rliqs, R rliql, const Rad<R>& Rd, R firg, R firi, R firb,
+                                                    R rliqs, R rliql, R firg, R firi, R firb,
                                                     R fsenu, R fsens, R fsenl, R fseng, R fseni, const Mid<R>& M,
                                                     R rhoa, R hvasug, R hvasui, R q1, R q2, R q3, R q4) {
     #pragma unroll
@@ -196,15 +209,7 @@ __device__ __forceinline__ void surface_diagnostics(const DD& D, const Stom<R>& 
             for (int j = 0; j < 3; ++j) { D.put(IBIS_DIAG_AN_LOWER, j, st.an_l[j]); D.put(IBIS_DIAG_AG_LOWER, j, st.ag_l[j]); }
             D.put(IBIS_DIAG_FWETU, fwetu); D.put(IBIS_DIAG_FWETS, fwets); D.put(IBIS_DIAG_FWETL, fwetl);
             D.put(IBIS_DIAG_RLIQU, rliqu); D.put(IBIS_DIAG_RLIQS, rliqs); D.put(IBIS_DIAG_RLIQL, rliql);
-            D.put(IBIS_DIAG_SOLU, Rd.solu); D.put(IBIS_DIAG_SOLS, Rd.sols); D.put(IBIS_DIAG_SOLL, Rd.soll);
-            D.put(IBIS_DIAG_SOLG, Rd.solg); D.put(IBIS_DIAG_SOLI, Rd.soli);
-            D.put(IBIS_DIAG_FIRU, Rd.firu); D.put(IBIS_DIAG_FIRS, Rd.firs); D.put(IBIS_DIAG_FIRL, Rd.firl);
             D.put(IBIS_DIAG_FIRG, firg); D.put(IBIS_DIAG_FIRI, firi); D.put(IBIS_DIAG_FIRB, firb);
-    #pragma unroll
-            for (int b = 0; b < 2; ++b) { D.put(IBIS_DIAG_ASURD, b, Rd.asurd[b]); D.put(IBIS_DIAG_ASURI, b, Rd.asuri[b]); }
-            D.put(IBIS_DIAG_TOPPARU, Rd.topparu); D.put(IBIS_DIAG_TOPPARL, Rd.topparl);
-    #pragma unroll
-            for (int j = 0; j < 4; ++j) { D.put(IBIS_DIAG_SCALCOEFU, j, Rd.scu[j]); D.put(IBIS_DIAG_SCALCOEFL, j, Rd.scl[j]); }
             D.put(IBIS_DIAG_FSENU, fsenu); D.put(IBIS_DIAG_FSENS, fsens); D.put(IBIS_DIAG_FSENL, fsenl);
             D.put(IBIS_DIAG_FSENG, fseng); D.put(IBIS_DIAG_FSENI, fseni);
             D.put(IBIS_DIAG_FVAPG, M.fvapg); D.put(IBIS_DIAG_FVAPI, M.fvapi);

@@ -197,10 +197,12 @@ __device__ __forceinline__ void surface_phase(Col<R>& c, const Forc<R>& F, const
     c.wliqu = wliqu; c.wliqs = wliqs; c.wliql = wliql;
     c.wsnou = wsnou; c.wsnos = wsnos; c.wsnol = wsnol;
 
-    if (D.on())
-        surface_diagnostics(D, st, fwetu, fwets, fwetl, rliqu, rliqs, rliql, Rd, (R)tv.firg, (R)tv.firi, (R)tv.firb,
+    if (D.on()) {
+        radiation_diagnostics(D, Rd);
+        surface_diagnostics(D, st, fwetu, fwets, fwetl, rliqu, rliqs, rliql, (R)tv.firg, (R)tv.firi, (R)tv.firb,
                             (R)tv.fsenu, (R)tv.fsens, (R)tv.fsenl, (R)tv.fseng, (R)tv.fseni, M, A.rhoa, hvasug, hvasui,
                             q1, q2, q3, q4);
+    }
 }
 
 // Steps 10-12 of timestep_body -- snow, soil water and heat (+ bedrock),
@@ -540,14 +542,15 @@ __device__ __forceinline__ void ground_phase(Col<R>& c, const Forc<R>& F, const 
     }
 }
 
-// One full hourly step of a column in one kernel.
-template <typename R, int NT, bool SUN_U, bool SUN_L, typename Q, typename DD, int SLD>
-__device__ __forceinline__ void column_step(Col<R>& c, const Forc<R>& F, const Stat<R>& S, const DD& D,
+// One full hourly step of a column in one kernel (y: the FP32 step's record of the hour
+// in shared memory, HourScratch; unused in float64).
+template <typename R, int NT, bool SUN_U, bool SUN_L, typename Y, typename Q, typename DD, int SLD>
+__device__ __forceinline__ void column_step(Col<R>& c, Y& y, const Forc<R>& F, const Stat<R>& S, const DD& D,
                                             const Acc<R, SLD>& Ac, const DevParams<R>& P, const Q& q) {
     Mid<R> M;
     if constexpr (sizeof(R) == 4) {
         SoilHour G;
-        surface_phase32<SUN_U, SUN_L>(c, F, S, D, P, q, M, G);
+        surface_phase32<SUN_U, SUN_L>(c, y, F, S, D, P, q, M, G);
         ground_phase32<NT>(c, F, S, D, Ac, P, q, M, G);
     } else {
         surface_phase<R, SUN_U, SUN_L>(c, F, S, D, P, q, M);

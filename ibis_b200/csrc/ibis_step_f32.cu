@@ -26,11 +26,20 @@ int diurnal(const float* daily, const float* lat, const float* sw_obs, const uns
             void* stream, const char* what, int cell0);
 }  // namespace ibis
 
+namespace {
+// The current device's SM count, which the driver keeps
+bool device_sms(int& sms) {
+    int dev = 0;
+    return cudaGetDevice(&dev) == cudaSuccess &&
+           cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess && sms > 0;
+}
+}  // namespace
+
 extern "C" int ibis_step_f32(float* prog, const float* stat, const float* forc, float* diag, float* acc, int ncell,
                              int ld, int nstep, const IbisParams* params, int* status, void* stream) {
-    // launches of several hours take the fastest fused configuration at full
-    // size (block 224, accumulators on chip); shorter ones the default
-    const int cfg = nstep >= ibis::kAccSmemMinSteps ? ibis::kLongFused : ibis::kDefaultFused;
+    // without a device, the step's own checks and its launch report what is wrong
+    int sms = 0;
+    const int cfg = ncell > 0 && device_sms(sms) ? ibis::auto_config(ncell, nstep, sms) : ibis::kDefaultFused;
     return ibis::hourly_step<float>(prog, stat, forc, diag, acc, ncell, ld, nstep, params, status, stream, nullptr,
                                     cfg);
 }
@@ -211,10 +220,10 @@ extern "C" int ibis_step_host_f32(float* prog, const float* stat, const float* h
     if (config < -1 || config >= ibis::kNumConfigs || (config >= 0 && ibis::kConfigs[config].form == 1))
         return -EINVAL;
     if (ncell == 0) return 0;
-    const int cfg = config >= 0 ? config : (nstep >= ibis::kAccSmemMinSteps ? ibis::kLongFused : ibis::kDefaultFused);
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return -ENODEV;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) return -ENODEV;
+    const int cfg = config >= 0 ? config : ibis::auto_config(ncell, nstep, sms);
     if (group == 0) {
         // whole blocks per group: a partial block in every group would add
         // blocks to the batch, and a batch of whole waves would spill into one more
@@ -332,10 +341,10 @@ extern "C" int ibis_day_host_f32(float* prog, const float* stat, const float* ho
     if (nh < 1 || nh > 254 || (double)nh * params->dtime != 86400.0) return -EINVAL;
     if (ncell == 0) return 0;
     const int nstep = nday * nh;
-    const int cfg = config >= 0 ? config : (nstep >= ibis::kAccSmemMinSteps ? ibis::kLongFused : ibis::kDefaultFused);
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return -ENODEV;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) return -ENODEV;
+    const int cfg = config >= 0 ? config : ibis::auto_config(ncell, nstep, sms);
     if (group == 0) {
         const int block = ibis::kConfigs[cfg].block;
         const double wave = (double)sms * block * ibis::kConfigs[cfg].minb;

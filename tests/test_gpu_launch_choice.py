@@ -1,0 +1,94 @@
+"""The library's choice of a launch configuration, and the shapes where the blocks of
+each can go wrong: batches of less than a warp, of partial warps and blocks, on both
+sides of the sizes where the choice changes.
+
+A column's step does not depend on its batch, so each batch is compared with one run
+of configuration 0 over the most columns: the same step code compiled for another
+block size, which may contract other multiply-adds; temperatures then differ by a few
+float32 ulps an hour (5e-5 K each), bounded here by 5 mK over at most five hours (the
+bound the FP32 step is held to against float64 for one hour), contents and sums by
+1e-4 and 1e-3 of their size.
+"""
+import numpy as np
+import pytest
+import torch
+
+from ibis_b200 import ensemble as E
+from ibis_b200 import synth
+from ibis_b200.columns import AUTO_FUSED, AUTO_SMALL, Columns
+from ibis_b200.params import FLAG_SUNSHADE_L, FLAG_SUNSHADE_U, FLAG_VMAX_MIX
+
+pytestmark = pytest.mark.gpu
+
+MOST = 33153
+HOURS = 5
+
+
+@pytest.fixture(scope="module")
+def reference(cuda_lib):
+    wl = synth.make_workload(MOST, HOURS, seed=77, edge_cases=True)
+    out = {}
+    for nstep in (1, HOURS):
+        cols = Columns.from_host(wl.prog, wl.stat, acc=True, mode=0)
+        cols.run(cols.forcing(wl.forc, 0, nstep), wl.params)
+        out[nstep] = (cols.prog_host(), cols.acc_host())
+    return wl, out
+
+
+def _head(wl, n):
+    cut = lambda d: {k: v[:n] for k, v in d.items()}
+    return cut(wl.prog), cut(wl.stat), {k: v[:, :n] for k, v in wl.forc.items()}
+
+
+@pytest.mark.parametrize("diag", [False, True])
+@pytest.mark.parametrize("nstep", [1, HOURS])
+@pytest.mark.parametrize("ncell", [1, 31, 33, 127, 225, 4735, 4737, 18945, MOST])
+def test_batches_of_every_shape_step_as_one(reference, ncell, nstep, diag):
+    wl, out = reference
+    prog, stat, forc = _head(wl, ncell)
+    cols = Columns.from_host(prog, stat, acc=True, diag=diag)
+    cols.prog[:, ncell:] = 7.0                       # the padding of each plane is nobody's
+    cols.acc[:, ncell:] = 7.0
+    cols.run(cols.forcing(forc, 0, nstep), wl.params)
+    torch.cuda.synchronize()
+    assert bool((cols.prog[:, ncell:] == 7.0).all()) and bool((cols.acc[:, ncell:] == 7.0).all())
+    assert not cols.nonfinite()[0]
+    p, a = cols.prog_host(), cols.acc_host()
+    p0, a0 = out[nstep]
+    for k in ("tsoi", "tg", "tu", "ts", "tl", "t12", "t34", "tsno", "ti"):
+        np.testing.assert_allclose(p[k], p0[k][:ncell], rtol=0, atol=5e-3, err_msg=k)
+    for k in ("wsoi", "wisoi", "fi"):
+        np.testing.assert_allclose(p[k], p0[k][:ncell], rtol=0, atol=1e-4, err_msg=k)
+    for k, w in a0.items():
+        if k.endswith("_mean"):
+            continue
+        scale = max(float(np.abs(w).max()), 1e-30)
+        assert float(np.abs(a[k] - w[:ncell]).max()) <= 1e-3 * scale, k
+
+
+def test_the_choice_follows_the_batch(cuda_lib):
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    cfg = lambda n, h: Columns(n, acc=False).launch_config(h)
+    assert cfg(1, 24) == cfg(32 * sms, 24) == cfg(32 * sms, 1) == AUTO_SMALL
+    assert cfg(32 * sms + 1, 1) == cfg(32 * sms + 1, 24) == cfg(128 * sms, 24) == 0
+    assert cfg(128 * sms + 1, 24) == cfg(224 * sms, 24) == AUTO_FUSED     # one wave of either
+    assert cfg(224 * sms + 1, 24) == cfg(256 * sms, 24) == 0              # one wave of 256 threads, two of 224
+
+
+@pytest.mark.parametrize("daily", [False, True])
+def test_every_ensemble_block_runs_with_every_switch(cuda_lib, daily):
+    """The largest block accepted needs more shared memory than an SM has with the
+    sunlit/shaded canopies, the IBIS 3.0 switches and daily weather together: it
+    runs in the largest that fits.  The same kernel in blocks of 32 gives the same bits."""
+    spec = E.make_ensemble(5, 13, site_hours=np.full(5, 24), seed=3, daily=daily)
+    spec.params.flags |= FLAG_SUNSHADE_U | FLAG_SUNSHADE_L | FLAG_VMAX_MIX
+    ens = E.Ensemble(spec)
+    out = []
+    for block in (32, 256):
+        assert ens.occupancy(block) > 0
+        ens.reset()
+        ens.run(block=block)
+        torch.cuda.synchronize()
+        assert not any(ens.nonfinite()[:2])
+        out.append((ens.prog.clone(), ens.acc.clone()))
+    assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
