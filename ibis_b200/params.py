@@ -152,6 +152,14 @@ def _ctypes_struct():
 
 IbisParamsC = _ctypes_struct()
 
+# Where the fields lie in the record, in doubles: the scalars' offsets by name, and the
+# arrays' names with the places of all their values one after another
+_SPEC = {n: c for n, c, _ in PARAM_FIELDS}
+_SCALAR_AT = {n: getattr(IbisParamsC, n).offset // 8 for n, c in _SPEC.items() if c == 1}
+_ARRAYS = tuple(n for n, c in _SPEC.items() if c > 1)
+_ARRAYS_AT = np.concatenate([getattr(IbisParamsC, n).offset // 8 + np.arange(_SPEC[n]) for n in _ARRAYS])
+_RECORD_DOUBLES = -(-ctypes.sizeof(IbisParamsC) // 8)
+
 
 class StepParams:
     """Mutable parameter record with the reference defaults.
@@ -162,16 +170,17 @@ class StepParams:
     """
 
     def __init__(self, **overrides):
+        # the scalars' values as they lie in the C record, kept beside the attributes
+        object.__setattr__(self, "_record", np.zeros(_RECORD_DOUBLES))
         for name, n, default in PARAM_FIELDS:
-            val = np.array(default, dtype=np.float64) if n > 1 else float(default)
-            object.__setattr__(self, name, val)
+            setattr(self, name, default)
         self.froot = DEFAULT_FROOT.reshape(-1).copy()
         self.flags = FLAG_BEDROCK | FLAG_ACC | FLAG_CH4 | FLAG_KAHAN
         for k, v in overrides.items():
             setattr(self, k, v)
 
     def __setattr__(self, key, value):
-        spec = {n: c for n, c, _ in PARAM_FIELDS}
+        spec = _SPEC
         if key == "flags":
             value = int(value)
             if value & ~KNOWN_FLAGS:
@@ -184,9 +193,17 @@ class StepParams:
                 value = arr
             else:
                 value = float(value)
+                self._record[_SCALAR_AT[key]] = value
         else:
             raise AttributeError(f"no parameter named {key!r}")
         object.__setattr__(self, key, value)
+
+    def __setstate__(self, state):
+        """Unpickled or shallow-copied: the scalars' record is the object's own."""
+        self.__dict__.update(state)
+        object.__setattr__(self, "_record", np.zeros(_RECORD_DOUBLES))
+        for name, at in _SCALAR_AT.items():
+            self._record[at] = self.__dict__[name]
 
     # convenience views
     @property
@@ -202,17 +219,18 @@ class StepParams:
         for name, n, _ in PARAM_FIELDS:
             v = getattr(self, name)
             object.__setattr__(out, name, v.copy() if n > 1 else v)
+        out._record[:] = self._record
         out.flags = self.flags
         return out
 
     def to_c(self):
-        s = IbisParamsC()
-        for name, n, _ in PARAM_FIELDS:
-            v = getattr(self, name)
-            if n > 1:
-                getattr(s, name)[:] = [float(x) for x in v]
-            else:
-                setattr(s, name, float(v))
+        """The C record.  Every launch asks for one (a launch-bound hourly call spent 55 of
+        its 60 us filling it field by field), so the scalars are kept as they lie in it
+        and the arrays, which a caller may write in place, are gathered in one go."""
+        rec = self._record.copy()
+        d = self.__dict__
+        rec[_ARRAYS_AT] = np.concatenate([d[n] for n in _ARRAYS])
+        s = IbisParamsC.from_buffer(rec)
         s.flags = self.flags
         return s
 
