@@ -17,23 +17,45 @@
 
 namespace ibis {
 
-template <typename R>
+// N planes of one cell, read before anything is written: every plane a kernel uses is
+// loaded at once (the planes it does not use are not loaded), so a thread waits out
+// one memory latency instead of one between every two stores -- the compiler cannot
+// move a load above a store to the same buffer.  A plane read after it was written
+// gives the value as stored.  At 95,333 cells in float32: day_begin 88 -> 15 us,
+// day_end 36 -> 24 us (the rest is double arithmetic).
+template <typename R, int N>
 struct Planes {
     R* __restrict__ base;
     int ld;
-    __device__ __forceinline__ double get(int p) const { return (double)base[(size_t)p * ld]; }
-    __device__ __forceinline__ void set(int p, double v) const { base[(size_t)p * ld] = (R)v; }
+    R v[N];
+    __device__ __forceinline__ Planes(R* b, int l) : base(b), ld(l) {
+#pragma unroll
+        for (int p = 0; p < N; ++p) v[p] = base[(size_t)p * ld];
+    }
+    __device__ __forceinline__ double get(int p) const { return (double)v[p]; }
+    __device__ __forceinline__ void set(int p, double x) {
+        v[p] = (R)x;
+        base[(size_t)p * ld] = v[p];
+    }
 };
+template <typename R>
+using StatPlanes = Planes<R, IBIS_STAT_COUNT>;
+template <typename R>
+using DayPlanes = Planes<R, IBIS_DAYST_COUNT>;
+template <typename R>
+using AccPlanes = Planes<R, 2 * IBIS_ACC_COUNT>;
+template <typename R>
+using ProgPlanes = Planes<R, IBIS_PROG_COUNT>;
 
 // An accumulator: its plane minus its Kahan compensation plane (zero when the
 // step sums without compensation).
 template <typename R>
-__device__ __forceinline__ double acc_value(const Planes<R>& A, int p) {
+__device__ __forceinline__ double acc_value(const AccPlanes<R>& A, int p) {
     return A.get(p) - A.get(p + IBIS_ACC_COUNT);
 }
 
 template <typename R>
-__device__ __forceinline__ void acc_zero(const Planes<R>& A, int p) {
+__device__ __forceinline__ void acc_zero(AccPlanes<R>& A, int p) {
     A.set(p, 0.0);
     A.set(p + IBIS_ACC_COUNT, 0.0);
 }
@@ -53,7 +75,7 @@ __device__ __forceinline__ double daylength_hours(double lat, double doy) {
 // Tb while the day length is decreasing and below Pstart, reset otherwise.
 // Returns through sen_u / sen_l whether photoperiod-gated senescence starts.
 template <typename R>
-__device__ __forceinline__ void seasonal_states(const Planes<R>& D, double td, const IbisDayParams& dp, bool& sen_u,
+__device__ __forceinline__ void seasonal_states(DayPlanes<R>& D, double td, const IbisDayParams& dp, bool& sen_u,
                                                 bool& sen_l) {
     const double tc = td - 273.16, lat = D.get(IBIS_DAYST_LATITUDE);
     const double dl = daylength_hours(lat, dp.jday);
@@ -71,7 +93,7 @@ __device__ __forceinline__ void seasonal_states(const Planes<R>& D, double td, c
 // pheno (phenology.py:89-287); sen_u / sen_l: photoperiod-gated senescence
 // (phenology.py:148-150, 170-172)
 template <typename R>
-__device__ __forceinline__ void phenology(const Planes<R>& S, const Planes<R>& D, double td, double stresstu,
+__device__ __forceinline__ void phenology(StatPlanes<R>& S, DayPlanes<R>& D, double td, double stresstu,
                                           double stresstl, const IbisDayParams& dp, double epsilon, bool sen_u,
                                           bool sen_l) {
     const double tmelt = 273.16, ddfac = 1.0 / dp.ddays;
@@ -149,7 +171,7 @@ __device__ __forceinline__ double clip_d(double x, double lo, double hi) { retur
 
 // soilbgc (biogeochem.py:23-243), one call per day; returns tco2mic.
 template <typename R>
-__device__ __forceinline__ double soil_bgc(const Planes<R>& D, const Planes<R>& S, const double* hsoi,
+__device__ __forceinline__ double soil_bgc(DayPlanes<R>& D, const StatPlanes<R>& S, const double* hsoi,
                                            const IbisDayParams& b, double ndaypy) {
     const double* cnr = b.cnr;
     const double totts = 1.0 / ndaypy;
@@ -272,7 +294,9 @@ __global__ void __launch_bounds__(128) day_begin_kernel(R* stat, R* dayst, R* ac
                                                         const IbisDayParams dp, const DayConst c) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= ncell) return;
-    const Planes<R> S{stat + i, ld}, D{dayst + i, ld}, A{acc + i, ld};
+    StatPlanes<R> S(stat + i, ld);
+    DayPlanes<R> D(dayst + i, ld);
+    AccPlanes<R> A(acc + i, ld);
     bool sen_u = false, sen_l = false;
     if (dp.seasonal_on != 0.0) {
         seasonal_states(D, (double)td[i], dp, sen_u, sen_l);
@@ -293,8 +317,10 @@ __global__ void __launch_bounds__(128) day_end_kernel(const R* prog, R* stat, R*
                                                       int ncell, int ld, const IbisDayParams dp, const DayConst c) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= ncell) return;
-    const Planes<R> S{stat + i, ld}, D{dayst + i, ld};
-    const Planes<R> A{const_cast<R*>(acc) + i, ld}, G{const_cast<R*>(prog) + i, ld};
+    StatPlanes<R> S(stat + i, ld);
+    DayPlanes<R> D(dayst + i, ld);
+    const AccPlanes<R> A(const_cast<R*>(acc) + i, ld);
+    const ProgPlanes<R> G(const_cast<R*>(prog) + i, ld);
     const double zweight = exp(-1.0 / 10.0), alpha10 = 1.0 - zweight, day_sec = 86400.0;
     D.set(IBIS_DAYST_A10TD, zweight * D.get(IBIS_DAYST_A10TD) + alpha10 * (double)td[i]);
     const int means[4] = {IBIS_DAYST_A10ANCUB, IBIS_DAYST_A10ANCLS, IBIS_DAYST_A10ANCL3, IBIS_DAYST_A10ANCL4};
