@@ -40,7 +40,6 @@ UNITS = {
     "ibis_x3_inst_d.cu": F32_FLAGS,
     "ibis_x3_inst_e.cu": F32_FLAGS,
     "ibis_x3_inst_f.cu": F32_FLAGS,
-    "ibis_x3_inst_g.cu": F32_FLAGS,
     "ibis_ensemble_f32.cu": F32_FLAGS,
     "ibis_ens_inst_a.cu": F32_FLAGS,
     "ibis_ens_inst_b.cu": F32_FLAGS,

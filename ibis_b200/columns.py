@@ -16,13 +16,13 @@ import torch
 from . import layout as L
 from . import lib as _lib
 from . import synth
-from .params import StepParams, FLAG_DIAG, FLAG_ACC, FLAG_CH4, FLAG_SOIL_MEANS
+from .params import (StepParams, FLAG_DIAG, FLAG_ACC, FLAG_CH4, FLAG_SOIL_MEANS, FLAG_SUNSHADE_L, FLAG_SUNSHADE_U,
+                     X3_FLAGS)
 
 INT_MAX = 2 ** 31 - 1
 # the fused configurations ibis_step_f32 chooses from (auto_config, csrc/ibis_kernels.cuh)
-AUTO_SMALL = 4          # single-warp blocks: batches of up to a warp per SM
-AUTO_FUSED = 6          # one block of 224 per SM, accumulators on chip
-AUTO_MIN_HOURS = 4      # shorter launches keep the accumulators in global memory (configuration 0)
+AUTO_FUSED = 0          # two blocks of 128 per SM
+AUTO_LARGE = 6          # one block of 224: the canopy variants with a larger record of the hour
 _ACC_FLAGS = FLAG_ACC | FLAG_CH4 | FLAG_SOIL_MEANS
 
 
@@ -64,9 +64,9 @@ class Columns:
         """``fused`` (one kernel per launch), ``split`` (surface + ground kernels per hour),
         or an integer launch configuration (see ``lib.configs()``).
 
-        ``fused`` leaves the configuration to the library in FP32, by the batch's
-        size and the hours of the call (:meth:`launch_config`); ``tune.tune``
-        times every configuration on the caller's own batch instead."""
+        ``fused`` leaves the configuration to the library in FP32
+        (:meth:`launch_config`); ``tune.tune`` times every configuration on the
+        caller's own batch instead."""
         if mode is None:
             mode = "fused"
         if isinstance(mode, (int, np.integer)) and not isinstance(mode, bool):
@@ -155,18 +155,14 @@ class Columns:
         return bool(s[0] & 1), int(s[1])
 
     # -------------------------------------------------------------- compute
-    def launch_config(self, nstep: int) -> int:
-        """The launch configuration a call of ``nstep`` hours uses: the columns' own, or
-        the library's choice for the batch (``auto_config``, csrc/ibis_kernels.cuh)."""
+    def launch_config(self, nstep: int, flags: int = 0) -> int:
+        """The launch configuration a call of ``nstep`` hours with the parameter record's
+        ``flags`` uses: the columns' own, or the library's choice for the batch."""
         if self.config is not None:
             return self.config
         sms = torch.cuda.get_device_properties(self.device).multi_processor_count
-        if self.ncell <= 32 * sms:
-            return AUTO_SMALL
-        if nstep < AUTO_MIN_HOURS or self.ncell <= 128 * sms:
-            return 0
-        waves = lambda threads: -(-self.ncell // (threads * sms))
-        return AUTO_FUSED if waves(224) <= waves(256) else 0
+        large = flags & (X3_FLAGS | FLAG_SUNSHADE_U | FLAG_SUNSHADE_L)
+        return AUTO_LARGE if large and self.ncell > 128 * sms else AUTO_FUSED
 
     def run(self, forc: torch.Tensor, params: StepParams, nstep: int | None = None, stream=None):
         """Advance the columns ``nstep`` hours with forcing ``forc`` (asynchronous)."""

@@ -51,9 +51,9 @@ __device__ __forceinline__ TwoStr2 two_stream2(float cosz, float k, float xai, c
                                                float o, float eps, const Par32& P) {
     const float ov = P.oriev[st], oh = P.orieh[st], orand = 1.0f - ov - oh;
     const float ztab = 0.5f - cosz * (1.0f / 3.0f);
-    const F2 rho(P.rhoveg[st], P.rhoveg[2 + st]), tau(P.tauveg[st], P.tauveg[2 + st]);
+    const F2 rho(P.rho2[st]), tau(P.tau2[st]);
     const float dry = 1.0f - y, ah = 0.5f * ov + oh;
-    const F2 ys = F2(P.omegasno[0], P.omegasno[1]) * (y * o);
+    const F2 ys = F2(P.osno2) * (y * o);
     const F2 om = mx2((rho + tau) * dry + ys, 1e-12f);
     const F2 rdry = dry * rcp2(om), ysh = ys * 0.5f * rcp2(om);
     const F2 betad = (rho * (ah + orand * (1.0f - ztab)) + tau * (0.5f * ov + orand * ztab)) * rdry + ysh;
@@ -247,11 +247,11 @@ __device__ __forceinline__ Surf2 intercept2(float tveg, F2 w, float xai, const F
     const float dt = P.dtime, eps = P.epsilon;
     const float fint = xai >= eps ? (1.0f - ex(-0.5f * xai)) / xai : 0.5f;
     const float xr = xai * P.rdt;
-    F2 drip = w * F2(P.rtdrip[st], P.rtblow[st]) * xai;
+    F2 drip = w * F2(P.drip2[st]) * xai;
     const F2 pf = pr0 * fint;
-    w = w * F2(P.kdrip[st], P.kblow[st]) + pf * dt;
+    w = w * F2(P.kdrip2[st]) + pf * dt;
     Surf2 s;
-    s.pflux = (pf * (tveg - tp) * F2(P.ch2o, P.cice)).sum();
+    s.pflux = (pf * (tveg - tp) * F2(P.water2)).sum();
     const F2 pr = pr0 * (1.0f - xai * fint);
     const F2 m = mn2(w, F2(wliqmax, wsnomax));
     const F2 kept = sel2(m.lo() < wliqmin, m.hi() < P.wsnomin, F2(0.0f), m);
@@ -360,7 +360,7 @@ __device__ __forceinline__ void aero_geometry32(Aero32& A, Turc& tc, float& cp, 
     cp = P.cair * (1.0f + float((double)P.cvap / (double)P.cair - 1.0) * F.qa);
     const float za = mx((F.ps - pa) / (rhoa * P.grav), ztop.hi() + 1.0f);
     const F2 leaf = (stat2(S, IBIS_STAT_LAI, 0) + stat2(S, IBIS_STAT_SAI, 0)) * 2.0f * F2(fl * (1.0f - fi), fu);
-    const F2 x = mn2(leaf * F2(1.0f / P.alaiml, 1.0f / P.alaimu), 3.0f);
+    const F2 x = mn2(leaf * F2(P.ralai2), 3.0f);
     const F2 x1 = mn2(x, 1.0f);
     const F2 rw = mx2(ztop - zbot, 0.01f), rrw = rcp2(rw);
     const F2 cveg = mx2(x, 1e-5f) * 0.4f * rrw;
@@ -634,12 +634,14 @@ struct alignas(8) HourExtra<true, true> { Sun4 su, sl; F2 vnl, cmu, cml, jfu, jf
 // Pairs: (upper leaves, upper stems) `_us`, (lower canopy, ground) `_lg`, (ground, snow) `_gi`
 struct alignas(8) TvHour {
     F2 x_us, ch_us, ch_lg, wl_us, ws_us, wl_lg, ws_lg, rl_us, fw_us, frad_us, pf_us;
-    F2 hv_gi, sol_gi, fir_gi, zir_gi, co_gi;
+    F2 hv_gi, sol_gi, fir_gi, zir_gi;
     F2 stress, toppar, scale;       // (upper, lower)
     F2 vnu;                         // nominal vmax of the upper big leaves
-    float xl, rliql, fwetl, fradl, pfluxl, psig, cp, firb, ta, qa, ps, fi;
+    float xl, rliql, fwetl, fradl, pfluxl, psig, cp, firb, qa, ps, fi, fr3, fr4, unused;
     double betaw;                   // soil-surface wetness factor
     double fb, fc, fs, rlai;        // leaf-area shares of the big leaves; lai0 / (lai0 + sai0)
+    double pg0, bg0, pi0, bi0;      // what the ground's and snow's rows have besides the air: pivot, right-hand side
+    double hv0, hs0, tap;           // latent heats at 0 K extrapolated; ta tfac
 };
 
 template <bool SUN, bool X3>
@@ -680,12 +682,11 @@ __device__ __forceinline__ void stomata32(Stom<float>& o, Col32& c, float tu, fl
             fcap = y.cap.lo();
             capu = !SUN_U && (P.flags & IBIS_FLAG_CAP_SCALE_U) != 0;
         } else {
-            cm = F2(q.coefm(0), q.coefm(1));
+            cm = F2(q.coefm2(0));
         }
         if constexpr (SUN_U) ss = y.su;
         const F2 tc = c3_pair<SUN_U, X3>(cs, gs, ci, ag, an, t, K.gst.lo(), K.kco.lo(), K.vm3.lo(), X.vnu, cm,
-                                         F2(P.gamma[0], P.gamma[1]), F2(P.coefb[0], P.coefb[1]),
-                                         F2(P.gsmin[0], P.gsmin[1]), ss, jf, capu, fcap, P);
+                                         F2(P.gam2[0]), F2(P.b02[0]), F2(P.gmin2[0]), ss, jf, capu, fcap, P);
         c.cs_u[0] = cs.lo(); c.cs_u[1] = cs.hi(); c.gs_u[0] = gs.lo(); c.gs_u[1] = gs.hi();
         c.ci_u[0] = ci.lo(); c.ci_u[1] = ci.hi();
         o.ag_u[0] = ag.lo(); o.ag_u[1] = ag.hi(); o.an_u[0] = an.lo(); o.an_u[1] = an.hi();
@@ -703,13 +704,12 @@ __device__ __forceinline__ void stomata32(Stom<float>& o, Col32& c, float tu, fl
             vn4 = y.vn4; cm4 = y.cm4; jf4 = y.jf4;
             fcap = y.cap.hi();
         } else {
-            vn = F2(q.vmax(8), q.vmax(11)); cm = F2(q.coefm(2), q.coefm(4));
+            vn = F2(q.vmaxl2()); cm = F2(q.coefm2(1));
             vn4 = q.vmax(10); cm4 = q.coefm(3);
         }
         if constexpr (SUN_L) ss = y.sl;
         const F2 tc = c3_pair<SUN_L, X3>(cs, gs, ci, ag, an, t, K.gst.hi(), K.kco.hi(), K.vm3.hi(), vn, cm,
-                                         F2(P.gamma[2], P.gamma[4]), F2(P.coefb[2], P.coefb[4]),
-                                         F2(P.gsmin[2], P.gsmin[4]), ss, jf, cap, fcap, P);
+                                         F2(P.gam2[1]), F2(P.b02[1]), F2(P.gmin2[1]), ss, jf, cap, fcap, P);
         c.cs_l[0] = cs.lo(); c.cs_l[1] = cs.hi(); c.gs_l[0] = gs.lo(); c.gs_l[1] = gs.hi();
         c.ci_l[0] = ci.lo(); c.ci_l[1] = ci.hi();
         o.ag_l[0] = ag.lo(); o.ag_l[1] = ag.hi(); o.an_l[0] = an.lo(); o.an_l[1] = an.hi();
@@ -769,7 +769,7 @@ struct TvResult {
 // elimination it replaces filled 45 entries and divided by nine pivots.
 __device__ __forceinline__ void turvap32(double (&W)[9], TvResult& o, const Col32& c, const Trans<float>& T,
                                          const F2& wus, const F2& wlg, float wif, const TvHour& X,
-                                         const Stom<float>& st, const Stat32& S, float e34, float q34s, bool last,
+                                         const Stom<float>& st, const Stat32& S, float r34, float q34s, bool last,
                                          const Par32& P) {
     const double eps = (double)P.epsilon, dt = (double)P.dtime;
     const double wu = wus.lo(), ws = wus.hi(), wl = wlg.lo(), wg = wlg.hi(), wi = wif;
@@ -785,22 +785,22 @@ __device__ __forceinline__ void turvap32(double (&W)[9], TvResult& o, const Col3
         const float ps = X.ps;
         const F2 ta((float)tu, (float)ts), tb((float)tl, (float)tg), tc((float)ti, (float)t34);
         const F2 ea = esat2(ta), eb = esat2(tb);
-        const F2 ec(esat(tc.lo()), e34);
-        const F2 qa_ = qsat2(ea, ps), qb = qsat2(eb, ps);
-        const F2 qc(qsat(ec.lo(), ps), q34s);
-        const F2 da = mn2(dqsat2(ta, qa_, ea), qa_ * 0.1f), db = mn2(dqsat2(tb, qb, eb), qb * 0.1f);
-        const F2 dc = dqsat2(tc, qc, ec);
+        const float ei = esat(tc.lo()), ri = 0.622f / mx(ps - ei * float(1.0 - 0.622), ei * 0.622f);
+        const F2 ra = sat_quotient2(ea, ps), rb = sat_quotient2(eb, ps), rc(ri, r34);
+        const F2 qa_ = ea * ra, qb = eb * rb, qc(ei * ri, q34s);
+        const F2 da = mn2(sat_derivative2(ta, qa_, ra), qa_ * 0.1f), db = mn2(sat_derivative2(tb, qb, rb), qb * 0.1f);
+        const F2 dc = sat_derivative2(tc, qc, rc);
         qu = qa_.lo(); qs = qa_.hi(); ql = qb.lo(); qg = qb.hi(); qi = qc.lo();
         dqu = da.lo(); dqs = da.hi(); dql = db.lo(); dqg = db.hi(); dqi = mn(dc.lo(), qc.lo() * 0.1f);
         dqs1 = dc.hi();
     }
     const double su = T.su, ss = T.ss, sl = T.sl, sg = T.sg, si = T.si, cu = T.cu, cl = T.cl, cp = X.cp;
-    const double qeps = 1.0e-10, hvap = (double)P.hvap, tmelt = (double)P.tmelt;
+    const double qeps = 1.0e-10, hvap = (double)P.hvap;
     // soil-surface humidity factor (canopy_exchange.py:532-572)
     const double hfac = (double)ex(X.psig / (P.rvap * (float)tg));
     const double xd = fma(cp, sg, (double)P.zir * cube(t34));
     const double betas = X.betaw * xd * rcp_nr(fma(hvap * dqs1 * sg, 1.0 - X.betaw, xd));
-    const double hfac2 = q34 * rcp_nr(fmax(qg, eps));
+    const double hfac2 = q34 * rcp_nr(dmax(qg, eps));
     double qgfac = betas > 0.0 ? fma(betas, hfac - hfac2, hfac2) : hfac2;
     if (q34 > qg + qeps) qgfac = 1.0;
     // vapour conductances (canopy_exchange.py:587-618)
@@ -808,15 +808,14 @@ __device__ __forceinline__ void turvap32(double (&W)[9], TvResult& o, const Col3
     const double fwux = (q12 > qu + qeps) ? 1.0 : X.fw_us.lo();
     const double fwsx = (q12 > qs + qeps) ? 1.0 : X.fw_us.hi();
     const double fwlx = (q34 > ql + qeps) ? 1.0 : X.fwetl;
-    const double suw = fmin(fwux * su, 0.8 * wet_us.lo() * rcp_nr(fmax(dt * (qu - q12), eps)));
-    const double ssw = fmin(fwsx * ss, 0.8 * wet_us.hi() * rcp_nr(fmax(dt * (qs - q12), eps)));
-    const double slw = fmin(fwlx * sl, 0.8 * (X.wl_lg.lo() + X.ws_lg.lo()) * rcp_nr(fmax(dt * (ql - q34), eps)));
-    const double sut = fmax(0.0, (0.5 - 0.5 * fwux) * (st.tcub * X.fb + st.tcuc * X.fc));
-    const double slt0 = fmax(0.0, (0.5 - 0.5 * fwlx) * (st.tcls * X.fs + (double)st.tcl4 * S(IBIS_STAT_FRAC, 10) +
-                                                       (double)st.tcl3 * S(IBIS_STAT_FRAC, 11)));
+    const double suw = dmin(fwux * su, 0.8 * wet_us.lo() * rcp_nr(dmax(dt * (qu - q12), eps)));
+    const double ssw = dmin(fwsx * ss, 0.8 * wet_us.hi() * rcp_nr(dmax(dt * (qs - q12), eps)));
+    const double slw = dmin(fwlx * sl, 0.8 * (X.wl_lg.lo() + X.ws_lg.lo()) * rcp_nr(dmax(dt * (ql - q34), eps)));
+    const double sut = dmax((0.5 - 0.5 * fwux) * (st.tcub * X.fb + st.tcuc * X.fc), 0.0);
+    const double slt0 = dmax((0.5 - 0.5 * fwlx) * (st.tcls * X.fs + (double)st.tcl4 * X.fr4 +
+                                                    (double)st.tcl3 * X.fr3), 0.0);
     const double slt = slt0 * X.rlai;
-    const double cvt = (double)P.cvap * ((double)X.ta - tmelt);
-    const double hv0 = fma((double)P.ch2o, tmelt, hvap + cvt), hs0 = fma((double)P.cice, tmelt, (double)P.hsub + cvt);
+    const double hv0 = X.hv0, hs0 = X.hs0;
     const double hvu = fma(-(double)P.ch2o, tu, hv0), hvl = fma(-(double)P.ch2o, tl, hv0), hvs = fma(-(double)P.ch2o, ts, hv0);
     const double hsu = fma(-(double)P.cice, tu, hs0), hsl = fma(-(double)P.cice, tl, hs0), hss = fma(-(double)P.cice, ts, hs0);
     const double suh = fma(suw, fma((double)X.rl_us.lo(), hvu - hsu, hsu), sut * hvu);
@@ -840,9 +839,8 @@ __device__ __forceinline__ void turvap32(double (&W)[9], TvResult& o, const Col3
     const bool bare = (X.x_us.lo() + X.x_us.hi() + X.xl) < P.epsilon;
     {
         const double r1 = sg * cp, r2 = sg * X.hv_gi.lo(), g = r2 * qgfac;
-        const double inv = rcp_nr(r1 + fma(g, dqg, (double)X.co_gi.lo()) + X.zir_gi.lo());
-        double b = fma((double)X.zir_gi.lo(), old[3], fma((double)X.co_gi.lo(), (double)c.tsoi[0], (double)X.sol_gi.lo() + (double)X.fir_gi.lo())) -
-                   g * fma(-dqg, tg, qg);
+        const double inv = rcp_nr(r1 + fma(g, dqg, X.pg0));
+        double b = fma(-g, fma(-dqg, tg, qg), X.bg0);
         // a bare cell's canopy heat goes to the ground (canopy_exchange.py:684-732)
         if (bare)
             b = b + (((double)X.frad_us.lo() - X.pf_us.lo()) * X.x_us.lo() + ((double)X.frad_us.hi() - X.pf_us.hi()) * X.x_us.hi() +
@@ -851,13 +849,12 @@ __device__ __forceinline__ void turvap32(double (&W)[9], TvResult& o, const Col3
     }
     {
         const double r1 = si * cp, r2 = si * X.hv_gi.hi();
-        const double inv = rcp_nr(r1 + fma(r2, dqi, (double)X.co_gi.hi()) + X.zir_gi.hi());
-        bi = (fma((double)X.zir_gi.hi(), old[4], fma((double)X.co_gi.hi(), (double)c.tsno[0], (double)X.sol_gi.hi() + (double)X.fir_gi.hi())) -
-              r2 * fma(-dqi, ti, qi)) * inv;
+        const double inv = rcp_nr(r1 + fma(r2, dqi, X.pi0));
+        bi = fma(-r2, fma(-dqi, ti, qi), X.bi0) * inv;
         ri = r1 * inv; ai = r2 * inv;
     }
     // the 4x4 system of (t12, q12 | t34, q34)
-    const double tap = (double)X.ta * (double)P.tfac, qa64 = X.qa;
+    const double tap = X.tap, qa64 = X.qa;
     double n12, nq12, n34, nq34;
     {
         const double cc = cu + cl;
@@ -910,9 +907,9 @@ __device__ __forceinline__ void turvap32(double (&W)[9], TvResult& o, const Col3
         o.fseng = (float)(cp * sg * (vg - n34));
         o.fseni = (float)(cp * si * (vi - n34));
         const double eu = fma(wu * dqu, nu - tu, qu) - nq12, el = fma(wl * dql, nl - tl, ql) - nq34;
-        const double fvapuw = suw * eu, fvaput = fmax(0.0, sut * eu);
+        const double fvapuw = suw * eu, fvaput = dmax(sut * eu, 0.0);
         const double fvaps = ssw * (fma(ws * dqs, ns - ts, qs) - nq12);
-        const double fvaplw = slw * el, fvaplt = fmax(0.0, slt0 * el);
+        const double fvaplw = slw * el, fvaplt = dmax(slt0 * el, 0.0);
         const double fvapg = sg * (qgfac * fma(wg * dqg, ng - tg, qg) - nq34);
         const double fvapi = si * (fma(wi * dqi, ni - ti, qi) - nq34);
         const double dg = wg * X.zir_gi.lo() * (ng - old[3]), di = wi * X.zir_gi.hi() * (ni - old[4]);
@@ -962,8 +959,8 @@ __device__ __forceinline__ void soil_stress32(SoilHour& G, const Col32& c, const
         const F2 z = clip2((1.0f - exp2_2(awc * sf)) * rz, 0.0f, 1.0f);
         G.zw[k] = z.lo();
         G.zw[k + 1] = z.hi();
-        tot = tot + F2(P.froot[2 * k], P.froot[2 * k + 1]) * z.lo();
-        tot = tot + F2(P.froot[2 * k + 2], P.froot[2 * k + 3]) * z.hi();
+        tot = tot + F2(P.fr2[k]) * z.lo();
+        tot = tot + F2(P.fr2[k + 1]) * z.hi();
     }
     G.stresstl = tot.lo();
     G.stresstu = tot.hi();
@@ -1051,12 +1048,25 @@ __device__ __forceinline__ void surface_phase32(Col32& c, Y& y, const Forc32& F,
         const float cs = S(IBIS_STAT_CSOI, 0), rs = S(IBIS_STAT_RHOSOI, 0);
         const float csoi0 = cs > 0.0f ? cs : P.csoi_mineral_val, rhosoi0 = rs > 0.0f ? rs : P.rhosoi_val;
         X.cp = cp;
-        X.ta = F.ta; X.qa = F.qa; X.ps = F.ps; X.fi = fi;
+        X.qa = F.qa; X.ps = F.ps; X.fi = fi;
         X.x_us = F2(lai1, sai1) * (2.0f * fu);
         X.xl = 2.0f * (lai0 + sai0) * fl * (1.0f - fi);
-        X.co_gi = F2(G.consoi0 / mx(0.5f * P.hsoi[0], eps), P.consno / mx(0.5f * mx(c.hsno[0], P.hsnotop), eps));
         const F2 tgi(c.tg, c.ti);
-        X.zir_gi = tgi * (tgi * tgi) * P.zir;
+        const F2 zir = tgi * (tgi * tgi) * P.zir;
+        X.zir_gi = zir;
+        {
+            const float cog = G.consoi0 / mx(0.5f * P.hsoi[0], eps);
+            const float coi = P.consno / mx(0.5f * mx(c.hsno[0], P.hsnotop), eps);
+            const double zg = zir.lo(), zi = zir.hi();
+            X.pg0 = cog + zg;
+            X.pi0 = coi + zi;
+            X.bg0 = fma(zg, (double)c.tg, fma((double)cog, (double)c.tsoi[0], (double)X.sol_gi.lo() + (double)X.fir_gi.lo()));
+            X.bi0 = fma(zi, (double)c.ti, fma((double)coi, (double)c.tsno[0], (double)X.sol_gi.hi() + (double)X.fir_gi.hi()));
+            const double tmelt = P.tmelt, cvt = (double)P.cvap * ((double)F.ta - tmelt);
+            X.hv0 = fma((double)P.ch2o, tmelt, (double)P.hvap + cvt);
+            X.hs0 = fma((double)P.cice, tmelt, (double)P.hsub + cvt);
+            X.tap = (double)F.ta * (double)P.tfac;
+        }
         const float p0 = S(IBIS_STAT_POROS, 0), w0 = c.wsoi[0], i0 = c.wisoi[0];
         const float rwp = p0 * P.rhow, liq = rwp * (1.0f - i0) * w0, ice = rwp * i0;
         const float chg = P.ch2o * c.wpud + P.cice * c.wipud +
@@ -1065,7 +1075,7 @@ __device__ __forceinline__ void surface_phase32(Col32& c, Y& y, const Forc32& F,
         X.ws_us = F2(C.wsnou, C.wsnos);
         X.wl_lg = F2(C.wliql, c.wpud + liq * P.hsoi[0]);
         X.ws_lg = F2(C.wsnol, c.wipud + ice * P.hsoi[0]);
-        X.ch_us = F2(P.chu, P.chs) + X.wl_us * P.ch2o + X.ws_us * P.cice;
+        X.ch_us = F2(P.chus2) + X.wl_us * P.ch2o + X.ws_us * P.cice;
         X.ch_lg = F2(P.chl + P.ch2o * C.wliql + P.cice * C.wsnol, chg);
         const float zwp = clip(0.5f * (c.wpud + c.wipud) / mx(P.wpudmax, eps), 0.0f, 0.5f);
         const float zws = (1.0f - i0) * w0 + i0;
@@ -1079,6 +1089,8 @@ __device__ __forceinline__ void surface_phase32(Col32& c, Y& y, const Forc32& F,
         X.fb = fr(0) + fr(1) + fr(2) + fr(4) + fr(6) + fr(7);
         X.fc = fr(3) + fr(5);
         X.fs = fr(8) + fr(9);
+        X.fr4 = S(IBIS_STAT_FRAC, 10);
+        X.fr3 = S(IBIS_STAT_FRAC, 11);
         X.rlai = (double)lai0 * rcp_nr(fmax((double)(lai0 + sai0), (double)eps));
     }
     double Wv[9] = {(double)c.tu, (double)c.ts, (double)c.tl, (double)c.t12, (double)c.t34,
@@ -1095,7 +1107,7 @@ __device__ __forceinline__ void surface_phase32(Col32& c, Y& y, const Forc32& F,
         const F2 tair((float)Wv[3], (float)Wv[4]), qair((float)Wv[5], (float)Wv[6]);
         Trans<float> T;
         transfer32(T, tc, y.A, tair.lo(), tair.hi(), qair.lo(), qair.hi(), first, P);
-        const F2 eair = esat2(tair), qsair = qsat2(eair, X.ps);
+        const F2 eair = esat2(tair), rair = sat_quotient2(eair, X.ps), qsair = eair * rair;
         stomata32<SUN_U, SUN_L>(st, c, tu, tl, qair, qsair, T.su, T.sl, y, P, q);
         if (!first) {
             const float tg = (float)Wv[7], ti = (float)Wv[8];
@@ -1103,7 +1115,7 @@ __device__ __forceinline__ void surface_phase32(Col32& c, Y& y, const Forc32& F,
             wlg = weight_veg2(F2(tl, tg), X.ch_lg, X.wl_lg, X.ws_lg, wlg, P);
             wi = weight_snow(ti, c.ti, wi, false, P);
         }
-        turvap32(Wv, tv, c, T, wus, wlg, wi, X, st, S, eair.hi(), qsair.hi(), it == 2, P);
+        turvap32(Wv, tv, c, T, wus, wlg, wi, X, st, S, rair.hi(), qsair.hi(), it == 2, P);
     }
     const float ti_new = mn((float)Wv[8], P.tmelt);
     const float tg_w = (float)Wv[7];
@@ -1180,7 +1192,6 @@ static_assert(NL == 6, "three pairs of soil layers");
 
 __device__ __forceinline__ F2 load2(const float (&a)[NL], int j) { return F2(a[2 * j], a[2 * j + 1]); }
 __device__ __forceinline__ F2 stat_pair(const Stat32& S, int p, int j) { return stat2(S, p, 2 * j); }
-__device__ __forceinline__ F2 par2(const float (&a)[NL], int j) { return F2(a[2 * j], a[2 * j + 1]); }
 
 // soilh2o (soil_physics.py:196-373): the implicit system in float, solved for the
 // hour's increments delta = w_new - w; w, wpud advanced, wflo the fluxes.  Its
@@ -1212,9 +1223,7 @@ __device__ __forceinline__ void soil_water32(F2 (&w2)[NP], float& wpud, float (&
 #pragma unroll
         for (int j = 0; j < NP; ++j) {
             const int k = 2 * j + 1;
-            const F2 wp(P.sw32_wp[k], k + 1 < NL ? P.sw32_wp[k + 1] : 0.0f);
-            const F2 wm(P.sw32_wm[k], k + 1 < NL ? P.sw32_wm[k + 1] : 1.0f);
-            const F2 rhm(P.sw32_rhm[k], k + 1 < NL ? P.sw32_rhm[k + 1] : 0.0f);
+            const F2 wp(P.iwp2[j]), wm(P.iwm2[j]), rhm(P.irh2[j]);
             const F2 a = wm * F2(hyd[k - 1], hyd[k]) + wp * F2(hyd[k], hyd[k + 1]);
             const F2 b = wm * F2(hs[k - 1], hs[k]) + wp * F2(hs[k], hs[k + 1]);
             const F2 zb = wm * F2(bex[k - 1], bex[k]) + wp * F2(bex[k], bex[k + 1]) + 0.5f;
@@ -1248,11 +1257,11 @@ __device__ __forceinline__ void soil_water32(F2 (&w2)[NP], float& wpud, float (&
         F2 wp(0.0f, w2[0].lo());
 #pragma unroll
         for (int j = 0; j < NP; ++j) {
-            const F2 dt = P.dtime * rcp2(mx2(pflo[j] * par2(P.hsoi, j), 1e-30f));
-            const F2 rhb = par2(P.sw32_rhb, j), gb = gp * rhb, gn = g[j] * par2(P.sw32_rhp, j);
-            const F2 d1 = dt * (fp * par2(P.sw32_c1, j) - gb);
-            const F2 d3 = dt * (F2(0.0f) - f[j] * par2(P.sw32_c6, j) - gn);
-            const F2 d2m = dt * (fp * par2(P.sw32_c5, j) - f[j] * par2(P.sw32_c3, j) + gn + gb);
+            const F2 dt = P.dtime * rcp2(mx2(pflo[j] * F2(P.h2[j]), 1e-30f));
+            const F2 rhb = F2(P.rhb2[j]), gb = gp * rhb, gn = g[j] * F2(P.rhp2[j]);
+            const F2 d1 = dt * (fp * F2(P.c12[j]) - gb);
+            const F2 d3 = dt * (F2(0.0f) - f[j] * F2(P.c62[j]) - gn);
+            const F2 d2m = dt * (fp * F2(P.c52[j]) - f[j] * F2(P.c32[j]) + gn + gb);
             const F2 wn(w2[j].hi(), j + 1 < NP ? w2[j + 1].lo() : 0.0f);
             F2 rk = e[j] - ep;
             if (j == 0) rk = rk + F2(src, 0.0f);
@@ -1275,7 +1284,7 @@ __device__ __forceinline__ void soil_water32(F2 (&w2)[NP], float& wpud, float (&
     float over_kg = 0.0f;      // saturation excess passed up, kg m-2
 #pragma unroll
     for (int j = NP - 1; j >= 0; --j) {
-        const F2 zz2 = P.rhow * par2(P.hsoi, j) * por[j] * mx2(1.0f - wi2[j], P.epsilon);
+        const F2 zz2 = P.rhow * F2(P.h2[j]) * por[j] * mx2(1.0f - wi2[j], P.epsilon);
         const F2 rz2 = rcp2(zz2);
         float wn[2];
 #pragma unroll
@@ -1318,7 +1327,7 @@ __device__ __forceinline__ void soil_heat32(F2 (&t)[NP], float (&tb)[NB], float 
     F2 res[NP], ts[NP], rc1[NP], c0[NP], dc[NP], c1[NP];
 #pragma unroll
     for (int j = 0; j < NP; ++j) {
-        const F2 h = par2(P.hsoi, j);
+        const F2 h = F2(P.h2[j]);
         res[j] = h * 0.5f * rcp2(mx2(cons[j], 1e-12f));
         ts[j] = t[j] + dtp[j];                            // starting temperatures, for the advected heat
         const F2 r2 = por[j] * (1.0f - wi[j]) * chr, r13 = rsol[j] + por[j] * wi[j] * cir;
@@ -1342,12 +1351,12 @@ __device__ __forceinline__ void soil_heat32(F2 (&t)[NP], float (&tb)[NB], float 
             con[j] = rcp2(res[j] + F2(res[j].hi(), res[j + 1].lo()));
             const F2 up_(ts[j].lo(), ts[j].hi()), dn(ts[j].hi(), ts[j + 1].lo());
             whf[j] = F2(wflo[k], wflo[k + 1]) * P.ch2o *
-                     (F2(P.hs_below[k], P.hs_below[k + 1]) * up_ + F2(P.hs_above[k], P.hs_above[k + 1]) * dn);
+                     (F2(P.hsb2[j]) * up_ + F2(P.hsa2[j]) * dn);
         } else {
             const float c5 = 1.0f / (res[j].lo() + res[j].hi());
             const float c6 = NBED > 0 ? 1.0f / (res[j].hi() + P.bed_res[0]) : 0.0f;
             con[j] = F2(c5, c6);
-            whf[j] = F2(wflo[k] * P.ch2o * (P.hs_below[k] * ts[j].lo() + P.hs_above[k] * ts[j].hi()), drain);
+            whf[j] = F2(wflo[k] * P.ch2o * (P.hs_below5 * ts[j].lo() + P.hs_above5 * ts[j].hi()), drain);
         }
     }
     // res holds half the layer's resistance with itself: con = 1 / (r[k-1] + r[k])
@@ -1413,7 +1422,7 @@ __device__ __forceinline__ float water_bounds32(F2 (&w)[NP], F2 (&i)[NP], const 
     float tot = 0.0f;
 #pragma unroll
     for (int j = 0; j < NP; ++j) {
-        const F2 z = par2(P.hsoi, j) * por[j] * P.rhow;
+        const F2 z = F2(P.h2[j]) * por[j] * P.rhow;
         const F2 zero(0.0f);
         F2 ww = mn2(sel2(w[j].lo() < eps, w[j].hi() < eps, zero, w[j]), 1.0f);
         const F2 ii = mn2(sel2(i[j].lo() < eps, i[j].hi() < eps, zero, i[j]), 1.0f);
@@ -1486,7 +1495,7 @@ __device__ __forceinline__ float methane32(float f_inund, float rh, const F2 (&t
     F2 tt(0.0f), tw(0.0f);
 #pragma unroll
     for (int j = 0; j < NP; ++j) {
-        const F2 an = mn2(mx2(par2(P.hsoi_bot, j) - mx2(par2(P.hsoi_top, j), zwt), 0.0f), par2(P.hsoi, j));
+        const F2 an = mn2(mx2(F2(P.bot2[j]) - mx2(F2(P.top2[j]), zwt), 0.0f), F2(P.h2[j]));
         const F2 th = sel2(t[j].lo() >= 273.15f, t[j].hi() >= 273.15f, an, F2(0.0f));
         tt = tt + th;
         tw = tw + th * t[j];
@@ -1514,8 +1523,16 @@ __device__ __forceinline__ void ground_phase32(Col32& c, const Forc32& F, const 
     const float tu = c.tu, tl = c.tl;
 
     // ---- 10. snow (loops.py:676-848)
-    float smelt, zheat, sflo_bot, fhtop_snow;
-    {
+    float smelt = 0.0f, zheat = 0.0f, sflo_bot = 0.0f, fhtop_snow = 0.0f;
+    // Bare of snow and none falling on it: the block's result is known (cover below
+    // fimin melts to none, layers at the melting point), and a warp of such columns
+    // skips it.  Launches with diagnostics report the block's fluxes too.
+    const bool snowy = DIAG || !(fi == 0.0f && M.snowg == 0.0f && c.hsno[0] == 0.0f && c.hsno[1] == 0.0f &&
+                                 c.hsno[2] == 0.0f && P.fimin > 0.0f);
+    if (!snowy) {
+        c.tsno[0] = c.tsno[1] = c.tsno[2] = P.tmelt;
+        c.tlsub = tl;
+    } else {
         float wliql = c.wliql, wsnol = c.wsnol;
         fhtop_snow = M.heati + M.rainl * (P.ch2o * (M.trainl - P.tmelt) + P.hfus + P.cice * (P.tmelt - c.tsno[0])) +
                      M.snowl * P.cice * (M.tsnowl - c.tsno[0]);
@@ -1534,8 +1551,6 @@ __device__ __forceinline__ void ground_phase32(Col32& c, const Forc32& F, const 
         const float fi1 = fi + dfi, rfi1 = 1.0f / mx(fi1, eps);
         float tm[NS], hm[NS];
         const bool fresh = (fi < eps) && (dfi > 0.0f);
-        smelt = 0.0f;
-        zheat = 0.0f;
         float htc = 0.0f;
 #pragma unroll
         for (int k = 0; k < NS; ++k) {
@@ -1657,10 +1672,10 @@ __device__ __forceinline__ void ground_phase32(Col32& c, const Forc32& F, const 
         const float gl = fulll ? gtransl : gtransl / mx(G.stresstl, eps);
 #pragma unroll
         for (int j = 0; j < NP; ++j) {
-            const F2 frl(P.froot[4 * j], P.froot[4 * j + 2]), fru(P.froot[4 * j + 1], P.froot[4 * j + 3]);
+            const F2 frl(P.frl2[j]), fru(P.fru2[j]);
             const F2 z(G.zw[2 * j], G.zw[2 * j + 1]);
             const F2 uu = fru * gu * (fullu ? F2(1.0f) : z), ul = frl * gl * (fulll ? F2(1.0f) : z);
-            const F2 h = par2(P.hsoi, j);
+            const F2 h = F2(P.h2[j]);
             pflo[j] = mx2(por[j] * mx2(1.0f - wisw[j], eps), eps);
             wsw[j] = mx2(wsw[j] - (uu + ul) * (dt / P.rhow) * rcp2(pflo[j] * h), 0.0f);
             F2 cx = (rsol[j] + por[j] * P.rhow * ((1.0f - wisw[j]) * wsw[j] * P.ch2o + wisw[j] * P.cice)) * h;
@@ -1738,7 +1753,7 @@ __device__ __forceinline__ void ground_phase32(Col32& c, const Forc32& F, const 
         F2 rt(0.0f);
 #pragma unroll
         for (int j = 0; j < NP; ++j)
-            rt = rt + t[j] * (F2(P.froot[4 * j], P.froot[4 * j + 2]) + F2(P.froot[4 * j + 1], P.froot[4 * j + 3]));
+            rt = rt + t[j] * (F2(P.frl2[j]) + F2(P.fru2[j]));
         const F2 tr = mx2(F2(c.ts, 0.5f * rt.sum()), 200.0f);
         const F2 fun = ex2((float(1.0 / 288.16) - rcp2(tr)) * 3500.0f);
         const float funca = fun.lo(), funcb = fun.hi();
@@ -1776,9 +1791,9 @@ __device__ __forceinline__ void ground_phase32(Col32& c, const Forc32& F, const 
                                  share);
                 }
             }
-            F2 r = F2(q.rroot(j), q.rroot(j + 1)) * stat2(S, IBIS_STAT_CBIOR, j) * funcb;
-            if (j < 10) r = r + F2(q.rwood(j), q.rwood(j + 1)) * stat2(S, IBIS_STAT_CBIOW, j) * (j < 8 ? wsu : funca);
-            const F2 inc = F2(q.keep(j), q.keep(j + 1)) * (an * share * (j < 8 ? covu : covl) - r) * cf;
+            F2 r = F2(q.rroot2(j)) * stat2(S, IBIS_STAT_CBIOR, j) * funcb;
+            if (j < 10) r = r + F2(q.rwood2(j)) * stat2(S, IBIS_STAT_CBIOW, j) * (j < 8 ? wsu : funca);
+            const F2 inc = F2(q.keep2(j)) * (an * share * (j < 8 ? covu : covl) - r) * cf;
             const F2 grew = Ac.add2(IBIS_ACC_AYNPP + j, IBIS_ACC_AYNPP + j + 1, inc);
             npp = npp + (Ac.kahan ? inc : grew);
         }

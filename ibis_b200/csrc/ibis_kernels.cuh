@@ -26,12 +26,11 @@ struct LaunchConfig {
 };
 constexpr LaunchConfig kConfigs[] = {
     {0, 128, 2, 0, 0}, {0, 64, 4, 0, 0},  {0, 96, 2, 0, 0},    {0, 128, 3, 0, 0},
-    {0, 32, 8, 0, 0},  {0, 192, 1, 0, 0}, {0, 224, 1, 0, 0},   {0, 256, 1, 0, 0},
+    {0, 160, 1, 0, 0}, {0, 192, 1, 0, 0}, {0, 224, 1, 0, 0},   {0, 256, 1, 0, 0},
     {1, 128, 2, 128, 3}, {1, 256, 1, 256, 2}, {1, 128, 3, 128, 4}, {2, 224, 1, 0, 0}};
 constexpr int kNumConfigs = sizeof(kConfigs) / sizeof(kConfigs[0]);
 constexpr int kDefaultFused = 0;
 constexpr int kLongFused = 6;
-constexpr int kSmallFused = 4;
 constexpr int kDefaultSplit = 8;
 
 // FP32 kernels keep each column's prognostic state in shared memory (array of
@@ -159,17 +158,16 @@ __device__ __forceinline__ void acc_move(float* __restrict__ g, int ld, float2* 
 // Bytes of shared memory per thread the on-chip accumulators take
 constexpr size_t kAccChipBytes = 2 * kAccPairs * sizeof(float2);
 
-// Whether a fused configuration keeps its accumulators in shared memory: the
-// column state plus the on-chip accumulator planes of MINB resident blocks must fit
-// the SM's 228 KB (1 KB reserved per block).  Launches of fewer than
-// kAccSmemMinSteps hours keep them in global memory instead (ACCSM = false):
-// the on-chip copy only pays back over several hours, and the larger
-// shared-memory carveout leaves less L1 for the register spills.
-template <typename R, int BLOCK, int MINB, bool ACCSM = true, size_t HOUR = sizeof(HourScratch<false, false>)>
+// Whether a fused configuration keeps its accumulators in shared memory: with the
+// column state and the hour's record, MINB resident blocks must fit the SM's 228 KB
+// (1 KB reserved per block) -- or one, for the variants whose record is larger.  On
+// chip they pay from the first hour: 33,001 columns for one hour 43 against 44 us with
+// the accumulators in global memory, for three 77 against 86 us.
+template <typename R, int BLOCK, int MINB, size_t HOUR>
 struct AccInSmem {
-    static constexpr bool value =
-        ACCSM && StateInSmem<R>::value &&
-        ((sizeof(Col<R>) + kAccChipBytes + HOUR) * BLOCK + 1024) * MINB <= 228 * 1024;
+    static constexpr size_t per_block = (sizeof(Col<R>) + kAccChipBytes + HOUR) * BLOCK + 1024;
+    static constexpr int resident = HOUR > sizeof(HourScratch<false, false>) ? 1 : MINB;
+    static constexpr bool value = StateInSmem<R>::value && per_block * resident <= 228 * 1024;
 };
 
 // A block's shared memory in the FP32 kernels: the columns' state, the on-chip
@@ -186,7 +184,6 @@ struct BlockSmem {
         return reinterpret_cast<Hour*>(smem + hour_off)[threadIdx.x];
     }
 };
-constexpr int kAccSmemMinSteps = 4;
 
 // The uniform parameter source of a kernel: with X3 the one that compiles in the
 // IBIS 3.0 extensions of the step (any IBIS_FLAGS_X3 flag selects those kernels).
@@ -198,8 +195,8 @@ __device__ __forceinline__ auto uniform_source(const DevParams<R>& P) {
 
 // The block's `n` threads (whole warps) start an hour together.  A warp that follows
 // another closely finds its instructions in the SM's instruction cache; warps spread
-// over the body each stream it from the next level (six hours of 33,152 columns: 0.146
-// ms together, 0.157 without in blocks of 64).  Once an hour is enough: a warp that
+// over the body each stream it from the next level (six hours of 95,333 columns in blocks
+// of 128: 0.434 ms together, 0.444 without).  Once an hour is enough: a warp that
 // falls behind fetches faster than the one it follows.
 template <bool ON>
 __device__ __forceinline__ void align_warps(unsigned n) {
@@ -212,7 +209,7 @@ __device__ __forceinline__ void align_warps(unsigned n) {
 // Status word written by the kernels: [0] bit 0 = a column left the step with a
 // non-finite prognostic value; [1] = smallest such cell index (INT_MAX if none).
 // DG: whether the kernel can write diagnostics.
-template <typename R, int NT, bool SU, bool SL, int BLOCK, int MINB, bool ACCSM, bool X3, bool DG>
+template <typename R, int NT, bool SU, bool SL, int BLOCK, int MINB, bool X3, bool DG>
 __global__ void __launch_bounds__(BLOCK, MINB) hourly_step_kernel(R* __restrict__ prog, const R* __restrict__ stat,
                                                              const R* __restrict__ forc, R* __restrict__ diag,
                                                              R* __restrict__ acc, int ncell, int ld, int nstep,
@@ -235,7 +232,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) hourly_step_kernel(R* __restrict_
     load_col(c, prog + i, ld);
     Stat<R> S{stat + i, ld};
     const Diag<R, DG> D{DG && diag && live ? diag + i : nullptr, ld};
-    constexpr bool kAccSmem = AccInSmem<R, BLOCK, MINB, ACCSM, sizeof(HourScratch<SU || SL, X3>)>::value;
+    constexpr bool kAccSmem = AccInSmem<R, BLOCK, MINB, sizeof(HourScratch<SU || SL, X3>)>::value;
     using SM = BlockSmem<R, SU || SL, X3, BLOCK, kAccSmem>;
     Acc<R, kAccSmem ? BLOCK : 0> A{acc ? acc + i : nullptr, ld, (P.flags & IBIS_FLAG_KAHAN) != 0};
     A.live = live;
@@ -371,7 +368,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) hourly_step_staged_kernel(
     R* __restrict__ prog, const R* __restrict__ stat, const R* __restrict__ forc, R* __restrict__ acc, int ncell,
     int ld, int nstep, long long forc_stride, const DevParams<R> P, int* __restrict__ status) {
     static_assert(sizeof(R) == 4 && StateInSmem<R>::value, "the staged form is the FP32 shared-memory kernel");
-    static_assert(AccInSmem<R, BLOCK, MINB, true, sizeof(HourScratch<SU || SL, X3>)>::value,
+    static_assert(AccInSmem<R, BLOCK, MINB, sizeof(HourScratch<SU || SL, X3>)>::value,
                   "the staged form keeps the accumulators on chip");
     using SM = StagedSmem<R, SU || SL, X3, BLOCK, MINB>;
     static_assert((SM::total + 1024) * MINB <= 228 * 1024, "staged shared memory exceeds the SM");
@@ -504,6 +501,71 @@ __global__ void __launch_bounds__(BLOCK, MINB) ground_kernel(R* __restrict__ pro
 // host side
 // ---------------------------------------------------------------------------
 
+static inline ParPair par_pair(double a, double b) {
+    const float v[2] = {(float)a, (float)b};
+    ParPair p;
+    memcpy(&p, v, sizeof p);
+    return p;
+}
+
+// The register pairs of the FP32 step (DevParams)
+template <typename R>
+static void set_pairs(DevParams<R>& d, const IbisParams& h) {
+    double top = 0.0;
+    for (int j = 0; j < NL / 2; ++j) {
+        const int k = 2 * j, m = k + 1;
+        auto below = [&](int q) { return h.hsoi[q < NL - 1 ? q + 1 : q]; };
+        auto above = [&](int q) { return h.hsoi[q > 0 ? q - 1 : 0]; };
+        d.h2[j] = par_pair(h.hsoi[k], h.hsoi[m]);
+        d.rhb2[j] = par_pair(1.0 / d.sw_hb[k], 1.0 / d.sw_hb[m]);
+        d.rhp2[j] = par_pair(1.0 / d.sw_hp[k], 1.0 / d.sw_hp[m]);
+        d.c12[j] = par_pair(0.5 * h.hsoi[k] / d.sw_hb[k], 0.5 * h.hsoi[m] / d.sw_hb[m]);
+        d.c32[j] = par_pair(0.5 * below(k) / d.sw_hp[k], 0.5 * below(m) / d.sw_hp[m]);
+        d.c52[j] = par_pair(0.5 * above(k) / d.sw_hb[k], 0.5 * above(m) / d.sw_hb[m]);
+        d.c62[j] = par_pair(0.5 * h.hsoi[k] / d.sw_hp[k], 0.5 * h.hsoi[m] / d.sw_hp[m]);
+        // interfaces m and m + 1; past the last layer, one layer of weight 1 and no gradient
+        const bool in = m + 1 < NL;
+        d.iwp2[j] = par_pair(d.sw_wp[m], in ? d.sw_wp[m + 1] : 0.0);
+        d.iwm2[j] = par_pair(d.sw_wm[m], in ? d.sw_wm[m + 1] : 1.0);
+        d.irh2[j] = par_pair(1.0 / d.sw_hm[m], in ? 1.0 / d.sw_hm[m + 1] : 0.0);
+        if (in) {
+            const double s0 = h.hsoi[k] + h.hsoi[m], s1 = h.hsoi[m] + h.hsoi[m + 1];
+            d.hsb2[j] = par_pair(h.hsoi[m] / s0, h.hsoi[m + 1] / s1);
+            d.hsa2[j] = par_pair(h.hsoi[k] / s0, h.hsoi[m] / s1);
+        }
+        d.top2[j] = par_pair(top, top + h.hsoi[k]);
+        d.bot2[j] = par_pair(top + h.hsoi[k], top + h.hsoi[k] + h.hsoi[m]);
+        top = top + h.hsoi[k] + h.hsoi[m];
+        d.frl2[j] = par_pair(h.froot[2 * k], h.froot[2 * m]);
+        d.fru2[j] = par_pair(h.froot[2 * k + 1], h.froot[2 * m + 1]);
+    }
+    for (int k = 0; k < NL; ++k) d.fr2[k] = par_pair(h.froot[2 * k], h.froot[2 * k + 1]);
+    for (int st = 0; st < 2; ++st) {
+        d.rho2[st] = par_pair(h.rhoveg[st], h.rhoveg[2 + st]);
+        d.tau2[st] = par_pair(h.tauveg[st], h.tauveg[2 + st]);
+        const int a = st ? 2 : 0, b = st ? 4 : 1;
+        d.gam2[st] = par_pair(h.gamma[a], h.gamma[b]);
+        d.b02[st] = par_pair(h.coefb[a], h.coefb[b]);
+        d.gmin2[st] = par_pair(h.gsmin[a], h.gsmin[b]);
+        d.cm2[st] = par_pair(h.coefm[a], h.coefm[b]);
+    }
+    d.osno2 = par_pair(h.omegasno[0], h.omegasno[1]);
+    const double drip[3] = {h.tdripu, h.tdrips, h.tdripl}, blow[3] = {h.tblowu, h.tblows, h.tblowl};
+    for (int k = 0; k < 3; ++k) {
+        d.drip2[k] = par_pair(1.0 / drip[k], 1.0 / blow[k]);
+        d.kdrip2[k] = par_pair(1.0 - h.dtime / drip[k], 1.0 - h.dtime / blow[k]);
+    }
+    d.water2 = par_pair(h.ch2o, h.cice);
+    d.ralai2 = par_pair(1.0 / h.alaiml, 1.0 / h.alaimu);
+    d.chus2 = par_pair(h.chu, h.chs);
+    d.vml2 = par_pair(h.vmax_pft[8], h.vmax_pft[11]);
+    for (int j = 0; j < 6; ++j) {
+        d.rroot2[j] = par_pair(d.rroot_s[2 * j], d.rroot_s[2 * j + 1]);
+        if (j < 5) d.rwood2[j] = par_pair(d.rwood_s[2 * j], d.rwood_s[2 * j + 1]);
+        d.keep2[j] = par_pair(d.keep[2 * j], d.keep[2 * j + 1]);
+    }
+}
+
 template <typename R>
 static DevParams<R> make_dev_params(const IbisParams& h) {
     DevParams<R> d;
@@ -523,6 +585,13 @@ static DevParams<R> make_dev_params(const IbisParams& h) {
     d.znorm = (R)(1.0 - exp(h.stressfac));
     d.rdt = (R)(1.0 / h.dtime);
     d.zir = (R)(4.0 * 0.95 * h.stef);
+    // respiration tables formed in float32 as the reference does (loops_gswp3.py:185-190)
+    const float per_s = (float)(h.ndaypy * 86400.0), mol = (float)(1000.0 / 12.0);
+    for (int j = 0; j < 12; ++j) {
+        d.rwood_s[j] = (R)(((float)h.rwood[j] / per_s) * mol);
+        d.rroot_s[j] = (R)(((float)h.rroot[j] / per_s) * mol);
+        d.keep[j] = (R)(1.0f - (float)h.rgrowth[j]);
+    }
     for (int k = 1; k < NL; ++k) {
         d.sw_hm[k] = 0.5 * (h.hsoi[k - 1] + h.hsoi[k]);
         d.sw_wp[k] = 0.5 * h.hsoi[k] / d.sw_hm[k];
@@ -533,23 +602,6 @@ static DevParams<R> make_dev_params(const IbisParams& h) {
         d.sw_hb[k] = hb > 1e-30 ? hb : 1e-30;
         double hp = k < NL - 1 ? 0.5 * (h.hsoi[k] + h.hsoi[k + 1]) : 1.0;
         d.sw_hp[k] = hp > 1e-30 ? hp : 1e-30;
-        const int km1 = k > 0 ? k - 1 : 0, kp1 = k < NL - 1 ? k + 1 : k;
-        d.sw32_wp[k] = (float)d.sw_wp[k];
-        d.sw32_wm[k] = (float)d.sw_wm[k];
-        d.sw32_rhm[k] = k > 0 ? (float)(1.0 / d.sw_hm[k]) : 0.0f;
-        d.sw32_rhb[k] = (float)(1.0 / d.sw_hb[k]);
-        d.sw32_rhp[k] = (float)(1.0 / d.sw_hp[k]);
-        d.sw32_c1[k] = (float)(0.5 * h.hsoi[k] / d.sw_hb[k]);
-        d.sw32_c3[k] = (float)(0.5 * h.hsoi[kp1] / d.sw_hp[k]);
-        d.sw32_c5[k] = (float)(0.5 * h.hsoi[km1] / d.sw_hb[k]);
-        d.sw32_c6[k] = (float)(0.5 * h.hsoi[k] / d.sw_hp[k]);
-    }
-    const double drip[3] = {h.tdripu, h.tdrips, h.tdripl}, blow[3] = {h.tblowu, h.tblows, h.tblowl};
-    for (int k = 0; k < 3; ++k) {
-        d.rtdrip[k] = (R)(1.0 / drip[k]);
-        d.rtblow[k] = (R)(1.0 / blow[k]);
-        d.kdrip[k] = (R)(1.0 - h.dtime / drip[k]);
-        d.kblow[k] = (R)(1.0 - h.dtime / blow[k]);
     }
     d.rtheta3 = (R)(1.0 / h.theta3);
     d.rbeta3 = (R)(1.0 / h.beta3);
@@ -558,10 +610,9 @@ static DevParams<R> make_dev_params(const IbisParams& h) {
     d.ksu = (R)(h.cleaf * sqrt(1.0 / h.dleaf[1]));
     d.kss = (R)(h.cstem * sqrt(1.0 / h.dstem[1]));
     d.ksl = (R)(h.cgrass * sqrt(1.0 / h.dleaf[0]));
-    for (int k = 1; k < NL; ++k) {
-        d.hs_below[k] = (R)(h.hsoi[k] / (h.hsoi[k - 1] + h.hsoi[k]));
-        d.hs_above[k] = (R)(h.hsoi[k - 1] / (h.hsoi[k - 1] + h.hsoi[k]));
-    }
+    d.hs_below5 = (R)(h.hsoi[5] / (h.hsoi[4] + h.hsoi[5]));
+    d.hs_above5 = (R)(h.hsoi[4] / (h.hsoi[4] + h.hsoi[5]));
+    set_pairs(d, h);
     const double cbed = h.consoi_bed > 1e-12 ? h.consoi_bed : 1e-12;
     for (int k = 0; k < NB; ++k) {
         d.bed_res[k] = (R)(0.5 * h.hsoi_bed[k] / cbed);
@@ -569,13 +620,6 @@ static DevParams<R> make_dev_params(const IbisParams& h) {
         d.bed_rw[k] = (R)(h.dtime / (h.csoi_bed * h.rhosoi_bed * h.hsoi_bed[k]));
     }
     d.rdt64 = 1.0 / h.dtime;
-    // respiration tables formed in float32 as the reference does (loops_gswp3.py:185-190)
-    const float per_s = (float)(h.ndaypy * 86400.0), mol = (float)(1000.0 / 12.0);
-    for (int j = 0; j < 12; ++j) {
-        d.rwood_s[j] = (R)(((float)h.rwood[j] / per_s) * mol);
-        d.rroot_s[j] = (R)(((float)h.rroot[j] / per_s) * mol);
-        d.keep[j] = (R)(1.0f - (float)h.rgrowth[j]);
-    }
     // crop_vfac's increments (loops.py:218-231), float32 values as the reference forms them
     for (int j = 0; j < 12; ++j) d.crop_inc[j] = (R)0.0;
     if (h.crop_c4_share < 0.0) {
@@ -651,14 +695,14 @@ cudaError_t fit_smem_once(unsigned long long& done, K k, int block, size_t smem,
     return e;
 }
 
-template <typename R, int NT, bool SU, bool SL, int BLOCK, int MINB, bool ACCSM, bool X3, bool DG>
+template <typename R, int NT, bool SU, bool SL, int BLOCK, int MINB, bool X3, bool DG>
 cudaError_t launch_fused(R* prog, const R* stat, const R* forc, R* diag, R* acc, int ncell, int ld, int nstep,
                          long long fstride, const DevParams<R>& P, int* status, cudaStream_t s) {
     const int grid = (ncell + BLOCK - 1) / BLOCK;
     constexpr size_t smem =
         BlockSmem<R, SU || SL, X3, BLOCK,
-                  AccInSmem<R, BLOCK, MINB, ACCSM, sizeof(HourScratch<SU || SL, X3>)>::value>::total;
-    auto k = hourly_step_kernel<R, NT, SU, SL, BLOCK, MINB, ACCSM, X3, DG>;
+                  AccInSmem<R, BLOCK, MINB, sizeof(HourScratch<SU || SL, X3>)>::value>::total;
+    auto k = hourly_step_kernel<R, NT, SU, SL, BLOCK, MINB, X3, DG>;
     static unsigned long long fitted = 0;
     cudaError_t e = fit_smem_once(fitted, k, BLOCK, smem, smem);
     if (e != cudaSuccess) return e;
@@ -674,7 +718,7 @@ template <typename R, int NT, bool SU, bool SL, int BLOCK, int MINB, bool X3>
 cudaError_t launch_staged(R* prog, const R* stat, const R* forc, R* acc, int ncell, int ld, int nstep,
                           long long fstride, const DevParams<R>& P, int* status, cudaStream_t s) {
     if ((reinterpret_cast<uintptr_t>(forc) & 15) != 0 || (fstride & 3) != 0 || (ld & 3) != 0)
-        return launch_fused<R, NT, SU, SL, BLOCK, MINB, true, X3, false>(prog, stat, forc, nullptr, acc, ncell, ld,
+        return launch_fused<R, NT, SU, SL, BLOCK, MINB, X3, false>(prog, stat, forc, nullptr, acc, ncell, ld,
                                                                          nstep, fstride, P, status, s);
     using SM = StagedSmem<R, SU || SL, X3, BLOCK, MINB>;
     const int grid = (ncell + BLOCK - 1) / BLOCK;
@@ -706,31 +750,25 @@ cudaError_t launch_split(R* prog, const R* stat, const R* forc, R* diag, R* acc,
     return cudaGetLastError();
 }
 
-// Launches that write diagnostics run the default configuration of their form, or
-// the small-batch one (dispatch_config): the only ones compiled with the diagnostics
-// writer; the float64 kernels always carry it.
+// Launches that write diagnostics run the default configuration of their form
+// (dispatch_config): the only ones compiled with the diagnostics writer; the float64
+// kernels always carry it.
 template <typename R, int NT, bool SU, bool SL, int CFG, bool X3 = false>
 cudaError_t run_config(R* prog, const R* stat, const R* forc, R* diag, R* acc, R* mid, int ncell, int ld, int nstep,
                        long long fs, const DevParams<R>& P, int* status, cudaStream_t s) {
     constexpr LaunchConfig C = kConfigs[CFG];
     if constexpr (sizeof(R) == 8) {
         // single-warp blocks: as many warps fit an SM, and a small batch spreads over more SMs
-        return launch_fused<R, NT, SU, SL, 32, 8, false, X3, true>(prog, stat, forc, diag, acc, ncell, ld,
-                                                                             nstep, fs, P, status, s);
+        return launch_fused<R, NT, SU, SL, 32, 8, X3, true>(prog, stat, forc, diag, acc, ncell, ld, nstep, fs, P,
+                                                            status, s);
     } else if constexpr (C.form == 0) {
-#define IBIS_FUSED(ACCSM, DG)                                                                                       \
-    launch_fused<R, NT, SU, SL, C.block, C.minb, ACCSM, X3, DG>(prog, stat, forc, diag, acc, ncell, ld, nstep, fs, P, \
-                                                                status, s)
-        // the default fused configuration (the plain entry points' and the
-        // per-hour callers') also has a global-accumulator twin for short launches
         if constexpr (CFG == kDefaultFused) {
-            if (diag) return nstep < kAccSmemMinSteps ? IBIS_FUSED(false, true) : IBIS_FUSED(true, true);
-            if (nstep < kAccSmemMinSteps) return IBIS_FUSED(false, false);
-        } else if constexpr (CFG == kSmallFused) {
-            if (diag) return IBIS_FUSED(true, true);
+            if (diag)
+                return launch_fused<R, NT, SU, SL, C.block, C.minb, X3, true>(prog, stat, forc, diag, acc, ncell, ld,
+                                                                              nstep, fs, P, status, s);
         }
-        return IBIS_FUSED(true, false);
-#undef IBIS_FUSED
+        return launch_fused<R, NT, SU, SL, C.block, C.minb, X3, false>(prog, stat, forc, diag, acc, ncell, ld, nstep,
+                                                                       fs, P, status, s);
     } else if constexpr (C.form == 2) {
         return launch_staged<R, NT, SU, SL, C.block, C.minb, X3>(prog, stat, forc, acc, ncell, ld, nstep, fs, P, status,
                                                                  s);
@@ -751,37 +789,29 @@ cudaError_t run_config(R* prog, const R* stat, const R* forc, R* diag, R* acc, R
 
 // Every (variant, configuration) pair the FP32 library instantiates: the F77
 // canopy (no sunlit/shaded split) in every configuration, the sunlit/shaded
-// variants in the default ones and the small-batch one.  X(NT, SU, SL, CFG).
+// variants and the IBIS 3.0 kernels (X3) in three.  X(NT, SU, SL, CFG).
 #define IBIS_F77_CONFIGS(X, NT)                                                                                \
     X(NT, false, false, 0) X(NT, false, false, 1) X(NT, false, false, 2) X(NT, false, false, 3)                \
     X(NT, false, false, 4) X(NT, false, false, 5) X(NT, false, false, 6) X(NT, false, false, 7)                \
     X(NT, false, false, 8) X(NT, false, false, 9) X(NT, false, false, 10) X(NT, false, false, 11)
 #define IBIS_SUN_CONFIGS(X, NT)                                                                                \
     X(NT, true, false, 0) X(NT, false, true, 0) X(NT, true, true, 0)                                           \
-    X(NT, true, false, 4) X(NT, false, true, 4) X(NT, true, true, 4)                                           \
+    X(NT, true, false, 6) X(NT, false, true, 6) X(NT, true, true, 6)                                           \
     X(NT, true, false, 8) X(NT, false, true, 8) X(NT, true, true, 8)
-// The IBIS 3.0 kernels (X3): every canopy variant in the same three, and the long
-// fused configuration for both canopies F77 or both sunlit/shaded.  X(NT, SU, SL, CFG).
 #define IBIS_X3_CONFIGS(X, NT)                                                                                 \
-    X(NT, false, false, 0) X(NT, false, false, 4) X(NT, false, false, 6) X(NT, false, false, 8)                \
-    X(NT, true, true, 0) X(NT, true, true, 4) X(NT, true, true, 6) X(NT, true, true, 8)                        \
-    X(NT, true, false, 0) X(NT, true, false, 4) X(NT, true, false, 8)                                          \
-    X(NT, false, true, 0) X(NT, false, true, 4) X(NT, false, true, 8)
+    X(NT, false, false, 0) X(NT, false, false, 6) X(NT, false, false, 8) IBIS_SUN_CONFIGS(X, NT)
 
-// The fused configuration of a launch that leaves it to the library, by how its
-// columns fill the chip (`sms` SMs).  Six hours on 148 SMs, milliseconds in blocks of
-// 32 / 2 x 128 / 224: 356 columns for a day 0.41 / 0.43 / 0.49; 12,007 0.125 / 0.122 /
-// 0.136; 33,152 0.169 / 0.146 / 0.144; 95,333 0.452 / 0.434 / 0.424.
-//   * up to a warp per SM: single-warp blocks, so every warp has an SM's caches to itself;
-//   * up to four: blocks of 128, one on each SM before any gets a second;
-//   * otherwise 2 x 128 or 1 x 224 threads per SM, whichever runs the batch in less: a
-//     wave of either takes the same within 2 %, so the number of waves decides.
-//     Launches too short to keep the accumulators on chip have the 128 form.
-inline int auto_config(int ncell, int nstep, int sms) {
-    if (ncell <= 32 * sms) return kSmallFused;
-    if (nstep < kAccSmemMinSteps || ncell <= 128 * sms) return kDefaultFused;
-    const int w8 = (ncell - 1) / (256 * sms), w7 = (ncell - 1) / (224 * sms);
-    return w7 <= w8 ? kLongFused : kDefaultFused;
+// The fused configuration of a launch that leaves it to the library (`sms` SMs).  Two
+// blocks of 128 per SM are the fastest at every size with the F77 canopy: six hours in
+// 2 x 128 / 4 x 64 / 1 x 224 / single-warp blocks, milliseconds: 12,007 columns 0.112 /
+// 0.117 / 0.128 / 0.133; 33,152 0.134 / 0.158 / 0.137 / 0.194; 95,333 0.404 / 0.409 /
+// 0.407 / 0.492 (four warps that run together fetch a body's instructions once for all).
+// The sunlit/shaded canopies and the IBIS 3.0 switches keep a larger record of the
+// hour: one block of 128 fits an SM with its accumulators, so batches of more than that
+// run as one block of 224.
+inline int auto_config(unsigned flags, int ncell, int sms) {
+    const bool large = (flags & (IBIS_FLAGS_X3 | IBIS_FLAG_SUNSHADE_U | IBIS_FLAG_SUNSHADE_L)) != 0;
+    return large && ncell > 128 * sms ? kLongFused : kDefaultFused;
 }
 
 template <typename R, int NT, bool SU, bool SL, bool X3>
@@ -792,20 +822,12 @@ cudaError_t dispatch_config(int cfg, R* prog, const R* stat, const R* forc, R* d
         // the float64 kernels always carry the IBIS 3.0 extensions: with their
         // switches off they perform the F77 step's operations
         return run_config<R, NT, SU, SL, kDefaultFused, true>(IBIS_ARGS);
-    } else if (diag) {
-        if (cfg == kSmallFused) return run_config<R, NT, SU, SL, kSmallFused, X3>(IBIS_ARGS);
-        if (kConfigs[cfg].form != 1) return run_config<R, NT, SU, SL, kDefaultFused, X3>(IBIS_ARGS);
-        return run_config<R, NT, SU, SL, kDefaultSplit, X3>(IBIS_ARGS);
-    } else if constexpr (X3) {
-        if (cfg == kSmallFused) return run_config<R, NT, SU, SL, kSmallFused, true>(IBIS_ARGS);
-        if (cfg == kLongFused && SU == SL) return run_config<R, NT, SU, SL, kLongFused, true>(IBIS_ARGS);
-        if (kConfigs[cfg].form != 1) return run_config<R, NT, SU, SL, kDefaultFused, true>(IBIS_ARGS);
-        return run_config<R, NT, SU, SL, kDefaultSplit, true>(IBIS_ARGS);
-    } else if constexpr (SU || SL) {
-        if (cfg == kSmallFused) return run_config<R, NT, SU, SL, kSmallFused>(IBIS_ARGS);
-        if (kConfigs[cfg].form != 1) return run_config<R, NT, SU, SL, kDefaultFused>(IBIS_ARGS);
-        return run_config<R, NT, SU, SL, kDefaultSplit>(IBIS_ARGS);
+    } else if constexpr (X3 || SU || SL) {
+        if (kConfigs[cfg].form == 1) return run_config<R, NT, SU, SL, kDefaultSplit, X3>(IBIS_ARGS);
+        if (cfg == kLongFused && !diag) return run_config<R, NT, SU, SL, kLongFused, X3>(IBIS_ARGS);
+        return run_config<R, NT, SU, SL, kDefaultFused, X3>(IBIS_ARGS);
     } else {
+        if (diag) cfg = kConfigs[cfg].form == 1 ? kDefaultSplit : kDefaultFused;
         switch (cfg) {
             case 1: return run_config<R, NT, SU, SL, 1>(IBIS_ARGS);
             case 2: return run_config<R, NT, SU, SL, 2>(IBIS_ARGS);

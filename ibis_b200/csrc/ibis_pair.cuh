@@ -8,6 +8,7 @@
 // as -use_fast_math does).
 #pragma once
 #include "ibis_math.cuh"
+#include "ibis_params.cuh"
 
 namespace ibis {
 
@@ -16,6 +17,7 @@ struct F2 {
     __device__ __forceinline__ F2() {}
     __device__ __forceinline__ F2(float a, float b) { asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(a), "f"(b)); }
     __device__ __forceinline__ F2(float s) : F2(s, s) {}
+    __device__ __forceinline__ F2(const ParPair& p) : v(p.v) {}
     __device__ __forceinline__ float lo() const {
         float a, b;
         asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
@@ -64,17 +66,31 @@ __device__ __forceinline__ F2 sel2(bool a, bool b, const F2& x, const F2& y) {
 }
 __device__ __forceinline__ F2 sel2(bool a, const F2& x, const F2& y) { return sel2(a, a, x, y); }
 
-// x**n per half for 0 <= n < 64, by repeated squaring
+// x**n per half for 0 <= n < 64, by repeated squaring.  Exponents of 16 and more
+// (a soil's Clapp-Hornberger exponent above 14) take the branch.
 __device__ __forceinline__ F2 ipow2(F2 x, int n0, int n1) {
     float r0 = 1.0f, r1 = 1.0f;
 #pragma unroll
-    for (int k = 0; k < 6; ++k) {
+    for (int k = 0; k < 4; ++k) {
         if (n0 & (1 << k)) r0 = r0 * x.lo();
         if (n1 & (1 << k)) r1 = r1 * x.hi();
-        if (k < 5) x = x * x;
+        if (k < 3) x = x * x;
+    }
+    if ((n0 | n1) >> 4) {
+#pragma unroll
+        for (int k = 4; k < 6; ++k) {
+            x = x * x;
+            if (n0 & (1 << k)) r0 = r0 * x.lo();
+            if (n1 & (1 << k)) r1 = r1 * x.hi();
+        }
     }
     return F2(r0, r1);
 }
+
+// The larger or smaller of two doubles by one comparison (the second where the first
+// is not a number, as fmax and fmin with an ordinary second)
+__device__ __forceinline__ double dmax(double a, double b) { return a > b ? a : b; }
+__device__ __forceinline__ double dmin(double a, double b) { return a < b ? a : b; }
 
 // Lowe (1977) saturation vapour pressure and its derivative (as esat and desat in
 // ibis_math.cuh: both branches on offsets clamped to their range) at two
@@ -105,11 +121,13 @@ __device__ __forceinline__ F2 desat2(const F2& t) {
 }
 #undef IBIS_LOWE2
 
-__device__ __forceinline__ F2 qsat2(const F2& e, float p) {
-    return e * 0.622f * rcp2(mx2(p - e * float(1.0 - 0.622), e * 0.622f));
+// Specific humidity at saturation, q = 0.622 e / max(p - 0.378 e, 0.622 e), and its
+// derivative desat q (1 + q (1/0.622 - 1)) / e, whose q / e is the same quotient.
+__device__ __forceinline__ F2 sat_quotient2(const F2& e, float p) {
+    return 0.622f * rcp2(mx2(p - e * float(1.0 - 0.622), e * 0.622f));
 }
-__device__ __forceinline__ F2 dqsat2(const F2& t, const F2& q, const F2& e) {
-    return desat2(t) * q * (1.0f + q * float(1.0 / 0.622 - 1.0)) * rcp2(e);
+__device__ __forceinline__ F2 sat_derivative2(const F2& t, const F2& q, const F2& qe) {
+    return desat2(t) * qe * (1.0f + q * float(1.0 / 0.622 - 1.0));
 }
 
 // Reciprocal of a finite, non-zero double by two Newton-Raphson steps

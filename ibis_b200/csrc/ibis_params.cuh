@@ -5,6 +5,11 @@
 
 namespace ibis {
 
+// Two floats as one 64-bit word
+struct ParPair {
+    unsigned long long v;
+};
+
 template <typename R>
 struct DevParams {
 #define IBIS_S(name) R name;
@@ -29,11 +34,6 @@ struct DevParams {
     double sw_hb[6];   // row k: max(0.5 h[0] | 0.5 h[k-1] + 0.5 h[k], 1e-30)
     double sw_hp[6];   // row k < 5: max(0.5 * (h[k] + h[k+1]), 1e-30)
     double rdt64;      // 1 / dtime in double
-    // the same geometry in float as multipliers, for the FP32 kernels' increment-form
-    // solve: sw_wp, sw_wm, 1/sw_hm, 1/sw_hb, 1/sw_hp, 0.5 h[k]/sw_hb, 0.5 h[k+1]/sw_hp,
-    // 0.5 h[k-1]/sw_hb, 0.5 h[k]/sw_hp
-    float sw32_wp[6], sw32_wm[6], sw32_rhm[6], sw32_rhb[6], sw32_rhp[6], sw32_c1[6], sw32_c3[6], sw32_c5[6],
-        sw32_c6[6];
     R rwood_s[12], rroot_s[12], keep[12];  // float32-formed respiration rates (loops_gswp3.py:185-190)
     R ch4_w;           // float32(dtime / 86400)
     R rh_conv;         // float32(12e-3 * 86400)
@@ -47,15 +47,28 @@ struct DevParams {
     // index of the launch's first column in the caller's numbering: a launch
     // over a group of columns (ibis_step_host_f32) reports status[1] in it
     int cell0;
-    // reciprocals and geometry the FP32 step multiplies by (formed in double on the host)
-    R rtdrip[3], rtblow[3];  // 1 / drip and blow-off times of the upper leaves, upper stems, lower canopy
-    R kdrip[3], kblow[3];    // 1 - dtime / time
+    // what the FP32 step multiplies by (formed in double on the host)
     R rtheta3, rbeta3, rtheta4, rbeta4;
     R ksu, kss, ksl;         // boundary-layer conductances of leaves, stems and lower canopy over rhoa sqrt(u)
-    R hs_below[6], hs_above[6];   // interface k (1..5): h[k] and h[k-1] over h[k-1] + h[k]
+    R hs_below5, hs_above5;  // h[5] and h[4] over h[4] + h[5]
     R bed_res[3];            // bedrock layer: half its thermal resistance
     R bed_con[3];            // conductance to the layer below
     R bed_rw[3];             // dtime over the heat capacity
+    // and the pairs of floats its packed arithmetic takes, each a 64-bit word (ParPair)
+    // so that one constant load fills a register pair
+    ParPair h2[3], rhb2[3], rhp2[3], c12[3], c32[3], c52[3], c62[3];   // soil layers (0,1), (2,3), (4,5): thickness,
+                             // 1/sw_hb, 1/sw_hp, 0.5 h[k]/sw_hb, 0.5 h[k+1]/sw_hp, 0.5 h[k-1]/sw_hb, 0.5 h[k]/sw_hp
+    ParPair iwp2[3], iwm2[3], irh2[3];   // interfaces (1,2), (3,4), (5,bottom): sw_wp, sw_wm, 1/sw_hm
+    ParPair hsb2[2], hsa2[2];            // interfaces (1,2), (3,4): h[k] and h[k-1] over h[k-1] + h[k]
+    ParPair top2[3], bot2[3];            // layer tops and bottoms
+    ParPair fr2[6], frl2[3], fru2[3];    // root profile: (lower, upper) of a layer; lower, upper of a pair of layers
+    ParPair rho2[2], tau2[2], osno2;     // (visible, near infrared) of the lower and upper story; snow's scattering
+    ParPair drip2[3], kdrip2[3];         // (1 / drip time, 1 / blow-off time), 1 - dtime / time: upper leaves, stems, lower
+    ParPair water2, ralai2, chus2;       // (ch2o, cice), 1 / (alaiml, alaimu), (chu, chs)
+    ParPair gam2[2], b02[2], gmin2[2];   // dark respiration, Ball-Berry intercept and least conductance of the
+                                         // C3 big leaves: broadleaf and conifer; shrub and C3 grass
+    ParPair cm2[2], vml2;                // their slopes; nominal vmax of the lower two
+    ParPair rroot2[6], rwood2[5], keep2[6];   // respiration rates of PFTs (0,1), (2,3) ...
     // per-band thickness weights of the wetland water-table average and their
     // sums (IBIS_FLAG_CH4_BANDS: from ch4b_z_wt_ref as ch4_wtop from z_wt_ref)
     R ch4b_wtop[3][6];
@@ -95,6 +108,12 @@ struct UniformQ {
     __device__ __forceinline__ R rwood(int j) const { return P.rwood_s[j]; }
     __device__ __forceinline__ R rroot(int j) const { return P.rroot_s[j]; }
     __device__ __forceinline__ R keep(int j) const { return P.keep[j]; }
+    // the pairs of the FP32 step: st 0 upper, 1 lower; j an even PFT
+    __device__ __forceinline__ ParPair coefm2(int st) const { return P.cm2[st]; }
+    __device__ __forceinline__ ParPair vmaxl2() const { return P.vml2; }
+    __device__ __forceinline__ ParPair rroot2(int j) const { return P.rroot2[j / 2]; }
+    __device__ __forceinline__ ParPair rwood2(int j) const { return P.rwood2[j / 2]; }
+    __device__ __forceinline__ ParPair keep2(int j) const { return P.keep2[j / 2]; }
 };
 
 // One parameter record for every cell, in the kernels that carry the IBIS 3.0
@@ -127,6 +146,18 @@ struct RunQ {
     __device__ __forceinline__ R rwood(int) const { return rwood_; }
     __device__ __forceinline__ R rroot(int) const { return rroot_; }
     __device__ __forceinline__ R keep(int) const { return keep_; }
+    static __device__ __forceinline__ ParPair pair(float a, float b) {
+        ParPair p;
+        asm("mov.b64 %0, {%1, %2};" : "=l"(p.v) : "f"(a), "f"(b));
+        return p;
+    }
+    __device__ __forceinline__ ParPair coefm2(int st) const {
+        return st ? pair(coefm_[2], coefm_[4]) : pair(coefm_[0], coefm_[1]);
+    }
+    __device__ __forceinline__ ParPair vmaxl2() const { return pair(vmax_[8], vmax_[11]); }
+    __device__ __forceinline__ ParPair rroot2(int) const { return pair(rroot_, rroot_); }
+    __device__ __forceinline__ ParPair rwood2(int) const { return pair(rwood_, rwood_); }
+    __device__ __forceinline__ ParPair keep2(int) const { return pair(keep_, keep_); }
 };
 
 // One run's parameters in the kernels that carry the IBIS 3.0 extensions (the

@@ -39,7 +39,7 @@ extern "C" int ibis_step_f32(float* prog, const float* stat, const float* forc, 
                              int ld, int nstep, const IbisParams* params, int* status, void* stream) {
     // without a device, the step's own checks and its launch report what is wrong
     int sms = 0;
-    const int cfg = ncell > 0 && device_sms(sms) ? ibis::auto_config(ncell, nstep, sms) : ibis::kDefaultFused;
+    const int cfg = params && device_sms(sms) ? ibis::auto_config(params->flags, ncell, sms) : ibis::kDefaultFused;
     return ibis::hourly_step<float>(prog, stat, forc, diag, acc, ncell, ld, nstep, params, status, stream, nullptr,
                                     cfg);
 }
@@ -223,7 +223,7 @@ extern "C" int ibis_step_host_f32(float* prog, const float* stat, const float* h
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return -ENODEV;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) return -ENODEV;
-    const int cfg = config >= 0 ? config : ibis::auto_config(ncell, nstep, sms);
+    const int cfg = config >= 0 ? config : ibis::auto_config(params->flags, ncell, sms);
     if (group == 0) {
         // whole blocks per group: a partial block in every group would add
         // blocks to the batch, and a batch of whole waves would spill into one more
@@ -344,7 +344,7 @@ extern "C" int ibis_day_host_f32(float* prog, const float* stat, const float* ho
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return -ENODEV;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) return -ENODEV;
-    const int cfg = config >= 0 ? config : ibis::auto_config(ncell, nstep, sms);
+    const int cfg = config >= 0 ? config : ibis::auto_config(params->flags, ncell, sms);
     if (group == 0) {
         const int block = ibis::kConfigs[cfg].block;
         const double wave = (double)sms * block * ibis::kConfigs[cfg].minb;

@@ -7,8 +7,8 @@ namespace ibis {
 #define IBIS_INST(NT, SU, SL, CFG) \
     template cudaError_t run_config<float, NT, SU, SL, CFG, true>(IBIS_RUN_ARGS(float));
 IBIS_INST(9, false, false, 0)
-IBIS_INST(9, false, false, 4)
 IBIS_INST(9, false, false, 6)
 IBIS_INST(9, false, false, 8)
+IBIS_INST(9, true, true, 0)
 #undef IBIS_INST
 }  // namespace ibis

@@ -6,9 +6,9 @@
 namespace ibis {
 #define IBIS_INST(NT, SU, SL, CFG) \
     template cudaError_t run_config<float, NT, SU, SL, CFG, true>(IBIS_RUN_ARGS(float));
-IBIS_INST(9, true, true, 0)
-IBIS_INST(9, true, true, 4)
 IBIS_INST(9, true, true, 6)
 IBIS_INST(9, true, true, 8)
+IBIS_INST(9, true, false, 0)
+IBIS_INST(9, true, false, 6)
 #undef IBIS_INST
 }  // namespace ibis

@@ -6,9 +6,9 @@
 namespace ibis {
 #define IBIS_INST(NT, SU, SL, CFG) \
     template cudaError_t run_config<float, NT, SU, SL, CFG, true>(IBIS_RUN_ARGS(float));
-IBIS_INST(9, false, true, 4)
-IBIS_INST(9, false, true, 8)
 IBIS_INST(6, false, false, 0)
-IBIS_INST(6, false, false, 4)
+IBIS_INST(6, false, false, 6)
+IBIS_INST(6, false, false, 8)
+IBIS_INST(6, true, true, 0)
 #undef IBIS_INST
 }  // namespace ibis

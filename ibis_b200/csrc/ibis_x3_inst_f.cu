@@ -6,9 +6,9 @@
 namespace ibis {
 #define IBIS_INST(NT, SU, SL, CFG) \
     template cudaError_t run_config<float, NT, SU, SL, CFG, true>(IBIS_RUN_ARGS(float));
-IBIS_INST(6, true, true, 6)
-IBIS_INST(6, true, true, 8)
-IBIS_INST(6, true, false, 0)
-IBIS_INST(6, true, false, 4)
+IBIS_INST(6, true, false, 8)
+IBIS_INST(6, false, true, 0)
+IBIS_INST(6, false, true, 6)
+IBIS_INST(6, false, true, 8)
 #undef IBIS_INST
 }  // namespace ibis

@@ -3,7 +3,7 @@ each can go wrong: batches of less than a warp, of partial warps and blocks, on 
 sides of the sizes where the choice changes.
 
 A column's step does not depend on its batch, so each batch is compared with one run
-of configuration 0 over the most columns: the same step code compiled for another
+of configuration 6 over the most columns: the same step code compiled for another
 block size, which may contract other multiply-adds; temperatures then differ by a few
 float32 ulps an hour (5e-5 K each), bounded here by 5 mK over at most five hours (the
 bound the FP32 step is held to against float64 for one hour), contents and sums by
@@ -15,7 +15,7 @@ import torch
 
 from ibis_b200 import ensemble as E
 from ibis_b200 import synth
-from ibis_b200.columns import AUTO_FUSED, AUTO_SMALL, Columns
+from ibis_b200.columns import AUTO_FUSED, AUTO_LARGE, Columns
 from ibis_b200.params import FLAG_SUNSHADE_L, FLAG_SUNSHADE_U, FLAG_VMAX_MIX
 
 pytestmark = pytest.mark.gpu
@@ -29,7 +29,7 @@ def reference(cuda_lib):
     wl = synth.make_workload(MOST, HOURS, seed=77, edge_cases=True)
     out = {}
     for nstep in (1, HOURS):
-        cols = Columns.from_host(wl.prog, wl.stat, acc=True, mode=0)
+        cols = Columns.from_host(wl.prog, wl.stat, acc=True, mode=6)
         cols.run(cols.forcing(wl.forc, 0, nstep), wl.params)
         out[nstep] = (cols.prog_host(), cols.acc_host())
     return wl, out
@@ -42,7 +42,7 @@ def _head(wl, n):
 
 @pytest.mark.parametrize("diag", [False, True])
 @pytest.mark.parametrize("nstep", [1, HOURS])
-@pytest.mark.parametrize("ncell", [1, 31, 33, 127, 225, 4735, 4737, 18945, MOST])
+@pytest.mark.parametrize("ncell", [1, 31, 33, 127, 129, 255, 18945, MOST])
 def test_batches_of_every_shape_step_as_one(reference, ncell, nstep, diag):
     wl, out = reference
     prog, stat, forc = _head(wl, ncell)
@@ -66,13 +66,32 @@ def test_batches_of_every_shape_step_as_one(reference, ncell, nstep, diag):
         assert float(np.abs(a[k] - w[:ncell]).max()) <= 1e-3 * scale, k
 
 
-def test_the_choice_follows_the_batch(cuda_lib):
+def test_the_choice_follows_the_batch_and_the_canopy(cuda_lib):
     sms = torch.cuda.get_device_properties(0).multi_processor_count
-    cfg = lambda n, h: Columns(n, acc=False).launch_config(h)
-    assert cfg(1, 24) == cfg(32 * sms, 24) == cfg(32 * sms, 1) == AUTO_SMALL
-    assert cfg(32 * sms + 1, 1) == cfg(32 * sms + 1, 24) == cfg(128 * sms, 24) == 0
-    assert cfg(128 * sms + 1, 24) == cfg(224 * sms, 24) == AUTO_FUSED     # one wave of either
-    assert cfg(224 * sms + 1, 24) == cfg(256 * sms, 24) == 0              # one wave of 256 threads, two of 224
+    cfg = lambda n, flags: Columns(n, acc=False).launch_config(24, flags)
+    assert cfg(1, 0) == cfg(128 * sms + 1, 0) == AUTO_FUSED == 0
+    for flags in (FLAG_SUNSHADE_U, FLAG_SUNSHADE_L, FLAG_VMAX_MIX):
+        assert cfg(128 * sms, flags) == AUTO_FUSED and cfg(128 * sms + 1, flags) == AUTO_LARGE == 6
+
+
+@pytest.mark.parametrize("flags", [FLAG_SUNSHADE_U, FLAG_SUNSHADE_U | FLAG_SUNSHADE_L | FLAG_VMAX_MIX])
+def test_large_records_step_as_small_ones(cuda_lib, flags):
+    """The canopy variants on both sides of their choice (18,944 and 18,945 columns on
+    148 SMs): the first 500 columns of each batch, and of the other configuration."""
+    wl = synth.make_workload(18945, 3, seed=21)
+    wl.params.flags |= flags
+    got = []
+    for n, mode in ((500, "fused"), (18944, "fused"), (18945, "fused"), (500, 6), (500, 0)):
+        prog, stat, forc = _head(wl, n)
+        cols = Columns.from_host(prog, stat, acc=True, mode=mode)
+        cols.run(cols.forcing(forc), wl.params)
+        got.append((cols.prog_host(), cols.acc_host()))
+    for p, a in got[1:]:
+        for k in ("tsoi", "tg", "tu", "tl", "ti"):
+            np.testing.assert_allclose(p[k][:500], got[0][0][k], rtol=0, atol=5e-3, err_msg=k)
+        for k in ("aynpp", "aygpptot", "adaet", "afsena", "ch4"):
+            w = got[0][1][k]
+            assert float(np.abs(a[k][:500] - w).max()) <= 1e-3 * float(np.abs(w).max()), k
 
 
 @pytest.mark.parametrize("daily", [False, True])
