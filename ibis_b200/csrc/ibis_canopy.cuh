@@ -509,7 +509,7 @@ struct TvOut {
 struct Sat64 { double q, dq; };
 
 // Saturation humidity and its capped derivative at the blended temperature.
-__device__ __forceinline__ Sat64 sat64(double t, double ps) {
+static __device__ __noinline__ Sat64 sat64(double t, double ps) {
     Sat64 s;
     double e = esat(t);
     s.q = qsat(e, ps);

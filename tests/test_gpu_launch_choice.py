@@ -111,3 +111,20 @@ def test_every_ensemble_block_runs_with_every_switch(cuda_lib, daily):
         assert not any(ens.nonfinite()[:2])
         out.append((ens.prog.clone(), ens.acc.clone()))
     assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
+
+
+@pytest.mark.parametrize("flags", [0, FLAG_SUNSHADE_U, FLAG_SUNSHADE_U | FLAG_SUNSHADE_L])
+@pytest.mark.parametrize("ncell", [1, 33, 1500])
+def test_the_plain_float64_kernel_gives_the_full_ones_bits(cuda_lib, ncell, flags):
+    """Without diagnostics and IBIS 3.0 switches float64 columns run a kernel that has
+    neither: operation for operation the same step, so not a bit may differ."""
+    wl = synth.make_workload(ncell, 4, seed=5, edge_cases=ncell > 1000)
+    wl.params.flags |= flags
+    out = []
+    for diag in (False, True):
+        cols = Columns.from_host(wl.prog, wl.stat, acc=True, diag=diag, dtype=torch.float64)
+        cols.run(cols.forcing(wl.forc), wl.params)
+        out.append((cols.prog_host(), cols.acc_host()))
+    for a, b in zip(*out):
+        for k in a:
+            assert np.array_equal(a[k], b[k], equal_nan=True), k
