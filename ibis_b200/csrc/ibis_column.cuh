@@ -21,16 +21,26 @@ constexpr int NL = 6;   // soil layers
 constexpr int NB = 3;   // bedrock layers
 constexpr int NS = 3;   // snow layers
 
+// A column's prognostic state.  The FP32 kernels hold it in shared memory, a thread's
+// words together: pairs that are used together start on 64-bit words, so that one access
+// moves both (8,752 -> 8,536 instructions of the kernel), and a thread takes 37 of those
+// words, odd, which spreads a warp's over the banks.
 template <typename R>
-struct Col {
-    R tsoi[NL], wsoi[NL], wisoi[NL], tg, wpud, wipud, tsoi_deep[NB];
-    R fi, tsno[NS], hsno[NS], ti, tlsub;
-    R tu, ts, tl, t12, t34, q12, q34;
-    R wliqu, wliqs, wliql, wsnou, wsnos, wsnol;
-    R ci_u[2], gs_u[2], cs_u[2], ci_l[3], gs_l[3], cs_l[3];
-    R a10su, a10du, a10sl, a10dl;
-    R firefac, nytimes, nfirestep, sdry, nfirestep_vpd, sdry_vpd;
+struct alignas(8) Col {
+    R tsoi[NL], wsoi[NL], wisoi[NL];
+    R tu, ts, t12, t34, q12, q34, tl, tg;
+    R ci_u[2], gs_u[2], cs_u[2];
+    R wliqu, wsnou, wliqs, wsnos, wliql, wsnol;
+    R a10su, a10sl, a10du, a10dl;
+    R wpud, wipud;
+    R fi, ti;
+    R tsno[NS], tlsub;
+    R hsno[NS], firefac;
+    R ci_l[3], nytimes, gs_l[3], nfirestep, cs_l[3], sdry;
+    R tsoi_deep[NB], nfirestep_vpd;
+    R sdry_vpd, unused[3];
 };
+static_assert(sizeof(Col<float>) == 37 * 8, "an odd number of 64-bit words");
 
 template <typename R>
 struct Forc {

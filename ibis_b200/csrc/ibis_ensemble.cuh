@@ -173,17 +173,16 @@ template <bool X3>
 using RunSource = std::conditional_t<X3, RunQ3<float>, RunQ<float>>;
 
 // The thread's record of the hour (HourScratch): after the block's column states and
-// run parameters (71 and 33 words a thread, so it starts on a 64-bit word)
+// run parameters (of whole warps, so it starts on a 128-bit word)
 template <bool SUN, bool X3>
 __device__ __forceinline__ HourScratch<SUN, X3>& ens_hour(unsigned char* smem) {
-    static_assert((sizeof(Col<float>) + sizeof(RunQ<float>)) % 8 == 0, "64-bit words");
     return reinterpret_cast<HourScratch<SUN, X3>*>(
         smem + blockDim.x * (sizeof(Col<float>) + sizeof(RunQ<float>)))[threadIdx.x];
 }
 
 template <int NT, bool SU, bool SL, bool DAILY, bool X3>
 __global__ void __launch_bounds__(256, 1) ensemble_kernel(const EnsArgs e, const DevParams<float> P) {
-    extern __shared__ unsigned char smem_raw[];
+    extern __shared__ __align__(16) unsigned char smem_raw[];
     Col<float>& c = reinterpret_cast<Col<float>*>(smem_raw)[threadIdx.x];
     RunSource<X3>& q =
         reinterpret_cast<RunSource<X3>*>(smem_raw + blockDim.x * sizeof(Col<float>))[threadIdx.x];
@@ -265,13 +264,13 @@ __global__ void __launch_bounds__(128, 2) ensemble_hour_kernel(const EnsArgs e, 
     const long long first = __ldg(e.run_forc + r);
     const int pos = e.run_pos ? __ldg(e.run_pos + r) : 0;
     if (!run_ok(e, r, site, nstep, first, pos)) return;
-    extern __shared__ unsigned char smem_raw[];
+    extern __shared__ __align__(16) unsigned char smem_raw[];
     Col<float>& c = reinterpret_cast<Col<float>*>(smem_raw)[threadIdx.x];
     RunSource<X3>& q =
         reinterpret_cast<RunSource<X3>*>(smem_raw + blockDim.x * sizeof(Col<float>))[threadIdx.x];
     load_col(c, e.prog + r, e.ld_run);
     load_run_params(q, e.run_params + r, e.ld_run, P);
-    const Stat<float> S{e.stat + site, e.ld_site};
+    Stat<float> S{e.stat + site, e.ld_site};
     const Acc<float> A{e.acc ? e.acc + r : nullptr, e.ld_run, (P.flags & IBIS_FLAG_KAHAN) != 0, hour + 1 == nstep};
     const Forc<float> F = load_forc_record(e.forc + (size_t)(first + hour) * IBIS_FORC_COUNT);
     column_step<float, NT, SU, SL>(c, ens_hour<SU || SL, X3>(smem_raw), F, S, Diag<float, false>{nullptr, 0}, A, P, q);
@@ -293,8 +292,8 @@ size_t ens_smem(int block, bool daily = false) {
 }
 
 // The largest block (whole warps, at most `block`) whose shared memory an SM holds:
-// 256 threads except with the sunlit/shaded canopies, the IBIS 3.0 switches and daily
-// weather together.
+// 256 threads except with the sunlit/shaded canopies, the IBIS 3.0 switches or daily
+// weather.
 template <bool SUN, bool X3>
 int ens_block(int block, bool daily) {
     while (block > 32 && ens_smem<SUN, X3>(block, daily) > 227 * 1024) block -= 32;

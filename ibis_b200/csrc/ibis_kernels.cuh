@@ -126,7 +126,7 @@ __device__ __forceinline__ Forc<R> load_forc(const R* __restrict__ f, int ld) {
 // stored after the last, so the hourly read-modify-writes stay on chip.  All loads
 // are issued before the stores, so a launch waits out one memory latency.
 template <bool TO_SMEM>
-__device__ __forceinline__ void acc_move(float* __restrict__ g, int ld, float2* __restrict__ chip, int sld,
+__device__ __forceinline__ void acc_move(float* __restrict__ g, int ld, float4* __restrict__ chip, int sld,
                                          unsigned flags) {
     const bool sums = (flags & IBIS_FLAG_ACC) != 0, ch4 = (flags & IBIS_FLAG_CH4) != 0;
     const bool kahan = (flags & IBIS_FLAG_KAHAN) != 0;
@@ -141,22 +141,19 @@ __device__ __forceinline__ void acc_move(float* __restrict__ g, int ld, float2* 
             if constexpr (TO_SMEM) {
                 v[c][s] = use ? *p : 0.0f;
             } else if (use) {
-                const float2 w = chip[(c * kAccPairs + s / 2) * sld];
-                *p = s & 1 ? w.y : w.x;
+                *p = reinterpret_cast<const float*>(chip + (s / 2) * sld)[2 * c + (s & 1)];
             }
         }
     }
     if constexpr (TO_SMEM) {
 #pragma unroll
-        for (int c = 0; c < 2; ++c)
-#pragma unroll
-            for (int j = 0; j < kAccPairs; ++j)
-                chip[(c * kAccPairs + j) * sld] = make_float2(v[c][2 * j], v[c][2 * j + 1]);
+        for (int j = 0; j < kAccPairs; ++j)
+            chip[j * sld] = make_float4(v[0][2 * j], v[0][2 * j + 1], v[1][2 * j], v[1][2 * j + 1]);
     }
 }
 
 // Bytes of shared memory per thread the on-chip accumulators take
-constexpr size_t kAccChipBytes = 2 * kAccPairs * sizeof(float2);
+constexpr size_t kAccChipBytes = kAccPairs * sizeof(float4);
 
 // Whether a fused configuration keeps its accumulators in shared memory: with the
 // column state and the hour's record, MINB resident blocks must fit the SM's 228 KB
@@ -179,7 +176,7 @@ struct BlockSmem {
     static constexpr size_t acc_off = (size_t)BLOCK * sizeof(Col<R>);
     static constexpr size_t hour_off = acc_off + (ACC ? (size_t)BLOCK * kAccChipBytes : 0);
     static constexpr size_t total = on ? hour_off + (size_t)BLOCK * sizeof(Hour) : 0;
-    static_assert(acc_off % 8 == 0 && hour_off % 8 == 0, "64-bit words");
+    static_assert(acc_off % 16 == 0 && hour_off % 8 == 0, "128- and 64-bit words");
     static __device__ __forceinline__ Hour& hour(unsigned char* smem) {
         return reinterpret_cast<Hour*>(smem + hour_off)[threadIdx.x];
     }
@@ -223,7 +220,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) hourly_step_kernel(R* __restrict_
     if (threadIdx.x >= nbar) return;
     const bool live = (int)threadIdx.x < nlive;
     const int i = live ? i0 + (int)threadIdx.x : ncell - 1;
-    extern __shared__ unsigned char smem_raw[];
+    extern __shared__ __align__(16) unsigned char smem_raw[];
     Col<R> creg;
     Col<R>* cp;
     if constexpr (StateInSmem<R>::value) cp = reinterpret_cast<Col<R>*>(smem_raw) + threadIdx.x;
@@ -237,7 +234,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) hourly_step_kernel(R* __restrict_
     Acc<R, kAccSmem ? BLOCK : 0> A{acc ? acc + i : nullptr, ld, (P.flags & IBIS_FLAG_KAHAN) != 0};
     A.live = live;
     if constexpr (kAccSmem) {
-        A.chip = reinterpret_cast<float2*>(smem_raw + SM::acc_off) + threadIdx.x;
+        A.on_chip(reinterpret_cast<float4*>(smem_raw + SM::acc_off) + threadIdx.x);
         if (acc) acc_move<true>(acc + i, ld, A.chip, BLOCK, P.flags);
     }
 #pragma unroll 1
@@ -404,7 +401,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) hourly_step_staged_kernel(
     Stat<R> S{stat + i, ld};
     const Diag<R, false> D{nullptr, ld};
     Acc<R, BLOCK> A{acc ? acc + i : nullptr, ld, (P.flags & IBIS_FLAG_KAHAN) != 0};
-    A.chip = reinterpret_cast<float2*>(smem_raw + SM::Block::acc_off) + threadIdx.x;
+    A.on_chip(reinterpret_cast<float4*>(smem_raw + SM::Block::acc_off) + threadIdx.x);
     if (acc) acc_move<true>(acc + i, ld, A.chip, BLOCK, P.flags);
 #pragma unroll 1
     for (int s = 0; s < nstep; ++s) {
@@ -448,7 +445,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) surface_kernel(R* __restrict__ pr
                                                                     const DevParams<R> P) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= ncell) return;
-    extern __shared__ unsigned char smem_raw[];
+    extern __shared__ __align__(16) unsigned char smem_raw[];
     Col<R> creg;
     Col<R>* cp;
     if constexpr (StateInSmem<R>::value) cp = reinterpret_cast<Col<R>*>(smem_raw) + threadIdx.x;
@@ -474,7 +471,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) ground_kernel(R* __restrict__ pro
                                                                    int* __restrict__ status) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= ncell) return;
-    extern __shared__ unsigned char smem_raw[];
+    extern __shared__ __align__(16) unsigned char smem_raw[];
     Col<R> creg;
     Col<R>* cp;
     if constexpr (StateInSmem<R>::value) cp = reinterpret_cast<Col<R>*>(smem_raw) + threadIdx.x;

@@ -39,18 +39,20 @@ __host__ __device__ constexpr int acc_slot(int plane) {
 
 // Accumulator view of one cell.  In the global form (SLD = 0) ``base`` addresses
 // every plane with leading dimension ``ld`` and the compensation term of plane p is
-// plane p + IBIS_ACC_COUNT.  In the on-chip form (SLD = the block size) ``chip``
-// holds pair j of the slots above at chip[j * SLD] and its compensation terms at
-// chip[(kAccPairs + j) * SLD]; ``base`` is still the global buffer, for the planes
-// that have no slot.  ``live`` is false for a lane that repeats another's cell.
+// plane p + IBIS_ACC_COUNT.  In the on-chip form (SLD = the distance of a thread's
+// words) chip[j * SLD] holds pair j of the slots above and its two compensation
+// terms, zero without compensation, one 128-bit access each way; ``base`` is still the
+// global buffer, for the planes that have no slot.  ``live`` is false for a lane that repeats another's cell.
 template <typename R, int SLD = 0>
 struct Acc {
     R* __restrict__ base;  // nullptr: no accumulators
     int ld;
     bool kahan;
     bool last = true;      // the launch's last hour for this cell: keep the end-of-hour values
-    float2* __restrict__ chip = nullptr;
+    float4* __restrict__ chip = nullptr;
     bool live = true;
+    float keep = 0.0f;     // on chip: 1 with compensation, 0 without
+    __device__ __forceinline__ void on_chip(float4* p) { chip = p; keep = kahan ? 1.0f : 0.0f; }
     __device__ __forceinline__ R& at(int plane) const { return base[(size_t)plane * ld]; }
     __device__ __forceinline__ R& comp(int plane) const { return base[(size_t)(plane + IBIS_ACC_COUNT) * ld]; }
     __device__ __forceinline__ void add(int plane, R x) const {
@@ -73,13 +75,9 @@ struct Acc {
     __device__ __forceinline__ F2 add2(int p0, int p1, const F2& x) const {
         F2 s, cc(0.0f);
         if constexpr (SLD > 0) {
-            const int j = acc_slot(p0) >> 1;
-            const float2 v = chip[j * SLD];
+            const float4 v = chip[(acc_slot(p0) >> 1) * SLD];
             s = F2(v.x, v.y);
-            if (kahan) {
-                const float2 w = chip[(kAccPairs + j) * SLD];
-                cc = F2(w.x, w.y);
-            }
+            cc = F2(v.z, v.w);
         } else {
             s = F2(at(p0), p1 < 0 ? 0.0f : at(p1));
             if (kahan) cc = F2(comp(p0), p1 < 0 ? 0.0f : comp(p1));
@@ -89,9 +87,8 @@ struct Acc {
         const F2 d = t - s;
         const F2 cn = d - y;
         if constexpr (SLD > 0) {
-            const int j = acc_slot(p0) >> 1;
-            chip[j * SLD] = make_float2(t.lo(), t.hi());
-            if (kahan) chip[(kAccPairs + j) * SLD] = make_float2(cn.lo(), cn.hi());
+            const F2 ck = cn * keep;
+            chip[(acc_slot(p0) >> 1) * SLD] = make_float4(t.lo(), t.hi(), ck.lo(), ck.hi());
         } else if (live) {
             at(p0) = t.lo();
             if (p1 >= 0) at(p1) = t.hi();

@@ -545,7 +545,7 @@ __device__ __forceinline__ void ground_phase(Col<R>& c, const Forc<R>& F, const 
 // One full hourly step of a column in one kernel (y: the FP32 step's record of the hour
 // in shared memory, HourScratch; unused in float64).
 template <typename R, int NT, bool SUN_U, bool SUN_L, typename Y, typename Q, typename DD, int SLD>
-__device__ __forceinline__ void column_step(Col<R>& c, Y& y, const Forc<R>& F, const Stat<R>& S, const DD& D,
+__device__ __forceinline__ void column_step(Col<R>& c, Y& y, const Forc<R>& F, Stat<R>& S, const DD& D,
                                             const Acc<R, SLD>& Ac, const DevParams<R>& P, const Q& q) {
     Mid<R> M;
     if constexpr (sizeof(R) == 4) {
