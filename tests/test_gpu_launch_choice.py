@@ -128,3 +128,29 @@ def test_the_plain_float64_kernel_gives_the_full_ones_bits(cuda_lib, ncell, flag
     for a, b in zip(*out):
         for k in a:
             assert np.array_equal(a[k], b[k], equal_nan=True), k
+
+
+@pytest.mark.parametrize("block", [64, 160, 256])
+def test_a_run_does_not_depend_on_its_block_or_order(cuda_lib, block):
+    """Runs of 0 to 7 hours, in the queue in no order: warps of a block that finish,
+    draw and run out of items at different hours, whole items of runs without an hour,
+    a year that ends inside the records.  Bit for bit as in blocks of one warp."""
+    spec = E.make_ensemble(7, 47, site_hours=np.full(7, 7), seed=9)
+    ens = E.Ensemble(spec, year_steps=5)
+    gen = torch.Generator().manual_seed(4)
+    hours = torch.randint(0, 8, (ens.nrun,), generator=gen, dtype=torch.int32)
+    hours[64:128] = 0
+    ens.run_nstep.copy_(hours)
+    out = []
+    for b, order in ((32, torch.arange(ens.nrun)), (block, torch.arange(ens.nrun)),
+                     (block, torch.randperm(ens.nrun, generator=gen))):
+        ens.order.copy_(order.to(torch.int32))
+        ens.reset()
+        ens.run(block=b)
+        torch.cuda.synchronize()
+        assert not any(ens.nonfinite()[:2])
+        out.append((ens.prog[:, :ens.nrun].clone(), ens.acc[:, :ens.nrun].clone(), ens.yearly.clone()))
+    assert bool((out[0][1][:, 64:128] == 0).all())
+    assert bool((out[0][2] != 0).any())
+    for got in out[1:]:
+        assert all(torch.equal(x, y) for x, y in zip(got, out[0]))
