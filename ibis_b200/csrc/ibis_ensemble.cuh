@@ -261,6 +261,7 @@ __global__ void __launch_bounds__(256, 1) ensemble_kernel(const EnsArgs e, const
                 load_col(c, e.prog + r, e.ld_run);
                 load_run_params(q, e.run_params + r, e.ld_run, P);
                 S.base = e.stat + site;
+                column_begin<float>(hour, S, P, q);
                 if (e.acc) {
                     A.base = e.acc + r;
                     acc_move<true>(A.base, e.ld_run, A.chip, 1, P.flags);
@@ -329,6 +330,7 @@ __global__ void __launch_bounds__(128, 2) ensemble_hour_kernel(const EnsArgs e, 
     Stat<float> S{e.stat + site, e.ld_site};
     const Acc<float> A{e.acc ? e.acc + r : nullptr, e.ld_run, (P.flags & IBIS_FLAG_KAHAN) != 0, hour + 1 == nstep};
     const Forc<float> F = load_forc_record(e.forc + (size_t)(first + hour) * IBIS_FORC_COUNT);
+    column_begin<float>(ens_hour<SU || SL, X3>(smem_raw), S, P, q);
     column_step<float, NT, SU, SL>(c, ens_hour<SU || SL, X3>(smem_raw), F, S, Diag<float, false>{nullptr, 0}, A, P, q);
     if (e.yearly && (pos + hour + 1) % e.year_steps == 0) {
         const int y = (pos + hour + 1) / e.year_steps - 1;

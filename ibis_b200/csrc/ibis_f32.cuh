@@ -625,11 +625,13 @@ struct HourExtra {};
 template <>
 struct alignas(8) HourExtra<true, false> { Sun4 su, sl; };
 // with the IBIS 3.0 switches also the big leaves' nominal vmax, slopes and light
-// factors (C4 grass last) and the capacity integrals (upper, lower)
+// factors (C4 grass last), the capacity integrals (upper, lower) and the upper and shrub
+// leaves' area per capacity (negative: shares by area)
+struct alignas(8) Leaves3 { F2 vnl, cmu, cml, jfu, jfl, cap; float vn4, cm4, jf4, rcap[3]; };
 template <>
-struct alignas(8) HourExtra<false, true> { F2 vnl, cmu, cml, jfu, jfl, cap; float vn4, cm4, jf4, unused; };
+struct alignas(8) HourExtra<false, true> : Leaves3 {};
 template <>
-struct alignas(8) HourExtra<true, true> { Sun4 su, sl; F2 vnl, cmu, cml, jfu, jfl, cap; float vn4, cm4, jf4, unused; };
+struct alignas(8) HourExtra<true, true> : Leaves3 { Sun4 su, sl; };
 
 // Pairs: (upper leaves, upper stems) `_us`, (lower canopy, ground) `_lg`, (ground, snow) `_gi`
 struct alignas(8) TvHour {
@@ -930,7 +932,21 @@ __device__ __forceinline__ void turvap32(double (&W)[9], TvResult& o, const Col3
 // conductivity, and the stress of every layer before the root profile's weights.
 struct SoilHour {
     float q1, q2, q3, q4, consoi0, zw[NL], stresstu, stresstl;
+    const float* rcap;   // Leaves3 (IBIS 3.0 kernels)
 };
+
+// The leaves' area per capacity of Leaves3, with gpp_split_by_capacity
+template <typename Q>
+__device__ __forceinline__ void area_per_capacity(float (&rcap)[3], const Stat32& S, const Q& q) {
+    float twm, tfs;
+    bool on;
+    capacity_group(kBroadleafPfts, S, q, twm, tfs, on);
+    rcap[0] = on ? tfs / twm : -1.0f;
+    capacity_group(kConiferPfts, S, q, twm, tfs, on);
+    rcap[1] = on ? tfs / twm : -1.0f;
+    capacity_group(kShrubPfts, S, q, twm, tfs, on);
+    rcap[2] = on ? tfs / twm : -1.0f;
+}
 
 // setsoi's conductivity of layer k (soil_physics.py:37-140): the dry solids'
 // times 56^liquid 224^ice, one power of two
@@ -966,7 +982,28 @@ __device__ __forceinline__ void soil_stress32(SoilHour& G, const Col32& c, const
     G.stresstu = tot.hi();
 }
 
-// Steps 1-9 of timestep_body (see surface_phase, ibis_step.cuh); y: the hour's record
+// What the record of the hour holds of the parameters and the static planes alone: the
+// big leaves' nominal capacities with the IBIS 3.0 switches (stomata.py:592-660).  No hour
+// changes them, so a launch forms them once, before its hours: 33,001
+// columns x 6 hours of the release formulation 231 -> 184 us.  The F77 step
+// has too little of the kind (the same of its leaf-area shares made it 4% slower).
+template <typename Y, typename Q>
+__device__ __forceinline__ void column_begin32(Y& y, const Stat32& S, const Par32& P, const Q& q) {
+    if constexpr (Q::x3) {
+        float vu[2], ju[2], mu[2], vl[3], jl[3], ml[3];
+        bool jon = false;
+        big_leaves<float, false>(vu, ju, mu, jon, S, P, q);
+        big_leaves<float, true>(vl, jl, ml, jon, S, P, q);
+        y.X.vnu = F2(vu[0], vu[1]); y.cmu = F2(mu[0], mu[1]); y.jfu = F2(ju[0], ju[1]);
+        y.vnl = F2(vl[0], vl[1]); y.cml = F2(ml[0], ml[1]); y.jfl = F2(jl[0], jl[1]);
+        y.vn4 = vl[2]; y.cm4 = ml[2]; y.jf4 = jl[2];
+        y.cap = F2(capacity_integral(S(IBIS_STAT_LAI, 1), P.cap_kn), capacity_integral(S(IBIS_STAT_LAI, 0), P.cap_kn));
+        if (P.flags & IBIS_FLAG_GPP_CAPACITY) area_per_capacity(y.rcap, S, q);
+    }
+}
+
+// Steps 1-9 of timestep_body (see surface_phase, ibis_step.cuh); y: the hour's record,
+// begun by column_begin32,
 // in shared memory
 template <bool SUN_U, bool SUN_L, typename Y, typename Q, typename D32>
 __device__ __forceinline__ void surface_phase32(Col32& c, Y& y, const Forc32& F, const Stat32& S, const D32& D,
@@ -1013,20 +1050,9 @@ __device__ __forceinline__ void surface_phase32(Col32& c, Y& y, const Forc32& F,
             const float r = lai0 > 0.0f ? 1.0f / mx(lai0, 1.0e-6f) : 0.0f;
             y.sl = Sun4{F2(ss.psun, ss.psha) * r, F2(ss.vsun, ss.vsha) * r};
         }
-        // the big leaves' nominal capacities (stomata.py:592-660)
-        if constexpr (Q::x3) {
-            float vu[2], ju[2], mu[2], vl[3], jl[3], ml[3];
-            bool jon = false;
-            big_leaves<float, false>(vu, ju, mu, jon, S, P, q);
-            big_leaves<float, true>(vl, jl, ml, jon, S, P, q);
-            X.vnu = F2(vu[0], vu[1]); y.cmu = F2(mu[0], mu[1]); y.jfu = F2(ju[0], ju[1]);
-            y.vnl = F2(vl[0], vl[1]); y.cml = F2(ml[0], ml[1]); y.jfl = F2(jl[0], jl[1]);
-            y.vn4 = vl[2]; y.cm4 = ml[2]; y.jf4 = jl[2];
-            y.cap = F2(capacity_integral(lai1, P.cap_kn), capacity_integral(lai0, P.cap_kn));
-        } else {
+        if constexpr (!Q::x3)
             X.vnu = F2(S(IBIS_STAT_EXIST, 0) > 0.5f ? q.vmax(0) : (S(IBIS_STAT_EXIST, 2) > 0.5f ? q.vmax(2) : q.vmax(4)),
                        S(IBIS_STAT_EXIST, 3) > 0.5f ? q.vmax(3) : q.vmax(5));
-        }
         if (D.on()) radiation_diagnostics(D, Rd);
 
         // ---- 4-5. precipitation cascade and wet fractions after it (loops.py:359-389)
@@ -1772,13 +1798,11 @@ __device__ __forceinline__ void ground_phase32(Col32& c, const Forc32& F, Stat32
         bool by_cap[3] = {false, false, false};
         if constexpr (Q::x3) {
             if (P.flags & IBIS_FLAG_GPP_CAPACITY) {
-                float twm, tfs;
-                capacity_group(kBroadleafPfts, S, q, twm, tfs, by_cap[0]);
-                rcap[0] = tfs / twm;
-                capacity_group(kConiferPfts, S, q, twm, tfs, by_cap[1]);
-                rcap[1] = tfs / twm;
-                capacity_group(kShrubPfts, S, q, twm, tfs, by_cap[2]);
-                rcap[2] = tfs / twm;
+#pragma unroll
+                for (int g = 0; g < 3; ++g) {
+                    by_cap[g] = G.rcap[g] >= 0.0f;
+                    rcap[g] = G.rcap[g];
+                }
             }
         }
         F2 npp(0.0f);

@@ -237,6 +237,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) hourly_step_kernel(R* __restrict_
         A.on_chip(reinterpret_cast<float4*>(smem_raw + SM::acc_off) + threadIdx.x);
         if (acc) acc_move<true>(acc + i, ld, A.chip, BLOCK, P.flags);
     }
+    column_begin<R>(SM::hour(smem_raw), S, P, uniform_source<R, X3>(P));
 #pragma unroll 1
     for (int s = 0; s < nstep; ++s) {
         align_warps<StateInSmem<R>::value && (BLOCK > 32)>(nbar);
@@ -403,6 +404,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) hourly_step_staged_kernel(
     Acc<R, BLOCK> A{acc ? acc + i : nullptr, ld, (P.flags & IBIS_FLAG_KAHAN) != 0};
     A.on_chip(reinterpret_cast<float4*>(smem_raw + SM::Block::acc_off) + threadIdx.x);
     if (acc) acc_move<true>(acc + i, ld, A.chip, BLOCK, P.flags);
+    column_begin<R>(SM::Block::hour(smem_raw), S, P, uniform_source<R, X3>(P));
 #pragma unroll 1
     for (int s = 0; s < nstep; ++s) {
         const unsigned parity = (unsigned)(s & 1);
@@ -457,6 +459,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) surface_kernel(R* __restrict__ pr
     Forc<R> F = load_forc(forc + i, ld);
     Mid<R> M;
     SoilHour G;      // formed again by the ground kernel
+    column_begin<R>(BlockSmem<R, SU || SL, X3, BLOCK, false>::hour(smem_raw), S, P, uniform_source<R, X3>(P));
     surface_phase32<SU, SL>(c, BlockSmem<R, SU || SL, X3, BLOCK, false>::hour(smem_raw), F, S, D, P,
                             uniform_source<R, X3>(P), M, G);
     mid_store(M, mid + i, ld);
@@ -486,6 +489,11 @@ __global__ void __launch_bounds__(BLOCK, MINB) ground_kernel(R* __restrict__ pro
     mid_load(M, mid + i, ld);
     SoilHour G;
     soil_hour32(G, c, F, S, P, uniform_source<R, X3>(P));
+    float rcap[3];
+    if constexpr (X3) {
+        if (P.flags & IBIS_FLAG_GPP_CAPACITY) area_per_capacity(rcap, S, uniform_source<R, X3>(P));
+        G.rcap = rcap;
+    }
     ground_phase32<NT>(c, F, S, D, A, P, uniform_source<R, X3>(P), M, G);
     R sum = store_col(c, prog + i, ld);
     if (status && !finite(sum)) {

@@ -542,6 +542,12 @@ __device__ __forceinline__ void ground_phase(Col<R>& c, const Forc<R>& F, const 
     }
 }
 
+// Once per launch, before a column's hours (FP32: column_begin32).
+template <typename R, typename Y, typename Q>
+__device__ __forceinline__ void column_begin(Y& y, const Stat<R>& S, const DevParams<R>& P, const Q& q) {
+    if constexpr (sizeof(R) == 4) column_begin32(y, S, P, q);
+}
+
 // One full hourly step of a column in one kernel (y: the FP32 step's record of the hour
 // in shared memory, HourScratch; unused in float64).
 template <typename R, int NT, bool SUN_U, bool SUN_L, typename Y, typename Q, typename DD, int SLD>
@@ -551,6 +557,7 @@ __device__ __forceinline__ void column_step(Col<R>& c, Y& y, const Forc<R>& F, S
     if constexpr (sizeof(R) == 4) {
         SoilHour G;
         surface_phase32<SUN_U, SUN_L>(c, y, F, S, D, P, q, M, G);
+        if constexpr (Q::x3) G.rcap = y.rcap;
         ground_phase32<NT>(c, F, S, D, Ac, P, q, M, G);
     } else {
         surface_phase<R, SUN_U, SUN_L>(c, F, S, D, P, q, M);

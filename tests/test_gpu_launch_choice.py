@@ -16,7 +16,7 @@ import torch
 from ibis_b200 import ensemble as E
 from ibis_b200 import synth
 from ibis_b200.columns import AUTO_FUSED, AUTO_LARGE, Columns
-from ibis_b200.params import FLAG_SUNSHADE_L, FLAG_SUNSHADE_U, FLAG_VMAX_MIX
+from ibis_b200.params import FLAG_COEFM_MIX, FLAG_GPP_CAPACITY, FLAG_SUNSHADE_L, FLAG_SUNSHADE_U, FLAG_VMAX_MIX
 
 pytestmark = pytest.mark.gpu
 
@@ -154,3 +154,23 @@ def test_a_run_does_not_depend_on_its_block_or_order(cuda_lib, block):
     assert bool((out[0][2] != 0).any())
     for got in out[1:]:
         assert all(torch.equal(x, y) for x, y in zip(got, out[0]))
+
+
+@pytest.mark.parametrize("mode", [0, 6, "split"])
+@pytest.mark.parametrize("flags", [FLAG_GPP_CAPACITY, FLAG_VMAX_MIX | FLAG_COEFM_MIX,
+                                   FLAG_GPP_CAPACITY | FLAG_VMAX_MIX | FLAG_SUNSHADE_U | FLAG_SUNSHADE_L])
+def test_a_launch_of_hours_is_as_many_launches_of_one(cuda_lib, flags, mode):
+    """What an IBIS 3.0 launch forms once of the parameters and static planes serves each
+    of its hours: the same kernel launched hour by hour forms it anew, to the same bits."""
+    wl = synth.make_workload(700, 4, seed=13, edge_cases=True)
+    wl.params.flags |= flags
+    out = []
+    for hours in (4, 1):
+        cols = Columns.from_host(wl.prog, wl.stat, acc=True, mode=mode)
+        for h in range(0, 4, hours):
+            cols.run(cols.forcing(wl.forc, h, h + hours), wl.params)
+        out.append((cols.prog_host(), cols.acc_host()))
+    for a, b in zip(*out):
+        for k in a:
+            if not k.endswith("_mean"):
+                assert np.array_equal(a[k], b[k], equal_nan=True), k
