@@ -56,9 +56,10 @@ struct Stat {
     __device__ __forceinline__ R operator()(int plane, int k) const { return __ldg(base + (size_t)(plane + k) * ld); }
     // Called once an hour: the compiler must take the view for a new one.  Otherwise it
     // hoists the loads of a hundred planes and their addresses out of the hour loop,
-    // where no register holds them: the FP32 kernel's local frame is 488 instead of
-    // 1,056 bytes without them, which eight warps read back every hour past an L1 that
-    // did not hold them (six hours of 95,333 columns 0.47 -> 0.44 ms).
+    // where no register holds them: a local frame of 1,056 instead of 488 bytes when this
+    // was introduced, which eight warps read back every hour past an L1 that did not hold
+    // them (six hours of 95,333 columns 0.47 -> 0.44 ms).  The FP32 step renews it twice
+    // more within the hour (ground_phase32).
     __device__ __forceinline__ void renew() { asm volatile("" : "+l"(base), "+r"(ld)); }
 };
 

@@ -10,12 +10,15 @@
 //     (ibis_pair.cuh);
 //   * what the three canopy passes share formed once before them;
 //   * the 9x9 canopy system (still in double) reduced to its 4x4 canopy-air block;
-//   * one reciprocal where the formulas divide several times by one quantity.
-// Against the templates' operations in float this took the fused kernel from 13,472 to
-// 9,072 instructions and six hours of 95,333 columns from 0.93 to 0.62 ms (0.26 to 0.18
-// at 12,007, an ensemble of 5,696 runs 0.49 to 0.28 ms; B200, 1965 MHz).  The error
-// against the float64 kernels fell by a sixth (geometric mean over every state and
-// accumulator field, 1 and 6 hours, 8,001 columns, six seasons).
+//   * one reciprocal where the formulas divide several times by one quantity;
+//   * constants as register pairs, the passes' shared values in shared memory, the
+//     statics' addresses not carried through the hour.
+// Against the templates' operations in float the fused kernel went from 13,472 to 8,472
+// instructions (7,540 of them in the hour's loop, below the caches' 8,192) and six hours
+// of 95,333 columns from 0.93 to 0.36-0.39 ms (0.26 to 0.10 at 12,007; 24 hours of 356
+// columns 0.94 to 0.34; B200, 1965 MHz).  The error against the float64 kernels fell by a
+// sixth (geometric mean over every state and accumulator field, 1 and 6 hours, 8,001
+// columns, six seasons).
 // Sums and products are regrouped, nothing else: every value keeps the precision it
 // had (the canopy island double, the rest float).
 #pragma once

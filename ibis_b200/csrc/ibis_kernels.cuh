@@ -34,8 +34,8 @@ constexpr int kLongFused = 6;
 constexpr int kDefaultSplit = 8;
 
 // FP32 kernels keep each column's prognostic state in shared memory (array of
-// structures: the 71-word stride is odd, so a warp's accesses to one field fall
-// in 32 different banks); that frees registers for the step's temporaries.
+// structures, an odd number of 64-bit words each); that frees registers for the step's
+// temporaries.
 template <typename R>
 struct StateInSmem {
     static constexpr bool value = IBIS_SMEM_STATE && sizeof(R) == 4;
@@ -194,7 +194,8 @@ __device__ __forceinline__ auto uniform_source(const DevParams<R>& P) {
 // another closely finds its instructions in the SM's instruction cache; warps spread
 // over the body each stream it from the next level (six hours of 95,333 columns in blocks
 // of 128: 0.434 ms together, 0.444 without).  Once an hour is enough: a warp that
-// falls behind fetches faster than the one it follows.
+// falls behind fetches faster than the one it follows.  (Both at the kernel's 8,750
+// instructions; the ensembles' kernel, 9,200, gains a sixth by the same.)
 template <bool ON>
 __device__ __forceinline__ void align_warps(unsigned n) {
     if constexpr (ON) {
@@ -807,10 +808,11 @@ cudaError_t run_config(R* prog, const R* stat, const R* forc, R* diag, R* acc, R
     X(NT, false, false, 0) X(NT, false, false, 6) X(NT, false, false, 8) IBIS_SUN_CONFIGS(X, NT)
 
 // The fused configuration of a launch that leaves it to the library (`sms` SMs).  Two
-// blocks of 128 per SM are the fastest at every size with the F77 canopy: six hours in
-// 2 x 128 / 4 x 64 / 1 x 224 / single-warp blocks, milliseconds: 12,007 columns 0.112 /
-// 0.117 / 0.128 / 0.133; 33,152 0.134 / 0.158 / 0.137 / 0.194; 95,333 0.404 / 0.409 /
-// 0.407 / 0.492 (four warps that run together fetch a body's instructions once for all).
+// blocks of 128 per SM are the fastest with the F77 canopy: six hours in 2 x 128 /
+// 4 x 64 / 1 x 224 / 1 x 256, milliseconds: 12,007 columns 0.121 / 0.125 / 0.139 / 0.140;
+// 33,001 0.138 / 0.150 / 0.148 / 0.143; 95,333 0.378 / 0.392 / 0.391 / 0.384 (single-warp
+// blocks, by the step before it, 19 to 45 % slower).  Only whole days of the largest
+// batches are faster in 1 x 256 (24 hours of 95,333 1.333 against 1.351 ms).
 // The sunlit/shaded canopies and the IBIS 3.0 switches keep a larger record of the
 // hour: one block of 128 fits an SM with its accumulators, so batches of more than that
 // run as one block of 224.
