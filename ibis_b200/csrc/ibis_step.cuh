@@ -209,8 +209,11 @@ __device__ __forceinline__ void surface_phase(Col<R>& c, const Forc<R>& F, const
 // freeze/thaw, the surface-temperature bound -- then the fire counters and the
 // day-loop accumulators (loops.py:676-1275; loops_gswp3.py:161-318).
 template <typename R, int NT, typename Q, typename DD, int SLD>
-__device__ __forceinline__ void ground_phase(Col<R>& c, const Forc<R>& F, const Stat<R>& S, const DD& D,
+__device__ __forceinline__ void ground_phase(Col<R>& c, const Forc<R>& F, Stat<R>& S, const DD& D,
                                              const Acc<R, SLD>& Ac, const DevParams<R>& P, const Q& q, const Mid<R>& M) {
+    // Renewed here and before the sums, as in ground_phase32: 1,009 columns x 3 hours
+    // 0.617 -> 0.600 ms.
+    S.renew();
     const R eps = P.epsilon, dt = P.dtime;
     const R fi = c.fi;
     const R lai0 = S(IBIS_STAT_LAI, 0), lai1 = S(IBIS_STAT_LAI, 1);
@@ -426,6 +429,7 @@ __device__ __forceinline__ void ground_phase(Col<R>& c, const Forc<R>& F, const 
 
     // ---- accumulators of the day loop (loops_gswp3.py:161-318)
     if (Ac.base) {
+        S.renew();
         if (P.flags & IBIS_FLAG_ACC) {
             const R smask = R(1.0) - c.fi;
             R root_t = R(0.0);
