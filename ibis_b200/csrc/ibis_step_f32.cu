@@ -126,26 +126,34 @@ extern "C" int ibis_step_split_noalloc_f32(float* prog, const float* stat, const
 // on one of a few compute streams, and its state is copied out on a second
 // copy stream, so the copies of one group overlap the steps of the others and
 // the groups' kernels fill the SMs together (no group waits for another
-// group's slowest column).  A batch of about a wave or less has no later
-// waves to hide copies behind: its hours are cut into chunks instead, the
-// copy of each chunk overlapping the steps of the chunk before.
+// group's slowest column).  A batch too small for two groups has its hours cut
+// into chunks instead, the copy of each chunk overlapping the steps of the chunk
+// before.
 // ---------------------------------------------------------------------------
 namespace {
 constexpr int kHostStreams = 16;    // compute streams the groups take in turn
 constexpr int kHostMaxGroups = 64;
 constexpr int kHostMaxPieces = 256; // (group, chunk of hours) pairs of one call
-// groups when the caller leaves the size to ibis_step_host_f32: at 95,333
-// cells x 24 hours, each group's day in two chunks, a day from host to host
-// takes 3.17 ms in 16 groups, 3.19 in 12, 3.20 in 24 and 3.26 in 20 (median of
-// 4 interleaved rounds; the same day with its forcing already on the device:
-// 2.99 ms)
-constexpr int kHostAutoGroups = 16;
+// Groups when the caller leaves both the size and the hours to ibis_step_host_f32: of at
+// least kHostGroupCells columns, at most kHostAutoGroups.  The steps take less time than
+// the copies, so what shows is the first group's copy in and the last one's out, and with
+// many groups the copies' and launches' own cost.  Host to host, microseconds, in 1 (its
+// hours in chunks) / 2 / 4 / 8 / 16 groups: 5,003 columns x 6 hours 224 / 196 / 183 / 212 /
+// 272; 12,007 469 / 367 / 334 / 272 / 296; 33,001 750 / 625 / 481 / 400 / 454; 95,333
+// 1,249 / 1,017 / 828 / 815 / 858; 95,333 x 24 hours in two pieces 3,258 / 2,909 / 2,582 /
+// 2,498 / 2,566.
+constexpr int kHostAutoGroups = 8;
+constexpr int kHostGroupCells = 1536;
+// ... and at least this many hours in a group's first piece, a third of its hours: at
+// 95,333 columns in 8 groups one piece against two take 815 / 914 us for 6 hours, 1,450 /
+// 1,454 for 12, 2,534 / 2,498 for 24.
+constexpr int kHostPieceHours = 4;
+// groups when the caller sets the hours of a chunk
+constexpr int kHostChunkedGroups = 16;
 // the same for ibis_day_host_f32 (forcing generated per group from daily weather)
 constexpr int kDayHostAutoGroups = 20;
-// batches of more than this many waves of the launch configuration are cut
-// into groups, smaller ones into chunks of hours.  A day from host to host,
-// groups / chunks: 1 wave (33,152 cells) 2.30 / 1.71 ms; 1.25 waves 2.37 /
-// 2.68 ms; 1.5 waves 2.54 / 2.77 ms; 2 waves 2.88 / 3.00 ms.
+// and then batches of at most this many waves of the launch configuration are one
+// group: more would multiply the pieces (kHostMaxPieces) for no later wave to use
 constexpr double kHostGroupWaves = 1.15;
 
 struct HostPipe {
@@ -181,9 +189,8 @@ int host_error(cudaError_t e, const char* what, const char* entry = "ibis_step_h
 // Hours of each chunk: `chunk` hours each; -c: c hours, then the rest; with
 // chunk 0 and several groups (`whole`), a third of the hours, then the rest
 // (every group's first third is copied before any group's remainder, so the
-// first wave starts after a third of its copy; measured at 49,728 - 95,333
-// cells x 24 hours, [8, 16] beat one chunk by 5-11 % and [4, 20], [12, 12],
-// [16, 8] and 2 x 12 or 4 x 6 equal chunks by up to 14 %); with chunk 0 and one
+// first wave starts after a third of its copy), or all of them where that third
+// is under kHostPieceHours; with chunk 0 and one
 // group, 4 hours growing by 1.75 per chunk, the last taking a remainder under
 // half its size (a copy of each chunk then stays within the steps of the chunk
 // before, and few launches keep their tails few).
@@ -194,7 +201,7 @@ int chunk_schedule(int nstep, int chunk, bool whole, int* out, int cap) {
         int m;
         if (chunk > 0) m = chunk;
         else if (chunk < 0) m = n == 0 ? -chunk : nstep - h;   // -c: c hours, then the rest
-        else if (whole) m = n == 0 ? (nstep + 2) / 3 : nstep - h;
+        else if (whole) m = n == 0 && nstep >= 3 * kHostPieceHours ? (nstep + 2) / 3 : nstep - h;
         else {
             m = (int)c;
             const int rem = nstep - h;
@@ -229,9 +236,14 @@ extern "C" int ibis_step_host_f32(float* prog, const float* stat, const float* h
         // blocks to the batch, and a batch of whole waves would spill into one more
         const int block = ibis::kConfigs[cfg].block;
         const double wave = (double)sms * block * ibis::kConfigs[cfg].minb;
-        group = ncell > kHostGroupWaves * wave
-                    ? ((ncell + kHostAutoGroups - 1) / kHostAutoGroups + block - 1) / block * block
-                    : (ncell + 31) / 32 * 32;
+        int want = 1;
+        if (chunk == 0) {
+            want = ncell / kHostGroupCells;
+            if (want > kHostAutoGroups) want = kHostAutoGroups;
+        } else if (ncell > kHostGroupWaves * wave) {
+            want = kHostChunkedGroups;
+        }
+        group = want > 1 ? ((ncell + want - 1) / want + block - 1) / block * block : (ncell + 31) / 32 * 32;
     }
     const int min_group = ((ncell + kHostMaxGroups - 1) / kHostMaxGroups + 31) / 32 * 32;
     if (group < min_group) group = min_group;

@@ -97,18 +97,19 @@ int ibis_step_split_noalloc_f32(float* prog, const float* stat, const float* for
  * back to HOST memory, for callers whose inputs start and end on the host (the
  * reference's timestep_body called on NumPy state, a day loop fed from files).
  * The copies overlap the steps on streams of the library's own:
- *   - a batch of more than 1.15 waves of the launch configuration is cut into
- *     groups of columns (`group` cells, a multiple of 32; 0 = a sixteenth of
- *     ncell, rounded up to whole blocks of the launch configuration; raised
- *     so there are at most 64 groups), each
+ *   - the batch is cut into groups of columns (`group` cells, a multiple of 32;
+ *     0 = up to eight groups of 1,536 columns or more, in whole blocks of the
+ *     launch configuration; raised so there are at most 64 groups), each
  *     group's forcing copied in, stepped and its state copied out while other
  *     groups step;
- *   - a smaller batch (group 0) is one group whose hours are cut into chunks,
- *     each chunk's copy overlapping the steps of the chunk before.
+ *   - a batch too small for two groups is one group whose hours are cut into
+ *     chunks, each chunk's copy overlapping the steps of the chunk before.
  *   `chunk` sets the hours per chunk: c > 0 equal chunks of c hours; -c, c
- *   hours then the rest; 0, for several groups a third of the hours then the
- *   rest (all groups' first chunks are copied before any group's second), for
- *   one group 4 hours growing by 1.75 per chunk; groups x chunks <= 256.
+ *   hours then the rest; 0, for several groups of 12 hours or more a third of the
+ *   hours then the rest (all groups' first chunks are copied before any group's
+ *   second), of fewer hours all at once, for one group 4 hours growing by 1.75 per
+ *   chunk; groups x chunks <= 256.  With `chunk` set and group 0 the groups are
+ *   sixteenths of a batch of more than 1.15 waves, and a smaller batch is one.
  *   host_forc  [nstep][IBIS_FORC_COUNT][ld]  pinned HOST: hourly forcing
  *   forc       [nstep][IBIS_FORC_COUNT][ld]  DEVICE: where the forcing lands
  *   host_prog  [IBIS_PROG_COUNT][ld] pinned HOST, or NULL: the state after the

@@ -174,3 +174,21 @@ def test_a_launch_of_hours_is_as_many_launches_of_one(cuda_lib, flags, mode):
         for k in a:
             if not k.endswith("_mean"):
                 assert np.array_equal(a[k], b[k], equal_nan=True), k
+
+
+@pytest.mark.parametrize("flags", [0, FLAG_SUNSHADE_U | FLAG_VMAX_MIX])
+@pytest.mark.parametrize("ncell,nstep", [(31, 3), (3071, 12), (3072, 11), (3072, 12), (12289, 2), (20000, 13)])
+def test_the_librarys_groups_of_host_batches_equal_one_launch(cuda_lib, ncell, nstep, flags):
+    """On both sides of the sizes where a batch from host memory is cut into groups, and
+    its groups' hours into pieces: the same kernel over the same columns, bit for bit."""
+    wl = synth.make_workload(ncell, nstep, seed=8)
+    wl.params.flags |= flags
+    ref = Columns.from_host(wl.prog, wl.stat, acc=True)
+    ref.run(ref.forcing(wl.forc), wl.params)
+    cols = Columns.from_host(wl.prog, wl.stat, acc=True)
+    h_forc = torch.from_numpy(synth.forcing_planes(wl.forc, cols.ld)).pin_memory()
+    h_prog = torch.zeros_like(cols.prog, device="cpu").pin_memory()
+    cols.run_host(h_forc, wl.params, host_prog=h_prog)
+    torch.cuda.synchronize()
+    assert torch.equal(cols.prog, ref.prog) and torch.equal(cols.acc, ref.acc)
+    assert torch.equal(h_prog[:, :ncell], ref.prog[:, :ncell].cpu())
