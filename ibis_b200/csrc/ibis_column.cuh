@@ -71,6 +71,15 @@ struct Diag {
     R* __restrict__ base;  // nullptr: diagnostics off
     int ld;
     __device__ __forceinline__ bool on() const { return ON && base != nullptr; }
+    // The same view, new to the compiler (Stat::renew): each group of planes is written
+    // through its own, so that no plane's address is carried from group to group (the FP32
+    // kernel with diagnostics: a local frame of 944 -> 296 bytes, one hour of 5,003 columns
+    // 29.7 -> 25.4 us on the device).
+    __device__ __forceinline__ Diag renewed() const {
+        Diag d = *this;
+        asm volatile("" : "+l"(d.base), "+r"(d.ld));
+        return d;
+    }
     __device__ __forceinline__ void put(int plane, R v) const { base[(size_t)plane * ld] = v; }
     __device__ __forceinline__ void put(int plane, int k, R v) const { base[(size_t)(plane + k) * ld] = v; }
 };

@@ -183,7 +183,8 @@ __device__ __forceinline__ void capacity_group(const int (&idx)[N], const Stat<R
 
 // ---- diagnostics of the radiation (loops.py:1158-1241)
 template <typename R, typename DD>
-__device__ __forceinline__ void radiation_diagnostics(const DD& D, const Rad<R>& Rd) {
+__device__ __forceinline__ void radiation_diagnostics(const DD& to, const Rad<R>& Rd) {
+    const DD D = to.renewed();
             D.put(IBIS_DIAG_SOLU, Rd.solu); D.put(IBIS_DIAG_SOLS, Rd.sols); D.put(IBIS_DIAG_SOLL, Rd.soll);
             D.put(IBIS_DIAG_SOLG, Rd.solg); D.put(IBIS_DIAG_SOLI, Rd.soli);
             D.put(IBIS_DIAG_FIRU, Rd.firu); D.put(IBIS_DIAG_FIRS, Rd.firs); D.put(IBIS_DIAG_FIRL, Rd.firl);
@@ -196,10 +197,11 @@ __device__ __forceinline__ void radiation_diagnostics(const DD& D, const Rad<R>&
 
 // ---- diagnostics of the surface phase (loops.py:1158-1241)
 template <typename R, typename DD>
-__device__ __forceinline__ void surface_diagnostics(const DD& D, const Stom<R>& st, R fwetu, R fwets, R fwetl, R rliqu,
+__device__ __forceinline__ void surface_diagnostics(const DD& to, const Stom<R>& st, R fwetu, R fwets, R fwetl, R rliqu,
                                                     R rliqs, R rliql, R firg, R firi, R firb,
                                                     R fsenu, R fsens, R fsenl, R fseng, R fseni, const Mid<R>& M,
                                                     R rhoa, R hvasug, R hvasui, R q1, R q2, R q3, R q4) {
+    const DD D = to.renewed();
     #pragma unroll
             for (int j = 0; j < 2; ++j) { D.put(IBIS_DIAG_AN_UPPER, j, st.an_u[j]); D.put(IBIS_DIAG_AG_UPPER, j, st.ag_u[j]); }
     #pragma unroll
@@ -222,11 +224,12 @@ __device__ __forceinline__ void surface_diagnostics(const DD& D, const Stom<R>& 
 
 // ---- diagnostics of the ground phase (loops.py:1158-1241)
 template <typename R, typename DD>
-__device__ __forceinline__ void ground_diagnostics(const DD& D, const R (&consoi)[NL], const R (&stressu)[NL],
+__device__ __forceinline__ void ground_diagnostics(const DD& to, const R (&consoi)[NL], const R (&stressu)[NL],
                                                    const R (&stressl)[NL], const R (&pflo_ft)[NL],
                                                    const R (&hflo)[NL + 1], R heatg_avg, R stresstu, R stresstl,
                                                    R gtransu, R gtransl, R grunof, R gdrain, R gadj, R raing_avg,
                                                    R traing_avg, R fhtop_soil, R sflo_bot, R fhtop_snow) {
+    const DD D = to.renewed();
     #pragma unroll
             for (int k = 0; k < NL; ++k) {
                 D.put(IBIS_DIAG_CONSOI, k, consoi[k]);
