@@ -213,13 +213,16 @@ __global__ void __launch_bounds__(BLOCK, MINB) hourly_step_kernel(R* __restrict_
                                                              R* __restrict__ acc, int ncell, int ld, int nstep,
                                                              long long forc_stride, const DevParams<R> P,
                                                              int* __restrict__ status) {
-    // A lane past the batch's end repeats the last cell, writing nothing, so that every
-    // warp is whole at the hours' barriers; warps past it take no part in them.
+    // Where the block's warps meet each hour, a lane past the batch's end repeats the last
+    // cell, writing nothing, so that every warp is whole at the barriers; warps past it
+    // take no part in them.  Without barriers (float64) it leaves at once: nothing would
+    // order its reads of the cell against the stores of the lane it repeats.
+    constexpr bool kTogether = StateInSmem<R>::value && (BLOCK > 32);
     const int i0 = blockIdx.x * BLOCK;
     const int nlive = ncell - i0 < BLOCK ? ncell - i0 : BLOCK;
     const unsigned nbar = (unsigned)(nlive + 31) & ~31u;
-    if (threadIdx.x >= nbar) return;
-    const bool live = (int)threadIdx.x < nlive;
+    if (threadIdx.x >= (kTogether ? nbar : (unsigned)nlive)) return;
+    const bool live = !kTogether || (int)threadIdx.x < nlive;
     const int i = live ? i0 + (int)threadIdx.x : ncell - 1;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     Col<R> creg;
@@ -241,7 +244,7 @@ __global__ void __launch_bounds__(BLOCK, MINB) hourly_step_kernel(R* __restrict_
     column_begin<R>(SM::hour(smem_raw), S, P, uniform_source<R, X3>(P));
 #pragma unroll 1
     for (int s = 0; s < nstep; ++s) {
-        align_warps<StateInSmem<R>::value && (BLOCK > 32)>(nbar);
+        align_warps<kTogether>(nbar);
         Forc<R> F = load_forc(forc + (size_t)s * forc_stride + i, ld);
         A.last = (s + 1 == nstep);
         S.renew();

@@ -73,6 +73,9 @@ struct Acc {
     // Two planes at once (FP32 kernels); returns what their sums grew by.  With
     // slots, p0 is an even one and p1 the next (p1 < 0: p0 alone).
     __device__ __forceinline__ F2 add2(int p0, int p1, const F2& x) const {
+        if constexpr (SLD == 0) {
+            if (!live) return x;     // the planes are the repeated cell's to read, too
+        }
         F2 s, cc(0.0f);
         if constexpr (SLD > 0) {
             const float4 v = chip[(acc_slot(p0) >> 1) * SLD];
@@ -89,7 +92,7 @@ struct Acc {
         if constexpr (SLD > 0) {
             const F2 ck = cn * keep;
             chip[(acc_slot(p0) >> 1) * SLD] = make_float4(t.lo(), t.hi(), ck.lo(), ck.hi());
-        } else if (live) {
+        } else {
             at(p0) = t.lo();
             if (p1 >= 0) at(p1) = t.hi();
             if (kahan) {

@@ -483,7 +483,7 @@ __device__ __forceinline__ void ground_phase(Col<R>& c, const Forc<R>& F, Stat<R
                 } else {
                     R old_ = Ac.get(IBIS_ACC_AYNPP + j);
                     R nw = old_ + inc;
-                    Ac.at(IBIS_ACC_AYNPP + j) = nw;
+                    if (Ac.live) Ac.at(IBIS_ACC_AYNPP + j) = nw;
                     npp = npp + (nw - old_);
                 }
             }
@@ -522,7 +522,7 @@ __device__ __forceinline__ void ground_phase(Col<R>& c, const Forc<R>& F, Stat<R
                 const R nee = S(IBIS_STAT_TCO2MIC) * cf - npp;
                 Ac.add(F.cosz <= R(0.0) ? IBIS_ACC_NEE_NIGHT : IBIS_ACC_NEE_DAY, nee);
             }
-            if (Ac.last) {
+            if (Ac.last && Ac.live) {
                 Ac.at(IBIS_ACC_STRESSTU_LAST) = stresstu;
                 Ac.at(IBIS_ACC_STRESSTL_LAST) = stresstl;
             }
