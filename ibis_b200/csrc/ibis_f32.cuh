@@ -189,8 +189,11 @@ __device__ __forceinline__ void radiation(Rad<float>& out, const Col32& c, const
     } else {
         out.solu = out.sols = out.soll = out.solg = out.soli = 0.0f;
         out.asurd[0] = out.asurd[1] = out.asuri[0] = out.asuri[1] = 0.0f;
-        const float su = F.si[0], sl = (1.0f - fu) * F.si[0];
-        out.scu[0] = out.scu[2] = out.scl[0] = out.scl[2] = 0.0f;
+        // no beam and no scattering: light times zero, which still shows a value that is
+        // not finite to the leaves' sums
+        const float none = 0.0f * F.sd[0] + 0.0f * F.si[0];
+        const float su = F.si[0] + none, sl = (1.0f - fu) * F.si[0] + none;
+        out.scu[0] = out.scu[2] = out.scl[0] = out.scl[2] = none;
         out.scu[1] = out.scu[3] = su;
         out.scl[1] = out.scl[3] = sl;
         out.topparu = su * gu;
