@@ -1538,7 +1538,7 @@ __device__ __forceinline__ float methane32(float f_inund, float rh, const F2 (&t
     const float decay = ex(-zp / mx(m.z_tau, 1e-6f) - zp / mx(m.tau_oxid, 1e-6f));
     const float q10 = pw(m.q10p, (tth - m.t_ref) * 0.1f);
     const float prod = mx(rh, 0.0f) * decay * m.r_ch4 * q10;
-    return tth >= 273.15f ? clip(f_inund, 0.0f, 1.0f) * prod : 0.0f;
+    return tth < 273.15f ? 0.0f : clip(f_inund, 0.0f, 1.0f) * prod;    // a temperature that is not a number shows
 }
 
 // Steps 10-12 of timestep_body, the fire counters and the day-loop accumulators

@@ -46,3 +46,8 @@ def _shows_as_in_float64(hour, group, field, k, value):
 @pytest.mark.parametrize("field", ["solad", "solai"])
 def test_visible_light_at_night(cuda_lib, field, value):
     _shows_as_in_float64(0, "FORC", field, 0, value)
+
+
+@pytest.mark.parametrize("field,k", [("tsoi", 1), ("tsoi", 5), ("wisoi", 3), ("tsoi_deep", 0)])
+def test_soil_state_in_the_methane_sum(cuda_lib, field, k):
+    _shows_as_in_float64(12, "PROG", field, k, float("nan"))
