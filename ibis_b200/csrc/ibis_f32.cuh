@@ -1563,9 +1563,12 @@ __device__ __forceinline__ void ground_phase32(Col32& c, const Forc32& F, Stat32
     float smelt = 0.0f, zheat = 0.0f, sflo_bot = 0.0f, fhtop_snow = 0.0f;
     // Bare of snow and none falling on it: the block's result is known (cover below
     // fimin melts to none, layers at the melting point), and a warp of such columns
-    // skips it.  Launches with diagnostics report the block's fluxes too.
+    // skips it.  Not where a layer's or the buried canopy's temperature is no finite number:
+    // the block would carry that into the soil, and the skip would heal it unnoticed.
+    // Launches with diagnostics report the block's fluxes too.
     const bool snowy = DIAG || !(fi == 0.0f && M.snowg == 0.0f && c.hsno[0] == 0.0f && c.hsno[1] == 0.0f &&
-                                 c.hsno[2] == 0.0f && P.fimin > 0.0f);
+                                 c.hsno[2] == 0.0f && P.fimin > 0.0f &&
+                                 finite((c.tsno[0] + c.tsno[1]) + (c.tsno[2] + c.tlsub)));
     if (!snowy) {
         c.tsno[0] = c.tsno[1] = c.tsno[2] = P.tmelt;
         c.tlsub = tl;

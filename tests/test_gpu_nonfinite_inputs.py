@@ -51,3 +51,9 @@ def test_visible_light_at_night(cuda_lib, field, value):
 @pytest.mark.parametrize("field,k", [("tsoi", 1), ("tsoi", 5), ("wisoi", 3), ("tsoi_deep", 0)])
 def test_soil_state_in_the_methane_sum(cuda_lib, field, k):
     _shows_as_in_float64(12, "PROG", field, k, float("nan"))
+
+
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+@pytest.mark.parametrize("field,k", [("tsno", 0), ("tsno", 1), ("tsno", 2), ("tlsub", 0)])
+def test_snow_temperatures_of_bare_columns(cuda_lib, field, k, value):
+    _shows_as_in_float64(12, "PROG", field, k, value)
