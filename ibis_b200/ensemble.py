@@ -314,10 +314,16 @@ class Ensemble:
     def occupancy(self, block: int) -> int:
         return int(self.lib.ibis_ensemble_occupancy(ctypes.byref(self._pc), int(block)))
 
+    def block_threads(self, block: int) -> int:
+        """The threads a block of ``block`` runs with: the largest an SM's shared memory holds (0: not taken)."""
+        return int(self.lib.ibis_ensemble_block(ctypes.byref(self._pc), int(self.daily), int(block)))
+
     def tune(self, blocks=None, reps: int = 1) -> dict:
-        """Time the persistent launch at each block size (multiples of 32 up to 256);
-        returns ``{"best": block, "ms": {block: ms}}``.  Restores the initial state."""
-        blocks = list(range(32, 257, 32)) if blocks is None else list(blocks)
+        """Time the persistent launch at each block size (multiples of 32, by default all
+        that an SM holds); returns ``{"best": block, "ms": {block: ms}}``.  Restores the
+        initial state."""
+        if blocks is None:
+            blocks = [b for b in range(32, 257, 32) if self.block_threads(b) == b]
         ms = {}
         st = torch.cuda.current_stream(self.device)
         for b in blocks:

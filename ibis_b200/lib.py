@@ -82,6 +82,7 @@ SIGNATURES = {
     "ibis_ensemble_f32": (ctypes.c_int, [_E, _P, ctypes.c_int, ctypes.c_void_p]),
     "ibis_ensemble_hours_f32": (ctypes.c_int, [_E, _P, ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p]),
     "ibis_ensemble_occupancy": (ctypes.c_int, [_P, ctypes.c_int]),
+    "ibis_ensemble_block": (ctypes.c_int, [_P, ctypes.c_int, ctypes.c_int]),
     "ibis_ensemble_daily_f32": (ctypes.c_int, [_E, ctypes.POINTER(IbisEnsembleDailyC), _P, ctypes.c_int,
                                                ctypes.c_void_p]),
     "ibis_diurnal_f32": (ctypes.c_int, [ctypes.c_void_p] * 3 + [ctypes.c_int] * 5

@@ -192,8 +192,9 @@ typedef struct IbisEnsemble {
 
 /* Every run of the ensemble from its first hour to its last in ONE persistent
  * launch: grid = SMs x resident blocks of `block` threads (a multiple of 32,
- * <= 256; 0 picks one from the run count), each warp drawing 32 runs at a time
- * from the work counter.  params->flags selects the model variants and the
+ * <= 256; 0 picks one from the run count; a block larger than an SM's shared
+ * memory holds runs as the largest that fits, ibis_ensemble_block), each warp
+ * drawing 32 runs at a time from the work counter.  params->flags selects the model variants and the
  * accumulators as for ibis_step_f32 (no diagnostics), the IBIS_FLAGS_X3
  * switches included: a run's vector replaces the parameters it carries, and
  * the switches' own tables (coefm_pft, the acclimation tables, crop scales)
@@ -238,6 +239,12 @@ int ibis_ensemble_daily_f32(const IbisEnsemble* ens, const IbisEnsembleDaily* da
 /* Resident blocks per SM of the persistent ensemble kernel at `block` threads,
  * for the variant params->flags selects (0 when it cannot run). */
 int ibis_ensemble_occupancy(const IbisParams* params, int block);
+
+/* The threads a block of `block` runs with in that kernel (`daily`: the
+ * daily-weather form): `block`, or the largest that an SM's shared memory holds
+ * (224, and 192 with the sunlit/shaded canopies, the IBIS 3.0 switches or daily
+ * weather); 0 for a block it does not take.  Needs no device. */
+int ibis_ensemble_block(const IbisParams* params, int daily, int block);
 
 /* Hourly forcing from daily weather on the device: for each of nday days and
  * each hour of the day (86400 / dtime hours), the FORC planes of that hour.
