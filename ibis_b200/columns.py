@@ -16,11 +16,10 @@ import torch
 from . import layout as L
 from . import lib as _lib
 from . import synth
-from .params import (StepParams, FLAG_DIAG, FLAG_ACC, FLAG_CH4, FLAG_SOIL_MEANS, FLAG_SUNSHADE_L, FLAG_SUNSHADE_U,
-                     X3_FLAGS)
+from .params import StepParams, FLAG_DIAG, FLAG_ACC, FLAG_CH4, FLAG_SOIL_MEANS
 
 INT_MAX = 2 ** 31 - 1
-# the fused configurations ibis_step_f32 chooses from (auto_config, csrc/ibis_kernels.cuh)
+# the fused configurations the library chooses from (ibis_launch_config)
 AUTO_FUSED = 0          # two blocks of 128 per SM
 AUTO_LARGE = 6          # one block of 224: the canopy variants with a larger record of the hour
 _ACC_FLAGS = FLAG_ACC | FLAG_CH4 | FLAG_SOIL_MEANS
@@ -156,13 +155,17 @@ class Columns:
 
     # -------------------------------------------------------------- compute
     def launch_config(self, nstep: int, flags: int = 0) -> int:
-        """The launch configuration a call of ``nstep`` hours with the parameter record's
-        ``flags`` uses: the columns' own, or the library's choice for the batch."""
-        if self.config is not None:
-            return self.config
+        """The launch configuration that runs a call of any ``nstep`` hours with the
+        parameter record's ``flags``: the columns' own or the library's choice for the
+        batch, brought to those compiled for the canopy and for diagnostics."""
+        if self.dtype != torch.float32:
+            return 0
+        flags = flags & ~FLAG_DIAG if self.diag is None else flags | FLAG_DIAG
         sms = torch.cuda.get_device_properties(self.device).multi_processor_count
-        large = flags & (X3_FLAGS | FLAG_SUNSHADE_U | FLAG_SUNSHADE_L)
-        return AUTO_LARGE if large and self.ncell > 128 * sms else AUTO_FUSED
+        cfg = _lib.load().ibis_launch_config(-1 if self.config is None else self.config, flags, self.ncell, sms)
+        if cfg < 0:
+            raise ValueError("no launch configuration for these columns")
+        return cfg
 
     def run(self, forc: torch.Tensor, params: StepParams, nstep: int | None = None, stream=None):
         """Advance the columns ``nstep`` hours with forcing ``forc`` (asynchronous)."""

@@ -30,7 +30,7 @@ constexpr LaunchConfig kConfigs[] = {
     {1, 128, 2, 128, 3}, {1, 256, 1, 256, 2}, {1, 128, 3, 128, 4}, {2, 224, 1, 0, 0}};
 constexpr int kNumConfigs = sizeof(kConfigs) / sizeof(kConfigs[0]);
 constexpr int kDefaultFused = 0;
-constexpr int kLongFused = 6;
+constexpr int kLongFused = 6;      // batches of the larger records of the hour (auto_config)
 constexpr int kDefaultSplit = 8;
 
 // FP32 kernels keep each column's prognostic state in shared memory (array of
@@ -760,7 +760,7 @@ cudaError_t launch_split(R* prog, const R* stat, const R* forc, R* diag, R* acc,
 }
 
 // Launches that write diagnostics run the default configuration of their form
-// (dispatch_config): the only ones compiled with the diagnostics writer; the float64
+// (compiled_config): the only ones compiled with the diagnostics writer; the float64
 // kernels always carry it.
 template <typename R, int NT, bool SU, bool SL, int CFG, bool X3 = false>
 cudaError_t run_config(R* prog, const R* stat, const R* forc, R* diag, R* acc, R* mid, int ncell, int ld, int nstep,
@@ -819,11 +819,21 @@ cudaError_t run_config(R* prog, const R* stat, const R* forc, R* diag, R* acc, R
 // The sunlit/shaded canopies and the IBIS 3.0 switches keep a larger record of the
 // hour: one block of 128 fits an SM with its accumulators, so batches of more than that
 // run as one block of 224.
+constexpr unsigned kLargeRecordFlags = IBIS_FLAGS_X3 | IBIS_FLAG_SUNSHADE_U | IBIS_FLAG_SUNSHADE_L;
 inline int auto_config(unsigned flags, int ncell, int sms) {
-    const bool large = (flags & (IBIS_FLAGS_X3 | IBIS_FLAG_SUNSHADE_U | IBIS_FLAG_SUNSHADE_L)) != 0;
-    return large && ncell > 128 * sms ? kLongFused : kDefaultFused;
+    return (flags & kLargeRecordFlags) && ncell > 128 * sms ? kLongFused : kDefaultFused;
 }
 
+// The configuration that runs where `cfg` is asked for: not every one is compiled for the
+// larger records and for launches that write diagnostics.
+inline int compiled_config(int cfg, unsigned flags) {
+    const bool large = (flags & kLargeRecordFlags) != 0, diag = (flags & IBIS_FLAG_DIAG) != 0;
+    if (!large && !diag) return cfg;
+    if (kConfigs[cfg].form == 1) return kDefaultSplit;
+    return large && !diag && cfg == kLongFused ? kLongFused : kDefaultFused;
+}
+
+// cfg: a compiled one (compiled_config)
 template <typename R, int NT, bool SU, bool SL, bool X3>
 cudaError_t dispatch_config(int cfg, R* prog, const R* stat, const R* forc, R* diag, R* acc, R* mid, int ncell,
                             int ld, int nstep, long long fs, const DevParams<R>& P, int* status, cudaStream_t s) {
@@ -837,11 +847,12 @@ cudaError_t dispatch_config(int cfg, R* prog, const R* stat, const R* forc, R* d
         }
         return run_config<R, NT, SU, SL, kDefaultFused, true>(IBIS_ARGS);
     } else if constexpr (X3 || SU || SL) {
-        if (kConfigs[cfg].form == 1) return run_config<R, NT, SU, SL, kDefaultSplit, X3>(IBIS_ARGS);
-        if (cfg == kLongFused && !diag) return run_config<R, NT, SU, SL, kLongFused, X3>(IBIS_ARGS);
-        return run_config<R, NT, SU, SL, kDefaultFused, X3>(IBIS_ARGS);
+        switch (cfg) {
+            case kDefaultSplit: return run_config<R, NT, SU, SL, kDefaultSplit, X3>(IBIS_ARGS);
+            case kLongFused: return run_config<R, NT, SU, SL, kLongFused, X3>(IBIS_ARGS);
+            default: return run_config<R, NT, SU, SL, kDefaultFused, X3>(IBIS_ARGS);
+        }
     } else {
-        if (diag) cfg = kConfigs[cfg].form == 1 ? kDefaultSplit : kDefaultFused;
         switch (cfg) {
             case 1: return run_config<R, NT, SU, SL, 1>(IBIS_ARGS);
             case 2: return run_config<R, NT, SU, SL, 2>(IBIS_ARGS);
@@ -876,6 +887,7 @@ static int hourly_step(R* prog, const R* stat, const R* forc, R* diag, R* acc, i
     if ((hp->flags & (IBIS_FLAG_ACC | IBIS_FLAG_CH4 | IBIS_FLAG_SOIL_MEANS)) && !acc) return -EINVAL;
     if ((hp->flags & IBIS_FLAG_DIAG) && !diag) return -EINVAL;
     if (!(hp->dtime > 0.0)) return -EINVAL;
+    cfg = compiled_config(cfg, hp->flags);
     DevParams<R> P = make_dev_params<R>(*hp);
     P.cell0 = cell0;
     if (!(hp->flags & IBIS_FLAG_DIAG)) diag = nullptr;

@@ -74,6 +74,11 @@ extern "C" int ibis_config_info(int config, int* form, int* block, int* min_bloc
     return 0;
 }
 
+extern "C" int ibis_launch_config(int config, unsigned int flags, int ncell, int sms) {
+    if (config < -1 || config >= ibis::kNumConfigs || ncell < 0 || sms <= 0) return -EINVAL;
+    return ibis::compiled_config(config >= 0 ? config : ibis::auto_config(flags, ncell, sms), flags);
+}
+
 // ---------------------------------------------------------------------------
 // Two-kernel step without any allocation by the caller or the library.
 //

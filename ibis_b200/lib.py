@@ -71,6 +71,7 @@ SIGNATURES = {
     "ibis_step_split_noalloc_f32": (ctypes.c_int, [ctypes.c_void_p] * 5 + [ctypes.c_int] * 3
                                     + [_P, ctypes.c_void_p, ctypes.c_void_p]),
     "ibis_config_info": (ctypes.c_int, [ctypes.c_int] + [_c_int_p] * 5),
+    "ibis_launch_config": (ctypes.c_int, [ctypes.c_int, ctypes.c_uint, ctypes.c_int, ctypes.c_int]),
     "ibis_wetland_dynamic_f32": (ctypes.c_int, [_V] * 4 + [ctypes.c_int] * 2 + [_P, _V]),
     "ibis_wetland_grid": (ctypes.c_int, [ctypes.POINTER(IbisWetlandBuilderC), _V]),
     "ibis_wetland_features": (ctypes.c_int, [ctypes.POINTER(IbisWetlandBuilderC)] + [_V] * 4),

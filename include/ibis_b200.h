@@ -75,6 +75,12 @@ int ibis_step_config_f32(float* prog, const float* stat, const float* forc, floa
 int ibis_num_configs(void);
 int ibis_config_info(int config, int* form, int* block, int* min_blocks, int* block2, int* min_blocks2);
 
+/* The configuration that runs where `config` is asked for (-1: left to the
+ * library, as ibis_step_f32 leaves it) with params->flags `flags` (IBIS_FLAG_DIAG
+ * among them) and `ncell` columns on a device of `sms` SMs: not every one is
+ * compiled for every canopy and for diagnostics.  Needs no device. */
+int ibis_launch_config(int config, unsigned int flags, int ncell, int sms);
+
 /* ibis_step_split_f32 for callers that cannot allocate device memory (an XLA
  * custom-call handler, which must not allocate behind XLA's own allocator; a
  * serving loop that reserved all device memory up front and has none left to
