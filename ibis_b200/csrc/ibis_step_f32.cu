@@ -157,9 +157,34 @@ constexpr int kHostPieceHours = 4;
 constexpr int kHostChunkedGroups = 16;
 // the same for ibis_day_host_f32 (forcing generated per group from daily weather)
 constexpr int kDayHostAutoGroups = 20;
-// and then batches of at most this many waves of the launch configuration are one
-// group: more would multiply the pieces (kHostMaxPieces) for no later wave to use
+
+// Columns of a group where the caller leaves them to the library (`daily`: to
+// ibis_day_host_f32).  Whole blocks: a partial block in every group would add blocks to
+// the batch, and a batch of whole waves would spill into one more.
+// Days from daily weather (small copies) are grouped once they are more than a wave of the
+// launch configuration: one launch then waits for a second, nearly empty wave, and groups
+// fill the SMs together.  In one group / in twenty, microseconds: 36,000 columns 769 / 976,
+// 37,800 (37,888 are a wave) 791 / 994, 38,000 1,032 / 998, 43,000 1,191 / 996; with the
+// release switches (a wave of 33,152) 33,100 831 / 1,142, 33,300 1,282 / 1,139.
+// Batches whose chunks of hours the caller sets are grouped above kHostGroupWaves waves,
+// which for a while longer keeps the pieces (kHostMaxPieces) to the chunks alone; which is
+// faster there depends on the chunk: a day of 38,200 columns in one / in sixteen groups, 4
+// hours each 1,252 / 1,477, 8 hours 1,417 / 1,265, 8 hours then the rest 1,614 / 1,294.
 constexpr double kHostGroupWaves = 1.15;
+int auto_group(bool daily, int cfg, int ncell, int chunk, int sms) {
+    const int block = ibis::kConfigs[cfg].block;
+    const double wave = (double)sms * block * ibis::kConfigs[cfg].minb;
+    int want = 1;
+    if (daily) {
+        if (ncell > wave) want = kDayHostAutoGroups;
+    } else if (chunk == 0) {
+        want = ncell / kHostGroupCells;
+        if (want > kHostAutoGroups) want = kHostAutoGroups;
+    } else if (ncell > kHostGroupWaves * wave) {
+        want = kHostChunkedGroups;
+    }
+    return want > 1 ? ((ncell + want - 1) / want + block - 1) / block * block : (ncell + 31) / 32 * 32;
+}
 
 struct HostPipe {
     bool ready = false;
@@ -222,6 +247,13 @@ int chunk_schedule(int nstep, int chunk, bool whole, int* out, int cap) {
 }
 }  // namespace
 
+extern "C" int ibis_host_group(int daily, int config, unsigned int flags, int ncell, int chunk, int sms) {
+    if (config < -1 || config >= ibis::kNumConfigs || (config >= 0 && ibis::kConfigs[config].form == 1) ||
+        ncell < 0 || sms <= 0)
+        return -EINVAL;
+    return auto_group(daily != 0, config >= 0 ? config : ibis::auto_config(flags, ncell, sms), ncell, chunk, sms);
+}
+
 extern "C" int ibis_step_host_f32(float* prog, const float* stat, const float* host_forc, float* forc, float* diag,
                                   float* acc, float* host_prog, int ncell, int ld, int nstep,
                                   const IbisParams* params, int* status, int group, int chunk, int config,
@@ -236,20 +268,7 @@ extern "C" int ibis_step_host_f32(float* prog, const float* stat, const float* h
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return -ENODEV;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) return -ENODEV;
     const int cfg = config >= 0 ? config : ibis::auto_config(params->flags, ncell, sms);
-    if (group == 0) {
-        // whole blocks per group: a partial block in every group would add
-        // blocks to the batch, and a batch of whole waves would spill into one more
-        const int block = ibis::kConfigs[cfg].block;
-        const double wave = (double)sms * block * ibis::kConfigs[cfg].minb;
-        int want = 1;
-        if (chunk == 0) {
-            want = ncell / kHostGroupCells;
-            if (want > kHostAutoGroups) want = kHostAutoGroups;
-        } else if (ncell > kHostGroupWaves * wave) {
-            want = kHostChunkedGroups;
-        }
-        group = want > 1 ? ((ncell + want - 1) / want + block - 1) / block * block : (ncell + 31) / 32 * 32;
-    }
+    if (group == 0) group = auto_group(false, cfg, ncell, chunk, sms);
     const int min_group = ((ncell + kHostMaxGroups - 1) / kHostMaxGroups + 31) / 32 * 32;
     if (group < min_group) group = min_group;
     const int ngroup = (ncell + group - 1) / group;
@@ -362,13 +381,7 @@ extern "C" int ibis_day_host_f32(float* prog, const float* stat, const float* ho
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return -ENODEV;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) return -ENODEV;
     const int cfg = config >= 0 ? config : ibis::auto_config(params->flags, ncell, sms);
-    if (group == 0) {
-        const int block = ibis::kConfigs[cfg].block;
-        const double wave = (double)sms * block * ibis::kConfigs[cfg].minb;
-        group = ncell > kHostGroupWaves * wave
-                    ? ((ncell + kDayHostAutoGroups - 1) / kDayHostAutoGroups + block - 1) / block * block
-                    : (ncell + 31) / 32 * 32;
-    }
+    if (group == 0) group = auto_group(true, cfg, ncell, 0, sms);
     const int min_group = ((ncell + kHostMaxGroups - 1) / kHostMaxGroups + 31) / 32 * 32;
     if (group < min_group) group = min_group;
     const int ngroup = (ncell + group - 1) / group;

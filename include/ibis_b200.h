@@ -135,8 +135,8 @@ int ibis_step_host_f32(float* prog, const float* stat, const float* host_forc, f
 
 /* Days of the step from daily weather in HOST memory, the state read back to
  * HOST memory: per group of columns (`group` as for ibis_step_host_f32, but
- * 0 = a twentieth of ncell in whole blocks), the
- * group's daily weather copied in, its hourly forcing generated on the device
+ * 0 = a twentieth of a batch of more than one wave of the launch configuration
+ * in whole blocks, and a smaller batch is one group), the group's daily weather copied in, its hourly forcing generated on the device
  * (as ibis_diurnal_f32 generates it, the variates keyed by each cell's index
  * in the caller's numbering, so the forcing equals one call over all cells),
  * its nday * 86400/dtime hours stepped and its state copied out, on streams of
@@ -154,6 +154,11 @@ int ibis_day_host_f32(float* prog, const float* stat, const float* host_daily, f
                       float* forc, float* diag, float* acc, float* host_prog, int ncell, int ld, int nday, int jday0,
                       int day0, unsigned int seed, unsigned int dflags, const IbisParams* params, int* status,
                       int group, int config, void* stream);
+
+/* The columns of a group that ibis_step_host_f32 (daily 0) or ibis_day_host_f32
+ * (daily 1) cuts a batch into with group 0, for its `config`, params->flags and
+ * `chunk` (hourly forcing only), on a device of `sms` SMs.  Needs no device. */
+int ibis_host_group(int daily, int config, unsigned int flags, int ncell, int chunk, int sms);
 
 /* A calibration ensemble: nrun runs, each one parameter vector at one site
  * over its own record of hourly forcing.  Per-run buffers use ld_run, per-site

@@ -47,6 +47,25 @@ def test_the_configuration_that_runs(flags):
     assert rule(0, flags, -1, 148) < 0 and rule(0, flags, 1, 0) < 0
 
 
+def test_groups_of_host_batches():
+    """Hourly forcing: up to eight groups of 1,536 columns or more, whatever a wave is; with
+    the chunks set, sixteen above 1.15 waves.  Daily weather: twenty above one wave.
+    Groups are whole blocks, and cover the batch in no more groups than wanted."""
+    sms, rule = 148, lib.load().ibis_host_group
+    for config, flags, block, wave in ((-1, 0, 128, 37888), (6, 0, 224, 33152), (-1, FLAG_SUNSHADE_U, 224, 33152)):
+        for ncell in (1, 1535, 3071, 3072, 12289, wave, wave + 1, int(1.15 * wave), int(1.15 * wave) + 1, 95333):
+            small = flags and ncell <= 128 * sms                # runs as two blocks of 128
+            for daily, chunk, want in ((0, 0, min(ncell // 1536, 8)), (0, 8, 16 if ncell > 1.15 * wave else 1),
+                                       (1, 0, 20 if ncell > wave else 1)):
+                group = rule(daily, config, flags, ncell, chunk, sms)
+                if want > 1:
+                    assert group % (128 if small else block) == 0 and -(-ncell // group) <= want
+                    assert group < ncell / want + (128 if small else block)
+                else:
+                    assert group == -(-ncell // 32) * 32
+    assert rule(0, 8, 0, 1, 0, sms) < 0 and rule(0, 12, 0, 1, 0, sms) < 0 and rule(0, -1, 0, -1, 0, sms) < 0
+
+
 @pytest.mark.gpu
 def test_columns_report_the_configuration_that_runs(cuda_lib):
     import torch
