@@ -236,7 +236,8 @@ struct Surf2 {
     float pflux;
 };
 
-// mix of two precipitation streams (the third of the reference's mix is always zero here)
+// mix of two precipitation streams (the reference's third carries no water here; what its
+// temperature, not finite, gives the mix is left_over's)
 __device__ __forceinline__ void mix_2(F2& xm, F2& tm, const F2& x1, const F2& t1, const F2& x2, const F2& t2,
                                       float eps) {
     const F2 s = x1 + x2;
@@ -244,6 +245,11 @@ __device__ __forceinline__ void mix_2(F2& xm, F2& tm, const F2& x1, const F2& t1
     const F2 zero(0.0f);
     tm = sel2(a, b, (t1 * x1 + t2 * x2) * rcp2(s), zero);
     xm = sel2(a, b, s, zero);
+}
+
+// A stream of no water from the canopy air: zero, or not a number from an infinite temperature
+__device__ __forceinline__ F2 left_over(float tair, const Par32& P) {
+    return 0.0f * F2(mx(tair, P.tmelt), mn(tair, P.tmelt));
 }
 
 // steph2o (interception.py:174-260) of one story (st: 0 upper leaves, 1 upper stems, 2 lower)
@@ -301,13 +307,13 @@ __device__ __forceinline__ void cascade32(Casc<float>& o, const Col32& c, const 
     if (rains && F.ta > P.tmelt + 1.0e-9f) tw = wet_bulb32(F.ta, F.qa, F.ps, P);
     const F2 zero(0.0f);
     const F2 pr = sel2(rains, snows, F2(F.rain, F.snow), zero);
-    const F2 tp = sel2(rains, snows, F2(mx(tw, P.tmelt), mn(F.ta, P.tmelt)), zero);
+    const F2 tp = sel2(rains, snows, F2(mx(tw, P.tmelt), mn(F.ta, P.tmelt)) + left_over(c.t12, P), zero);
     const Surf2 u = intercept2<0>(c.tu, F2(c.wliqu, c.wsnou), 2.0f * S(IBIS_STAT_LAI, 1), pr, tp, q.wliqumax(),
                                   P.wsnoumax, q.wliqmin(), P);
     const Surf2 s = intercept2<1>(c.ts, F2(c.wliqs, c.wsnos), 2.0f * S(IBIS_STAT_SAI, 1), u.pr, u.tp, q.wliqsmax(),
                                   P.wsnosmax, q.wliqmin(), P);
     F2 pl, tl, pg, tg;
-    mix_2(pl, tl, s.pr * fu, s.tp, pr * (1.0f - fu), tp, eps);
+    mix_2(pl, tl, s.pr * fu, s.tp, pr * (1.0f - fu), tp + left_over(c.t34, P), eps);
     const Surf2 l = intercept2<2>(c.tl, F2(c.wliql, c.wsnol), 2.0f * (S(IBIS_STAT_LAI, 0) + S(IBIS_STAT_SAI, 0)), pl,
                                   tl, q.wliqlmax(), P.wsnolmax, q.wliqmin(), P);
     mix_2(pg, tg, l.pr * fl, l.tp, pl * (1.0f - fl), tl, eps);

@@ -57,3 +57,12 @@ def test_soil_state_in_the_methane_sum(cuda_lib, field, k):
 @pytest.mark.parametrize("field,k", [("tsno", 0), ("tsno", 1), ("tsno", 2), ("tlsub", 0)])
 def test_snow_temperatures_of_bare_columns(cuda_lib, field, k, value):
     _shows_as_in_float64(12, "PROG", field, k, value)
+
+
+@pytest.mark.parametrize("field", ["t12", "t34"])
+def test_canopy_air_where_it_rains_or_snows(cuda_lib, field):
+    """An infinite air temperature shows where precipitation is mixed with the canopy's; the
+    dry columns' is solved anew."""
+    (s32, a32), (s64, a64) = (_run(dt, 12, "PROG", field, 0, float("inf")) for dt in (torch.float32, torch.float64))
+    assert bool(s64.any()) and not bool(s64.all())
+    assert torch.equal(s32, s64) and torch.equal(a32, a64)
