@@ -1264,7 +1264,10 @@ __device__ __forceinline__ void soil_water32(F2 (&w2)[NP], float& wpud, float (&
             const F2 wp(P.iwp2[j]), wm(P.iwm2[j]), rhm(P.irh2[j]);
             const F2 a = wm * F2(hyd[k - 1], hyd[k]) + wp * F2(hyd[k], hyd[k + 1]);
             const F2 b = wm * F2(hs[k - 1], hs[k]) + wp * F2(hs[k], hs[k + 1]);
-            const F2 zb = wm * F2(bex[k - 1], bex[k]) + wp * F2(bex[k], bex[k + 1]) + 0.5f;
+            // rounded to a whole exponent: from the difference, so that layers of one soil give its
+            // own exponent whatever the weights' rounding (half-integer ones lie on the tie)
+            const F2 b0(bex[k - 1], bex[k]);
+            const F2 zb = b0 + wp * (F2(bex[k], bex[k + 1]) - b0) + 0.5f;
             const float n0 = floorf(zb.lo()), n1 = floorf(zb.hi());
             const F2 wa0(w[k - 1], w[k]), wa1(w[k], w[k + 1]);
             const F2 ws = consistent ? wp * wa0 + wm * wa1 : wm * wa0 + wp * wa1;
