@@ -13,12 +13,13 @@
 //   * one reciprocal where the formulas divide several times by one quantity;
 //   * constants as register pairs, the passes' shared values in shared memory, the
 //     statics' addresses not carried through the hour.
-// Against the templates' operations in float the fused kernel went from 13,472 to 8,472
-// instructions (7,540 of them in the hour's loop, below the caches' 8,192) and six hours
-// of 95,333 columns from 0.93 to 0.36-0.39 ms (0.26 to 0.10 at 12,007; 24 hours of 356
-// columns 0.94 to 0.34; B200, 1965 MHz).  The error against the float64 kernels fell by a
-// sixth (geometric mean over every state and accumulator field, 1 and 6 hours, 8,001
-// columns, six seasons).
+// Against the templates' operations in float the fused kernel went from 13,472 to 8,488
+// instructions (about 7,600 of them in the hour, by the size of the kernel without the
+// step; the caches hold 8,192) and six hours of 95,333 columns from 0.92 to 0.40 ms (0.26
+// to 0.10 at 12,007; 24 hours of 356 columns 0.93 to 0.32-0.38, by the box; B200, 1965 MHz).
+// Against the float64 kernels the error of a state or accumulator field is 0.85 times what
+// it was (geometric mean of 106 fields, 1 and 6 hours, 8,001 columns, six seasons; 15
+// fields' grew, none by more than a fifth: profiles/fp32_step_error_8001x6h.md).
 // Sums and products are regrouped, nothing else: every value keeps the precision it
 // had (the canopy island double, the rest float).
 #pragma once

@@ -14,7 +14,10 @@ namespace ibis {
 // day loop keeps (kAccSlots of them, two to a 64-bit word so that a pair is one
 // load, one packed Kahan step and one store); the others -- the day means of the
 // soil state, the last hour's stress and the optional ET and NEE components, all
-// written only under their own flags or once a launch -- stay in the global buffer.
+// written only under their own flags or once a launch -- stay in the global buffer:
+// two blocks of 128 fill an SM's shared memory without them (231 of 233 KB).  With the
+// 19 day means, 95,333 columns x 24 hours take 1.66 against 1.37 ms, x 6 hours 0.50
+// against 0.40, 356 x 24 hours 0.52 against 0.35.
 constexpr int kAccSlots = 25;
 constexpr int kAccPairs = (kAccSlots + 1) / 2;
 
