@@ -490,25 +490,27 @@ __device__ __forceinline__ F2 weight_veg2(const F2& t, const F2& ch, const F2& w
 // stomata (physics/stomata.py:198-1080): the leaves of a story in pairs
 // ===========================================================================
 
-// farquhar's smoothed minimum of two rates (quadratic with curvature theta)
-__device__ __forceinline__ F2 colimit2(const F2& j1, const F2& j2, float theta, float rtheta) {
+// farquhar's smoothed minimum of two rates (quadratic with curvature theta); `least` is
+// the reference's 1e-15 beside the root, in the rates' own units
+constexpr float kLeast = 1.0e-15f;
+__device__ __forceinline__ F2 colimit2(const F2& j1, const F2& j2, float theta, float rtheta, float least) {
     const F2 b = j1 + j2, c = j1 * j2;
-    const F2 q = (b + sq2(mx2(b * b - c * (4.0f * theta), 0.0f))) * 0.5f + 1.0e-15f;
+    const F2 q = (b + sq2(mx2(b * b - c * (4.0f * theta), 0.0f))) * 0.5f + least;
     return mn2(q * rtheta, c * rcp2(q));
 }
 
-__device__ __forceinline__ float colimit1(float j1, float j2, float theta, float rtheta) {
+__device__ __forceinline__ float colimit1(float j1, float j2, float theta, float rtheta, float least) {
     const float b = j1 + j2, c = j1 * j2;
-    const float q = 0.5f * (b + sq(mx(b * b - c * (4.0f * theta), 0.0f))) + 1.0e-15f;
+    const float q = 0.5f * (b + sq(mx(b * b - c * (4.0f * theta), 0.0f))) + least;
     return mn(q * rtheta, c / q);
 }
 
 // gross C3 rate from the light-, enzyme- and export-limited rates
-__device__ __forceinline__ F2 c3_gross(const F2& je, const F2& jc, const F2& js, const Par32& P) {
-    return colimit2(colimit2(je, jc, P.theta3, P.rtheta3), js, P.beta3, P.rbeta3);
+__device__ __forceinline__ F2 c3_gross(const F2& je, const F2& jc, const F2& js, const Par32& P, float least = kLeast) {
+    return colimit2(colimit2(je, jc, P.theta3, P.rtheta3, least), js, P.beta3, P.rbeta3, least);
 }
-__device__ __forceinline__ float c4_gross(float je, float jc, float ji, const Par32& P) {
-    return colimit1(colimit1(je, jc, P.theta4, P.rtheta4), ji, P.beta4, P.rbeta4);
+__device__ __forceinline__ float c4_gross(float je, float jc, float ji, const Par32& P, float least = kLeast) {
+    return colimit1(colimit1(je, jc, P.theta4, P.rtheta4, least), ji, P.beta4, P.rbeta4, least);
 }
 
 // Temperature functions of the two canopies' leaves (upper low half, lower high half)
@@ -528,7 +530,8 @@ __device__ __forceinline__ Kin2 kinetics2(const F2& tleaf, const Par32& P) {
     return k;
 }
 
-// One story's constants of a pass
+// One story's constants of a pass (scale: the light scaling or, with the sunlit/shaded
+// split, the smallest rate of the canopy's in units per leaf area)
 struct Story {
     float gmn, rgb, rh, stress, scale, s, par, fw;
 };
@@ -574,8 +577,8 @@ __device__ __forceinline__ F2 c3_pair(F2& cs, F2& gs, F2& ci_, F2& ag_o, F2& an_
     if constexpr (X3) Xf = X * jf;
     F2 ag, an;
     if constexpr (SUN) {
-        ag = c3_gross(Xf * ss.p.lo(), Y * ss.v.lo(), Z * ss.v.lo(), P) +
-             c3_gross(Xf * ss.p.hi(), Y * ss.v.hi(), Z * ss.v.hi(), P);
+        ag = c3_gross(Xf * ss.p.lo(), Y * ss.v.lo(), Z * ss.v.lo(), P, t.scale) +
+             c3_gross(Xf * ss.p.hi(), Y * ss.v.hi(), Z * ss.v.hi(), P, t.scale);
         an = ag - rd * ss.v.sum();
     } else {
         ag = c3_gross(Xf * t.par, Y, Z, P);
@@ -736,8 +739,8 @@ __device__ __forceinline__ void stomata32(Stom<float>& o, Col32& c, float tu, fl
         const float xe = 4.59e-06f * P.alpha4 * jf4, ji = 18.0e3f * vmax * c4;
         float ag4, an4;
         if constexpr (SUN_L) {
-            ag4 = c4_gross(xe * ss.p.lo(), vmax * ss.v.lo(), ji * ss.v.lo(), P) +
-                  c4_gross(xe * ss.p.hi(), vmax * ss.v.hi(), ji * ss.v.hi(), P);
+            ag4 = c4_gross(xe * ss.p.lo(), vmax * ss.v.lo(), ji * ss.v.lo(), P, t.scale) +
+                  c4_gross(xe * ss.p.hi(), vmax * ss.v.hi(), ji * ss.v.hi(), P, t.scale);
             an4 = ag4 - rd * ss.v.sum();
         } else {
             ag4 = c4_gross(xe * t.par, vmax, ji, P);
@@ -1051,18 +1054,21 @@ __device__ __forceinline__ void surface_phase32(Col32& c, Y& y, const Forc32& F,
                        sai1 > eps ? (Rd.sols + Rd.firs) / (2.0f * sai1) : 0.0f);
         X.fradl = (lai0 + sai0) > eps ? (Rd.soll + Rd.firl) / (2.0f * (lai0 + sai0)) : 0.0f;
         X.toppar = F2(Rd.topparu, Rd.topparl);
-        X.scale = light_scaling2(Rd, F2(lai1, lai0), F2(sai1, sai0), c,
-                                 Q::x3 && (P.flags & IBIS_FLAG_LEAF_ONLY) != 0, P);
+        F2 scale = light_scaling2(Rd, F2(lai1, lai0), F2(sai1, sai0), c,
+                                  Q::x3 && (P.flags & IBIS_FLAG_LEAF_ONLY) != 0, P);
         if constexpr (SUN_U) {
             const SunShade<float> ss = sunshade(Rd.scu, Rd.dbeamu, Rd.termu6, Rd.termu7, lai1, sai1, P);
             const float r = lai1 > 0.0f ? 1.0f / mx(lai1, 1.0e-6f) : 0.0f;    // rates per leaf area
             y.su = Sun4{F2(ss.psun, ss.psha) * r, F2(ss.vsun, ss.vsha) * r};
+            scale = F2(kLeast * mx(r, 1.0f), scale.hi());
         }
         if constexpr (SUN_L) {
             const SunShade<float> ss = sunshade(Rd.scl, Rd.dbeaml, Rd.terml6, Rd.terml7, lai0, sai0, P);
             const float r = lai0 > 0.0f ? 1.0f / mx(lai0, 1.0e-6f) : 0.0f;
             y.sl = Sun4{F2(ss.psun, ss.psha) * r, F2(ss.vsun, ss.vsha) * r};
+            scale = F2(scale.lo(), kLeast * mx(r, 1.0f));
         }
+        X.scale = scale;
         if constexpr (!Q::x3)
             X.vnu = F2(S(IBIS_STAT_EXIST, 0) > 0.5f ? q.vmax(0) : (S(IBIS_STAT_EXIST, 2) > 0.5f ? q.vmax(2) : q.vmax(4)),
                        S(IBIS_STAT_EXIST, 3) > 0.5f ? q.vmax(3) : q.vmax(5));
